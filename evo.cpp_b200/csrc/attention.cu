@@ -73,6 +73,8 @@ split_rope_append_vec_kernel(const bf16 *__restrict__ qkv, const float *__restri
                              const std::size_t heads, const std::size_t head_dim,
                              const std::size_t static_position_offset, const float position_scale,
                              const bool head_major, const int *__restrict__ dynamic_position) {
+  wait_for_producers(qkv, query, key_cache, value_cache, dynamic_position);
+  release_dependents();
   // replayed launches (CUDA graphs) read the position from device memory
   const std::size_t position_offset =
       dynamic_position != nullptr ? static_cast<std::size_t>(*dynamic_position) : static_position_offset;
@@ -290,11 +292,10 @@ int split_rope_append(const void *qkv, const float *inverse_frequency,
     const std::size_t wanted = (threads + 255) / 256;
     const unsigned int grid = static_cast<unsigned int>(wanted > cap ? cap : wanted);
     const auto kernel = four ? split_rope_append_vec_kernel<4> : split_rope_append_vec_kernel<1>;
-    kernel<<<grid, 256, 0, stream>>>(static_cast<const bf16 *>(qkv), inverse_frequency,
-                                     static_cast<bf16 *>(query), static_cast<bf16 *>(key_cache),
-                                     static_cast<bf16 *>(value_cache), rows, heads, head_dim,
-                                     position_offset, position_scale, head_major, dynamic_position);
-    return check_launch("QKV split/RoPE/append kernel");
+    return launch_dependent("QKV split/RoPE/append kernel", kernel, dim3(grid), 256, 0, stream, true, 1,
+                            static_cast<const bf16 *>(qkv), inverse_frequency, static_cast<bf16 *>(query),
+                            static_cast<bf16 *>(key_cache), static_cast<bf16 *>(value_cache), rows, heads, head_dim,
+                            position_offset, position_scale, head_major, dynamic_position);
   }
   if (dynamic_position != nullptr)
     return fail(kUnsupported, "a device-side position needs the vectorised split kernel");

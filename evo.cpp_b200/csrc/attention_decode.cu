@@ -59,9 +59,8 @@ attention_decode_kernel(const bf16 *__restrict__ query, const bf16 *__restrict__
                         const bf16 *__restrict__ value_cache, const Q8PageTable pages, bf16 *__restrict__ output,
                         const int rows, const int static_total_keys, const int heads,
                         const int *__restrict__ dynamic_prefix) {
-  // lets a one-row projection launched with programmatic stream serialisation start (and fetch its
-  // weights) under this kernel; it still waits for this grid to finish before it reads the result
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(query, key_cache, value_cache, output, dynamic_prefix);
+  release_dependents();
   // replayed launches (CUDA graphs) read the number of keys already cached from device memory
   const int total_keys = dynamic_prefix != nullptr ? *dynamic_prefix + rows : static_total_keys;
   __shared__ float warp_partials[kWarps][kPartial];
@@ -192,26 +191,11 @@ template <bool kQ8>
 int launch_decode(const void *query, const void *key_cache, const void *value_cache, const Q8PageTable &pages,
                   const std::size_t rows, const std::size_t total_keys, const std::size_t heads, void *output,
                   cudaStream_t stream, const int *dynamic_prefix) {
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(kSplits, static_cast<unsigned int>(heads), static_cast<unsigned int>(rows));
-  config.blockDim = dim3(kDecodeThreads);
-  config.dynamicSmemBytes = 0;
-  config.stream = stream;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = kSplits;
-  attribute.val.clusterDim.y = 1;
-  attribute.val.clusterDim.z = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  const cudaError_t error = cudaLaunchKernelEx(
-      &config, attention_decode_kernel<kQ8>, static_cast<const bf16 *>(query),
-      static_cast<const bf16 *>(key_cache), static_cast<const bf16 *>(value_cache), pages,
-      static_cast<bf16 *>(output), static_cast<int>(rows), static_cast<int>(total_keys), static_cast<int>(heads),
-      dynamic_prefix);
-  if (error != cudaSuccess)
-    return fail(kCuda, std::string("attention decode kernel launch failed: ") + cudaGetErrorString(error));
-  return check_launch("attention decode kernel");
+  const dim3 grid(kSplits, static_cast<unsigned int>(heads), static_cast<unsigned int>(rows));
+  return launch_dependent("attention decode kernel", attention_decode_kernel<kQ8>, grid, kDecodeThreads, 0, stream, true, kSplits,
+                          static_cast<const bf16 *>(query), static_cast<const bf16 *>(key_cache),
+                          static_cast<const bf16 *>(value_cache), pages, static_cast<bf16 *>(output), static_cast<int>(rows),
+                          static_cast<int>(total_keys), static_cast<int>(heads), dynamic_prefix);
 }
 }  // namespace
 

@@ -29,6 +29,8 @@ head_norm_append_kernel(const T *__restrict__ projection, const std::size_t stri
                         T *__restrict__ value_cache, const int static_position,
                         const int *__restrict__ dynamic_position, const int capacity, const int heads,
                         const int kv_heads, const int dim, const int value_dim, const float epsilon) {
+  wait_for_producers(projection, query, key_cache, value_cache, dynamic_position);
+  release_dependents();
   const std::size_t row = blockIdx.x;
   const std::size_t at = (dynamic_position != nullptr ? *dynamic_position : static_position) + row;
   const T *const source = projection + row * stride;
@@ -165,8 +167,8 @@ __global__ void __launch_bounds__(kRowThreads)
 window_attention_row_kernel(const T *__restrict__ query, const T *__restrict__ key_cache,
                             const T *__restrict__ value_cache, const T *__restrict__ gate, T *__restrict__ output,
                             const RowParams p) {
-  // a one-row projection launched with programmatic stream serialisation may start under this kernel
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(query, key_cache, value_cache, gate, output);
+  release_dependents();
   constexpr int kWidth = kElements * kLanes, kGroups = 32 / kLanes;  // keys that a warp takes at once
   __shared__ float warp_partials[kRowWarps][kWidth + 2];
   __shared__ float cta_partial[kWidth + 2];
@@ -393,22 +395,11 @@ RowParams row_params(const WindowAttentionArgs &a) {
 
 template <typename T, int kVec, int kElements, int kLanes = 8>
 int launch_rows(const WindowAttentionArgs &a, cudaStream_t stream) {
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = kSplits;
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(kSplits, static_cast<unsigned int>(a.heads), static_cast<unsigned int>(a.rows));
-  config.blockDim = dim3(kRowThreads);
-  config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  if (cudaLaunchKernelEx(&config, window_attention_row_kernel<T, kVec, kElements, kLanes>, static_cast<const T *>(a.query),
-                         static_cast<const T *>(a.key_cache), static_cast<const T *>(a.value_cache),
-                         static_cast<const T *>(a.gate), static_cast<T *>(a.output), row_params(a)) != cudaSuccess)
-    return fail(kCuda, std::string("cannot launch the window attention row kernel: ") +
-                           cudaGetErrorString(cudaGetLastError()));
-  return check_launch("window attention row kernel");
+  const dim3 grid(kSplits, static_cast<unsigned int>(a.heads), static_cast<unsigned int>(a.rows));
+  return launch_dependent("window attention row kernel", window_attention_row_kernel<T, kVec, kElements, kLanes>, grid, kRowThreads,
+                          0, stream, true, kSplits, static_cast<const T *>(a.query), static_cast<const T *>(a.key_cache),
+                          static_cast<const T *>(a.value_cache), static_cast<const T *>(a.gate), static_cast<T *>(a.output),
+                          row_params(a));
 }
 
 template <typename T>
@@ -457,16 +448,14 @@ int head_norm_append(const HeadNormArgs &a, cudaStream_t stream) {
   const auto launch = [&](auto tag) {
     using T = decltype(tag);
     const auto kernel = quads ? head_norm_append_kernel<T, true> : head_norm_append_kernel<T, false>;
-    kernel<<<static_cast<unsigned int>(a.rows), kAppendThreads, 0, stream>>>(
-        static_cast<const T *>(a.projection), a.stride, static_cast<int>(a.key_column),
-        static_cast<int>(a.value_column), a.query_gain, a.key_gain, static_cast<T *>(a.query),
-        static_cast<T *>(a.key_cache), static_cast<T *>(a.value_cache), static_cast<int>(a.position),
-        a.dynamic_position, static_cast<int>(a.capacity), static_cast<int>(a.heads), static_cast<int>(a.kv_heads),
-        static_cast<int>(a.dim), static_cast<int>(a.value_dim), a.epsilon);
+    return launch_dependent("head norm kernel", kernel, dim3(static_cast<unsigned int>(a.rows)), kAppendThreads, 0, stream, true, 1,
+                            static_cast<const T *>(a.projection), a.stride, static_cast<int>(a.key_column),
+                            static_cast<int>(a.value_column), a.query_gain, a.key_gain, static_cast<T *>(a.query),
+                            static_cast<T *>(a.key_cache), static_cast<T *>(a.value_cache), static_cast<int>(a.position),
+                            a.dynamic_position, static_cast<int>(a.capacity), static_cast<int>(a.heads),
+                            static_cast<int>(a.kv_heads), static_cast<int>(a.dim), static_cast<int>(a.value_dim), a.epsilon);
   };
-  if (a.type == Activation::kBf16) launch(bf16{});
-  else launch(float{});
-  return check_launch("head norm kernel");
+  return a.type == Activation::kBf16 ? launch(bf16{}) : launch(float{});
 }
 
 int window_attention(const WindowAttentionArgs &a, cudaStream_t stream) {

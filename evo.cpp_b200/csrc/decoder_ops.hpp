@@ -51,8 +51,12 @@ struct LinearF32Args {
   std::size_t row_fanout = 1;
   const int *tile_group = nullptr, *tile_count = nullptr;
   std::size_t tile_rows = 128;
+  bool dependent_launch = false;  // one row: as LinearArgs::dependent_launch
 };
 int linear_f32(const LinearF32Args &args, cudaStream_t stream);
+// gemv.cu: the weight-streaming kernel for one row, which linear_f32() uses where it applies.
+bool one_row_linear_f32_applicable(const LinearF32Args &args);
+int one_row_linear_f32(const LinearF32Args &args, cudaStream_t stream);
 int linear_f32(const float *input, const void *weight, std::size_t rows, std::size_t in_features,
                std::size_t out_features, float *output, bool accumulate, cudaStream_t stream);
 // stream[r, :] = table[token[r], :] in F32, and the same row in `copy` (optional).  Ids >= vocabulary: see embedding().

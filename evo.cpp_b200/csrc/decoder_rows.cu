@@ -74,6 +74,8 @@ embed_positions_kernel(const std::uint32_t *__restrict__ tokens, const bf16 *__r
                        const bf16 *__restrict__ positions, const float *__restrict__ gain, const int width,
                        const std::uint32_t vocabulary, const int position, const int *__restrict__ dynamic_position,
                        const float epsilon, float *__restrict__ output, int *const error_word) {
+  wait_for_producers(tokens, dynamic_position, output);
+  release_dependents();
   __shared__ float scratch[kThreads / 32];
   const std::size_t row = blockIdx.x;
   const std::uint32_t token = tokens[row];
@@ -109,6 +111,8 @@ template <typename T, bool kVector>
 __global__ void __launch_bounds__(kThreads)
 rms_norm_residual_kernel(const float *__restrict__ input, const float *__restrict__ gain, const int width,
                          const float epsilon, T *__restrict__ output) {
+  wait_for_producers(input, output);
+  release_dependents();
   __shared__ float scratch[kThreads / 32];
   const float *const x = input + static_cast<std::size_t>(blockIdx.x) * width;
   T *const out = output + static_cast<std::size_t>(blockIdx.x) * width;
@@ -128,6 +132,8 @@ template <typename T, bool kVector>
 __global__ void __launch_bounds__(kThreads)
 poly_norm_kernel(const T *input, const float *__restrict__ coefficients, const int width, const float epsilon,
                  T *output) {
+  wait_for_producers(input, output);
+  release_dependents();
   __shared__ float scratch[kThreads / 32];
   const T *const z = input + static_cast<std::size_t>(blockIdx.x) * width;
   T *const out = output + static_cast<std::size_t>(blockIdx.x) * width;
@@ -196,6 +202,8 @@ __global__ void __launch_bounds__(kThreads)
 embed_rows_kernel(const std::uint32_t *__restrict__ tokens, const bf16 *__restrict__ table, const int width,
                   const std::uint32_t vocabulary, float *__restrict__ stream_rows, T *__restrict__ copy,
                   int *const error_word) {
+  wait_for_producers(tokens, stream_rows, copy);
+  release_dependents();
   const std::size_t row = blockIdx.x;
   const std::uint32_t token = tokens[row];
   const bool known = token < vocabulary;
@@ -225,8 +233,8 @@ struct LayerNormParams {
 template <typename In, typename Out, bool kVector, int kKeep>
 __global__ void __launch_bounds__(kThreads)
 layer_norm_kernel(const In *__restrict__ input, Out *__restrict__ output, const LayerNormParams p) {
-  // a one-row projection launched with programmatic stream serialisation may start under this kernel
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(input, output);
+  release_dependents();
   __shared__ float scratch[kThreads / 32];
   const std::size_t row = blockIdx.x;
   const int groups = (p.width + 7) / 8;
@@ -439,10 +447,10 @@ int embed_positions(const std::uint32_t *tokens, const void *table, const void *
   if (error == nullptr) return status;
   const bool vector = row_vector_ok(width, table, positions, output) && aligned16(gain);
   const auto kernel = vector ? embed_positions_kernel<true> : embed_positions_kernel<false>;
-  kernel<<<static_cast<unsigned int>(rows), kThreads, 0, stream>>>(
-      tokens, static_cast<const bf16 *>(table), static_cast<const bf16 *>(positions), gain, static_cast<int>(width),
-      static_cast<std::uint32_t>(vocabulary), static_cast<int>(position), dynamic_position, epsilon, output, error);
-  return check_launch("embedding kernel with positions");
+  return launch_dependent("embedding kernel with positions", kernel, dim3(static_cast<unsigned int>(rows)), kThreads, 0, stream,
+                          true, 1, tokens, static_cast<const bf16 *>(table), static_cast<const bf16 *>(positions), gain,
+                          static_cast<int>(width), static_cast<std::uint32_t>(vocabulary), static_cast<int>(position),
+                          dynamic_position, epsilon, output, error);
 }
 
 int rms_norm_residual(const float *input, const float *gain, const std::size_t rows, const std::size_t width,
@@ -456,12 +464,12 @@ int rms_norm_residual(const float *input, const float *gain, const std::size_t r
   const int w = static_cast<int>(width);
   if (type == Activation::kBf16) {
     const auto kernel = vector ? rms_norm_residual_kernel<bf16, true> : rms_norm_residual_kernel<bf16, false>;
-    kernel<<<grid, kThreads, 0, stream>>>(input, gain, w, epsilon, static_cast<bf16 *>(output));
-  } else {
-    const auto kernel = vector ? rms_norm_residual_kernel<float, true> : rms_norm_residual_kernel<float, false>;
-    kernel<<<grid, kThreads, 0, stream>>>(input, gain, w, epsilon, static_cast<float *>(output));
+    return launch_dependent("residual norm kernel", kernel, dim3(grid), kThreads, 0, stream, true, 1, input, gain, w, epsilon,
+                            static_cast<bf16 *>(output));
   }
-  return check_launch("residual norm kernel");
+  const auto kernel = vector ? rms_norm_residual_kernel<float, true> : rms_norm_residual_kernel<float, false>;
+  return launch_dependent("residual norm kernel", kernel, dim3(grid), kThreads, 0, stream, true, 1, input, gain, w, epsilon,
+                          static_cast<float *>(output));
 }
 
 int poly_norm(const void *input, const float *coefficients, const std::size_t rows, const std::size_t width,
@@ -475,14 +483,12 @@ int poly_norm(const void *input, const float *coefficients, const std::size_t ro
   const int w = static_cast<int>(width);
   if (type == Activation::kBf16) {
     const auto kernel = vector ? poly_norm_kernel<bf16, true> : poly_norm_kernel<bf16, false>;
-    kernel<<<grid, kThreads, 0, stream>>>(static_cast<const bf16 *>(input), coefficients, w, epsilon,
-                                          static_cast<bf16 *>(output));
-  } else {
-    const auto kernel = vector ? poly_norm_kernel<float, true> : poly_norm_kernel<float, false>;
-    kernel<<<grid, kThreads, 0, stream>>>(static_cast<const float *>(input), coefficients, w, epsilon,
-                                          static_cast<float *>(output));
+    return launch_dependent("polynomial activation kernel", kernel, dim3(grid), kThreads, 0, stream, true, 1,
+                            static_cast<const bf16 *>(input), coefficients, w, epsilon, static_cast<bf16 *>(output));
   }
-  return check_launch("polynomial activation kernel");
+  const auto kernel = vector ? poly_norm_kernel<float, true> : poly_norm_kernel<float, false>;
+  return launch_dependent("polynomial activation kernel", kernel, dim3(grid), kThreads, 0, stream, true, 1,
+                          static_cast<const float *>(input), coefficients, w, epsilon, static_cast<float *>(output));
 }
 
 int distance_bias_table(const float *r1, const float *r2, const std::size_t heads, const std::size_t distances,
@@ -509,14 +515,11 @@ int embed_rows(const std::uint32_t *tokens, const void *table, const std::size_t
   const auto launch = [&](auto tag) {
     using T = decltype(tag);
     const auto kernel = vector ? embed_rows_kernel<T, true> : embed_rows_kernel<T, false>;
-    kernel<<<static_cast<unsigned int>(rows), kThreads, 0, stream>>>(tokens, static_cast<const bf16 *>(table),
-                                                                     static_cast<int>(width),
-                                                                     static_cast<std::uint32_t>(vocabulary), stream_rows,
-                                                                     static_cast<T *>(copy), error);
+    return launch_dependent("embedding kernel of the residual stream", kernel, dim3(static_cast<unsigned int>(rows)), kThreads, 0,
+                            stream, true, 1, tokens, static_cast<const bf16 *>(table), static_cast<int>(width),
+                            static_cast<std::uint32_t>(vocabulary), stream_rows, static_cast<T *>(copy), error);
   };
-  if (type == Activation::kBf16) launch(bf16{});
-  else launch(float{});
-  return check_launch("embedding kernel of the residual stream");
+  return type == Activation::kBf16 ? launch(bf16{}) : launch(float{});
 }
 
 int layer_norm(const LayerNormArgs &a, cudaStream_t stream) {
@@ -539,17 +542,12 @@ int layer_norm(const LayerNormArgs &a, cudaStream_t stream) {
                         : a.width <= 8 * kThreads  ? layer_norm_kernel<In, Out, true, 1>
                         : a.width <= 16 * kThreads ? layer_norm_kernel<In, Out, true, 2>
                                                    : layer_norm_kernel<In, Out, true, kCached>;
-    kernel<<<static_cast<unsigned int>(a.rows), kThreads, 0, stream>>>(static_cast<const In *>(a.input),
-                                                                       static_cast<Out *>(a.output), p);
+    return launch_dependent("layer norm kernel", kernel, dim3(static_cast<unsigned int>(a.rows)), kThreads, 0, stream, true, 1,
+                            static_cast<const In *>(a.input), static_cast<Out *>(a.output), p);
   };
-  if (a.input_type == Activation::kBf16) {
-    if (a.output_type == Activation::kBf16) launch(bf16{}, bf16{});
-    else launch(bf16{}, float{});
-  } else {
-    if (a.output_type == Activation::kBf16) launch(float{}, bf16{});
-    else launch(float{}, float{});
-  }
-  return check_launch("layer norm kernel");
+  if (a.input_type == Activation::kBf16)
+    return a.output_type == Activation::kBf16 ? launch(bf16{}, bf16{}) : launch(bf16{}, float{});
+  return a.output_type == Activation::kBf16 ? launch(float{}, bf16{}) : launch(float{}, float{});
 }
 
 int convert_rows(const float *input, const std::size_t elements, void *output, const Activation type, cudaStream_t stream) {
@@ -588,6 +586,7 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
       (a.row_group != nullptr && a.rows > 65535U))
     return fail(kInvalidArgument, "F32 linear arguments are invalid");
   if (a.rows == 0) return kOk;
+  if (one_row_linear_f32_applicable(a)) return one_row_linear_f32(a, stream);
   F32Params p{};
   p.weight = static_cast<const bf16 *>(a.weight);
   p.output = a.output;

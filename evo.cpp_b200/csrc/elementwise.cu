@@ -367,19 +367,15 @@ __global__ void __launch_bounds__(kThreads)
 rms_norm_few_rows_kernel(const bf16 *__restrict__ input, const float *__restrict__ scale,
                          bf16 *__restrict__ output, std::uint8_t *__restrict__ codes, const int width,
                          const float epsilon, const float quant_scale) {
-  // lets a one-row projection launched with programmatic stream serialisation start (and fetch its
-  // weights) under this kernel; it still waits for this grid to finish before it reads the result
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(input, scale, output, codes);
+  release_dependents();
   __shared__ float partial[32];
   const std::size_t row = blockIdx.x;
   const unsigned short *const in = reinterpret_cast<const unsigned short *>(input) + row * width;
   unsigned short raw[kPerThread];
   float gain[kPerThread];
 #pragma unroll
-  for (int k = 0; k < kPerThread; ++k) gain[k] = __ldg(scale + threadIdx.x + k * kThreads);
-  // launched with programmatic stream serialisation, the gains above were requested while the kernel
-  // that writes the row may still be running; otherwise this returns at once
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (int k = 0; k < kPerThread; ++k) gain[k] = scale[threadIdx.x + k * kThreads];
 #pragma unroll
   for (int k = 0; k < kPerThread; ++k) raw[k] = in[threadIdx.x + k * kThreads];
   float sum = 0.0F;
@@ -426,6 +422,8 @@ rms_norm_stream_kernel(const bf16 *__restrict__ input, const float *__restrict__
   extern __shared__ __align__(16) unsigned short row_cache[];  // 2 x width BF16 values, then width BF16 scales
   __shared__ float partial[32];
   const std::size_t width = kWidth != 0 ? static_cast<std::size_t>(kWidth) : runtime_width;
+  wait_for_producers(input, scale, output, codes);
+  release_dependents();
   std::uint32_t *const scale_pairs = reinterpret_cast<std::uint32_t *>(row_cache + 2 * width);
   for (std::size_t i = threadIdx.x; i < width / 2; i += kThreads)
     scale_pairs[i] = round_pair(scale[2 * i], scale[2 * i + 1]);  // visible after the first barrier below
@@ -510,6 +508,8 @@ __global__ void pointwise_kernel(const bf16 *__restrict__ first,
                                  const bf16 *__restrict__ second,
                                  bf16 *__restrict__ output,
                                  const std::size_t elements) {
+  wait_for_producers(first, second, output);
+  release_dependents();
   const std::size_t vectors = elements / 8;
   const std::size_t stride = static_cast<std::size_t>(blockDim.x) * gridDim.x;
   const std::size_t tid =
@@ -556,6 +556,8 @@ __global__ void embedding_kernel(const std::uint32_t *__restrict__ tokens,
                                  const std::size_t width,
                                  const std::size_t vocabulary,
                                  int *const error_word) {
+  wait_for_producers(tokens, output);
+  release_dependents();
   const std::size_t elements = rows * width;
   const std::size_t stride = static_cast<std::size_t>(blockDim.x) * gridDim.x;
   for (std::size_t i = static_cast<std::size_t>(blockIdx.x) * blockDim.x +
@@ -577,6 +579,8 @@ __global__ void split_triples_kernel(const bf16 *__restrict__ projection,
                                      bf16 *__restrict__ x1,
                                      bf16 *__restrict__ value,
                                      const std::size_t elements) {
+  wait_for_producers(projection, x2, x1, value);
+  release_dependents();
   const std::size_t stride = static_cast<std::size_t>(blockDim.x) * gridDim.x;
   for (std::size_t i = static_cast<std::size_t>(blockIdx.x) * blockDim.x +
                        threadIdx.x;
@@ -678,7 +682,7 @@ int quantize_f32(const float *input, const std::size_t elements,
 
 int rms_norm(const void *input, const float *scale, const std::size_t rows,
              const std::size_t width, const float epsilon, void *output,
-             void *codes, const float quant_scale, cudaStream_t stream, const bool dependent_launch) {
+             void *codes, const float quant_scale, cudaStream_t stream) {
   if (input == nullptr || scale == nullptr ||
       (output == nullptr && codes == nullptr) || width == 0 ||
       width > 24576 || rows > 0x7fffffffU)
@@ -693,20 +697,9 @@ int rms_norm(const void *input, const float *scale, const std::size_t rows,
                        (output == nullptr || aligned(output, 15)) && (codes == nullptr || aligned(codes, 7));
   if (rows <= 8 && width % kThreads == 0) {
     const auto launch_few = [&](auto kernel) {
-      cudaLaunchAttribute attribute{};
-      attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attribute.val.programmaticStreamSerializationAllowed = dependent_launch ? 1 : 0;
-      cudaLaunchConfig_t config{};
-      config.gridDim = dim3(static_cast<unsigned int>(rows));
-      config.blockDim = dim3(kThreads);
-      config.stream = stream;
-      config.attrs = &attribute;
-      config.numAttrs = 1;
-      if (cudaLaunchKernelEx(&config, kernel, static_cast<const bf16 *>(input), scale, static_cast<bf16 *>(output),
-                             static_cast<std::uint8_t *>(codes), static_cast<int>(width), epsilon,
-                             quant_scale) != cudaSuccess)
-        return fail(kCuda, "cannot launch the RMSNorm kernel");
-      return check_launch("RMSNorm kernel");
+      return launch_dependent("RMSNorm kernel", kernel, dim3(static_cast<unsigned int>(rows)), kThreads, 0, stream, true, 1,
+                              static_cast<const bf16 *>(input), scale, static_cast<bf16 *>(output),
+                              static_cast<std::uint8_t *>(codes), static_cast<int>(width), epsilon, quant_scale);
     };
     switch (width / kThreads) {
       case 1: return launch_few(rms_norm_few_rows_kernel<1>);
@@ -730,10 +723,9 @@ int rms_norm(const void *input, const float *scale, const std::size_t rows,
           resident < 1)
         resident = 1;
       const std::size_t grid = std::min<std::size_t>(rows, static_cast<std::size_t>(kSmCount) * resident);
-      kernel<<<static_cast<unsigned int>(grid), kThreads, smem, stream>>>(
-          static_cast<const bf16 *>(input), scale, static_cast<bf16 *>(output), static_cast<std::uint8_t *>(codes),
-          rows, width, epsilon, quant_scale);
-      return check_launch("RMSNorm kernel");
+      return launch_dependent("RMSNorm kernel", kernel, dim3(static_cast<unsigned int>(grid)), kThreads, smem, stream, true, 1,
+                              static_cast<const bf16 *>(input), scale, static_cast<bf16 *>(output),
+                              static_cast<std::uint8_t *>(codes), rows, width, epsilon, quant_scale);
     };
     // width 4096 (the 7B shape) gets the fully unrolled kernel: 30.7 against 32.8 us when it writes E4M3
     // codes, no difference for BF16 output; at 8192 the unrolled form measured slower (49 against 45 us)
@@ -758,10 +750,8 @@ static int launch_pointwise(const void *a, const void *b, void *out,
   if (!aligned16(a) || !aligned16(out) || (b != nullptr && !aligned16(b)))
     return fail(kInvalidArgument,
                 std::string(what) + " buffers must be 16-byte aligned");
-  pointwise_kernel<Op><<<grid_for(elements / 8 + 1), kThreads, 0, stream>>>(
-      static_cast<const bf16 *>(a), static_cast<const bf16 *>(b),
-      static_cast<bf16 *>(out), elements);
-  return check_launch(what);
+  return launch_dependent(what, pointwise_kernel<Op>, dim3(grid_for(elements / 8 + 1)), kThreads, 0, stream, true, 1,
+                          static_cast<const bf16 *>(a), static_cast<const bf16 *>(b), static_cast<bf16 *>(out), elements);
 }
 
 int gelu(const void *input, void *output, const std::size_t elements,
@@ -808,10 +798,8 @@ int embedding(const std::uint32_t *tokens, const void *table,
   int status = kOk;
   int *const error_word = device_error_word(&status);
   if (error_word == nullptr) return status;
-  embedding_kernel<<<grid_for(rows * width), kThreads, 0, stream>>>(
-      tokens, static_cast<const bf16 *>(table), static_cast<bf16 *>(output),
-      rows, width, vocabulary, error_word);
-  return check_launch("embedding kernel");
+  return launch_dependent("embedding kernel", embedding_kernel, dim3(grid_for(rows * width)), kThreads, 0, stream, true, 1, tokens,
+                          static_cast<const bf16 *>(table), static_cast<bf16 *>(output), rows, width, vocabulary, error_word);
 }
 
 int split_triples(const void *projection, const std::size_t rows,
@@ -821,10 +809,9 @@ int split_triples(const void *projection, const std::size_t rows,
       value == nullptr || width == 0)
     return fail(kInvalidArgument, "projection split arguments are invalid");
   if (rows == 0) return kOk;
-  split_triples_kernel<<<grid_for(rows * width), kThreads, 0, stream>>>(
-      static_cast<const bf16 *>(projection), static_cast<bf16 *>(x2),
-      static_cast<bf16 *>(x1), static_cast<bf16 *>(value), rows * width);
-  return check_launch("projection split kernel");
+  return launch_dependent("projection split kernel", split_triples_kernel, dim3(grid_for(rows * width)), kThreads, 0, stream, true,
+                          1, static_cast<const bf16 *>(projection), static_cast<bf16 *>(x2), static_cast<bf16 *>(x1),
+                          static_cast<bf16 *>(value), rows * width);
 }
 
 int transpose(const void *input, const std::size_t rows,

@@ -79,8 +79,8 @@ route_logits_kernel(const float *__restrict__ logits, const std::size_t stride, 
 template <typename T, bool kVector, int kPerLane>
 __global__ void __launch_bounds__(32 * kRouteWarps)
 route_rows_kernel(const T *__restrict__ input, const bf16 *__restrict__ router, const int width, const Choice c) {
-  // a grouped projection launched with programmatic stream serialisation may start under this kernel
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(input);
+  release_dependents();
   __shared__ float logits[kDecoderMaxExperts / kRouterSplits + kRouteWarps];  // of this CTA's experts
   cg::cluster_group cluster = cg::this_cluster();
   const int split = static_cast<int>(cluster.block_rank()), warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -174,24 +174,12 @@ group_rows_kernel(const T *__restrict__ input, T *__restrict__ grouped, const in
 template <typename T>
 int launch_route_rows(const RouteArgs &a, const Choice &c, cudaStream_t stream) {
   const bool vector = a.width % 8 == 0 && aligned16(a.input) && aligned16(a.router);
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = kRouterSplits;
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(kRouterSplits, static_cast<unsigned int>(a.rows));
-  config.blockDim = dim3(32 * kRouteWarps);
-  config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
   const auto kernel = a.experts <= 64 ? (vector ? route_rows_kernel<T, true, 2> : route_rows_kernel<T, false, 2>)
                                       : (vector ? route_rows_kernel<T, true, kMaxPerLane>
                                                 : route_rows_kernel<T, false, kMaxPerLane>);
-  if (cudaLaunchKernelEx(&config, kernel,
-                         static_cast<const T *>(a.input), static_cast<const bf16 *>(a.router), static_cast<int>(a.width),
-                         c) != cudaSuccess)
-    return fail(kCuda, std::string("cannot launch the router kernel: ") + cudaGetErrorString(cudaGetLastError()));
-  return check_launch("router kernel");
+  return launch_dependent("router kernel", kernel, dim3(kRouterSplits, static_cast<unsigned int>(a.rows)), 32 * kRouteWarps, 0,
+                          stream, true, kRouterSplits, static_cast<const T *>(a.input), static_cast<const bf16 *>(a.router),
+                          static_cast<int>(a.width), c);
 }
 
 }  // namespace

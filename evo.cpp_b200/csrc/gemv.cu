@@ -2,13 +2,17 @@
 // At these sizes a projection is a weight stream: every weight byte is read
 // once and the arithmetic is negligible, so the tensor-core tile kernel (which
 // launches one CTA per 128 x 256 tile and leaves most SMs idle) is replaced by
-// a kernel in which a CTA owns a few weight rows, its threads split K in
+// kernels in which a CTA owns weight rows, its threads split K in
 // 16-byte chunks, and partial sums are folded with shuffles and shared memory.  Same epilogue
 // contract as the tile kernel (scale, fused or separately rounded bias,
 // residual, gate over row-interleaved up-projections).
 #include <cuda_fp8.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
+#include "decoder_types.cuh"
 #include "gates.cuh"
 #include "ops_internal.hpp"
 
@@ -19,7 +23,7 @@ constexpr int kThreads = 256;
 constexpr int kMaxRows = 8;
 
 struct GemvParams {
-  const void *x;       // [rows, K] BF16 or E4M3 codes
+  const void *x;       // [rows, K] BF16 or E4M3 codes; F32 in one-row streams of F32 activations
   const void *w;       // [N, K] same type
   const bf16 *bias, *residual;
   bf16 *out;
@@ -34,6 +38,7 @@ struct GemvParams {
   // grouped weights [groups, N, K]: blockIdx.y = output row r, x row r / row_fanout, weight of group row_group[r]
   const int *row_group;
   int row_fanout;
+  int row_group_settled;   // LinearArgs::row_group_settled
   const float *row_scale;  // grouped weights only
 };
 
@@ -73,6 +78,42 @@ __device__ __forceinline__ bf16 gelu_round_small(const float x) {
     case 0xc0a8: return __ushort_as_bfloat16(0xb4fc);
     case 0xc0ab: return __ushort_as_bfloat16(0xb4ab);
     default: return computed;
+  }
+}
+
+// Result `column` of row r (of `out_index` where rows are grouped) from its sum, or from the sums of a gated pair.
+template <class Total>
+__device__ __forceinline__ void finish_column(const GemvParams &p, const int r, const std::size_t out_index,
+                                              const int out_columns, const int column, const float alpha, const int local,
+                                              const Total &total) {
+  if (p.out_f32 != nullptr) {
+    float *const slot = p.out_f32 + out_index * out_columns + column;
+    float value = total(local) * alpha;
+    if (p.bias_f32 != nullptr) value += p.bias_f32[column];
+    *slot = soft_cap(p.accumulate_f32 != 0 ? *slot + value : value, p.softcap);
+    return;
+  }
+  bf16 *const out_row = p.out + out_index * out_columns;
+  if (p.gate_mode >= kGateRelu) {
+    float value = total(2 * local) * alpha, up = total(2 * local + 1) * alpha;
+    if (p.bias_f32 != nullptr) {
+      const int row = (column / 128) * 256 + column % 128;
+      value += p.bias_f32[row];
+      up += p.bias_f32[row + 128];
+    }
+    out_row[column] = f2bf(gated_value(p.gate_mode, p.gate_limit, value, up));
+  } else if (p.gate_mode != 0) {
+    const float first = total(2 * local) * p.alpha, second = rbf(total(2 * local + 1) * p.alpha);
+    const float activated = p.gate_mode == 2 ? bf2f(gelu_round_small(first)) : rbf(first);
+    out_row[column] = f2bf(activated * second);
+  } else {
+    float value = total(local) * alpha;
+    if (p.bias_mode == 1) value += bf2f(p.bias[column]);
+    value = rbf(value);
+    if (p.bias_mode == 2) value = rbf(value + bf2f(p.bias[column]));
+    if (p.residual != nullptr)
+      value = rbf(value + bf2f(p.residual[static_cast<std::size_t>(r) * out_columns + column]));
+    out_row[column] = f2bf(value);
   }
 }
 
@@ -173,79 +214,253 @@ gemv_kernel(const GemvParams p) {
   if (r >= p.rows || column >= out_columns) return;
   const std::size_t out_index = grouped ? blockIdx.y : r;
   const float alpha = grouped && p.row_scale != nullptr ? p.alpha * p.row_scale[out_index] : p.alpha;
-  const auto total = [&](const int c) {
+  finish_column(p, r, out_index, out_columns, column, alpha, local, [&](const int c) {
     float sum = 0.0F;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) sum += partial[w][c][r];
     return sum;
+  });
+}
+
+// One row: the projection is a stream of the weights and nothing else, so what counts is that loads are in flight
+// all the time, also while kernels in front of this one are still running.  A CTA owns a contiguous share of the
+// output columns and each of its eight warps an eighth of K, whose piece of x stays in registers.  A thread
+// copies its 16-byte pieces of the weight rows into its own slots of a ring in shared memory
+// (cp.async) and reads only what it copied itself: no barrier in the loop, and the ring is filled before the thread
+// waits for the producer of x (the weights do not depend on it).  The warps' partial sums of all columns meet in
+// shared memory once, at the end.  The CTAs of two such kernels fit an SM, so the next projection of a decode step
+// fills its ring while this one drains.
+// Grouped rows (blockIdx.y) take their weights' rows the same way, once they know their group.
+// Bound: HBM.  Back to back in a graph, weights beyond L2 (us; in brackets one CTA per four rows with registers and
+// prefetches into L2): 8448 x 2048 6.2 (8.3), 4096 x 4096 5.9 (7.4), gated 22528 x 4096 26.9 = 6.9 TB/s (29.3),
+// 4096 x 11264 15.0 (19.0), 5760 x 1920 4.5 (6.2).  One CTA per SM with twice the ring is up to 20 % slower (its eight
+// warps do not keep up), four with half of it as fast but 15 % slower at K = 11264.
+constexpr int kRingBytes = 48 * 1024, kStreamCtas = 2;
+// Four CTAs fit an SM and no fifth: where a kernel starts beside others, none of its SMs gets more than two extra.
+constexpr int kStreamShared = 54 * 1024;
+constexpr int kStreamRows = (kStreamShared - kRingBytes) / (kWarps * static_cast<int>(sizeof(float)));  // per CTA
+
+// kUnit: pieces per thread that are copied and waited for at a time, whole rows (kRowsPerStage of kChunks pieces) or, of
+// long rows, single pieces.
+template <bool kFp8, class X, int kChunks, int kRowsPerStage, int kUnit>
+__global__ void __launch_bounds__(kThreads, kChunks >= 5 ? 2 : 3)
+gemv_stream_kernel(const GemvParams p) {
+  constexpr int kPer = kFp8 ? 16 : 8;  // elements per 16-byte piece
+  constexpr int kUnits = kRingBytes / (kUnit * kThreads * 16);
+  static_assert(kUnits >= 3 && (kUnit == 1 ? kRowsPerStage == 1 : kUnit == kRowsPerStage * kChunks), "ring");
+  extern __shared__ __align__(16) uint4 ring[];  // [kUnits][kUnit][kThreads]
+  float *const partial = reinterpret_cast<float *>(ring + kUnits * kUnit * kThreads);  // [rows][kWarps]
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const bool gated = p.gate_mode != 0, grouped = p.row_group != nullptr;
+  const int out_columns = gated ? p.N / 2 : p.N;
+  const auto share = [&](const unsigned int cta) {
+    return static_cast<int>(static_cast<unsigned long long>(out_columns) * cta / gridDim.x);
   };
-  if (p.out_f32 != nullptr) {
-    float *const slot = p.out_f32 + out_index * out_columns + column;
-    float value = total(local) * alpha;
-    if (p.bias_f32 != nullptr) value += p.bias_f32[column];
-    *slot = soft_cap(p.accumulate_f32 != 0 ? *slot + value : value, p.softcap);
-    return;
-  }
-  bf16 *const out_row = p.out + out_index * out_columns;
-  if (p.gate_mode >= kGateRelu) {
-    float value = total(2 * local) * alpha, up = total(2 * local + 1) * alpha;
-    if (p.bias_f32 != nullptr) {
-      const int row = (column / 128) * 256 + column % 128;
-      value += p.bias_f32[row];
-      up += p.bias_f32[row + 128];
+  const int column0 = share(blockIdx.x), columns = share(blockIdx.x + 1) - column0;
+  const int rows = gated ? 2 * columns : columns;  // gated: all first rows, then their partners
+  const int groups = (rows + kRowsPerStage - 1) / kRowsPerStage;
+  const std::size_t row_bytes = static_cast<std::size_t>(p.K) * (kFp8 ? 1 : 2);
+  // the thread's pieces of a row: piece0 + 32 c, the warps' shares side by side
+  const int pieces = p.K / kPer, slice = (pieces + kWarps - 1) / kWarps;
+  const int piece0 = warp * slice + lane, piece_end = min(pieces, (warp + 1) * slice);
+  const unsigned char *weights = static_cast<const unsigned char *>(p.w) + static_cast<std::size_t>(piece0) * 16;
+  const auto source_of = [&](const int row) {
+    unsigned int weight_row = column0 + row;
+    if (gated) {
+      const bool second = row >= columns;
+      weight_row -= second ? columns : 0;
+      weight_row += (weight_row & ~127U) + (second ? 128U : 0U);
     }
-    out_row[column] = f2bf(gated_value(p.gate_mode, p.gate_limit, value, up));
-  } else if (gated) {
-    const float first = total(2 * local) * p.alpha, second = rbf(total(2 * local + 1) * p.alpha);
-    const float activated = p.gate_mode == 2 ? bf2f(gelu_round_small(first)) : rbf(first);
-    out_row[column] = f2bf(activated * second);
+    return weights + static_cast<std::size_t>(weight_row) * row_bytes;
+  };
+  const auto copy = [&](const int unit, const int piece, const unsigned char *const source, const int c) {
+    if (piece0 + 32 * c < piece_end)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<std::uint32_t>(
+                       __cvta_generic_to_shared(ring + (unit * kUnit + piece) * kThreads + tid))),
+                   "l"(source + 512 * c)
+                   : "memory");
+  };
+  int next_row = 0, next_chunk = 0;  // what the next unit holds
+  const auto fetch = [&](const int unit) {
+    if constexpr (kUnit == 1) {
+      if (next_row < rows) copy(unit, 0, source_of(next_row), next_chunk);
+      if (++next_chunk == kChunks) next_chunk = 0, ++next_row;
+    } else {
+#pragma unroll
+      for (int r = 0; r < kRowsPerStage; ++r) {
+        if (next_row + r < rows) {
+          const unsigned char *const source = source_of(next_row + r);
+#pragma unroll
+          for (int c = 0; c < kChunks; ++c) copy(unit, r * kChunks + c, source, c);
+        }
+      }
+      next_row += kRowsPerStage;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // pieces past the thread's share stay zero, on both sides of the product (single pieces: their slots change, so they
+  // are skipped instead)
+  if constexpr (kUnit != 1) {
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c)
+      if (piece0 + 32 * c >= piece_end)
+        for (int i = 0; i < kUnits * kRowsPerStage; ++i) ring[(i * kChunks + c) * kThreads + tid] = make_uint4(0U, 0U, 0U, 0U);
+  }
+  const auto fill = [&] {
+#pragma unroll
+    for (int unit = 0; unit < kUnits; ++unit) fetch(unit);
+  };
+  const X *x = static_cast<const X *>(p.x);
+  if (grouped) {
+    // which weights these are is a result of the kernel in front, or of one further back
+    const int *row_group = p.row_group;
+    if (!p.row_group_settled) wait_for_producers(x, row_group);
+    weights += static_cast<std::size_t>(__ldcg(row_group + blockIdx.y)) * p.N * row_bytes;
+    fill();
+    release_dependents();
+    if (p.row_group_settled) wait_for_producers(x);
+    x += static_cast<std::size_t>(blockIdx.y / p.row_fanout) * p.K;
   } else {
-    float value = total(local) * alpha;
-    if (p.bias_mode == 1) value += bf2f(p.bias[column]);
-    value = rbf(value);
-    if (p.bias_mode == 2) value = rbf(value + bf2f(p.bias[column]));
-    if (p.residual != nullptr)
-      value = rbf(value + bf2f(p.residual[static_cast<std::size_t>(r) * out_columns + column]));
-    out_row[column] = f2bf(value);
+    fill();
+    release_dependents();
+    wait_for_producers(x);
+  }
+  float xv[kChunks][kPer];
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    if (piece0 + 32 * c < piece_end) {
+      const X *const source = x + static_cast<std::size_t>(piece0 + 32 * c) * kPer;
+      if constexpr (std::is_same_v<X, float>) load_floats<8>(source, xv[c]);
+      else unpack16<kFp8>(*reinterpret_cast<const uint4 *>(source), xv[c]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) xv[c][i] = 0.0F;
+    }
+  }
+  int unit = 0;
+  const auto advance = [&] {
+    fetch(unit);
+    unit = unit + 1 == kUnits ? 0 : unit + 1;
+  };
+  const auto dot = [&](const int piece, const int c) {
+    float wv[kPer], sum = 0.0F;
+    unpack16<kFp8>(ring[(unit * kUnit + piece) * kThreads + tid], wv);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) sum = fmaf(xv[c][i], wv[i], sum);
+    return sum;
+  };
+  for (int group = 0; group < groups; ++group) {
+    float sum[kRowsPerStage];
+    if constexpr (kUnit == 1) {
+      float part[kChunks];
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kUnits - 1) : "memory");
+        part[c] = piece0 + 32 * c < piece_end ? dot(0, c) : 0.0F;
+        advance();
+      }
+      sum[0] = part[0];
+#pragma unroll
+      for (int c = 1; c < kChunks; ++c) sum[0] += part[c];
+    } else {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kUnits - 1) : "memory");
+#pragma unroll
+      for (int r = 0; r < kRowsPerStage; ++r) {
+        sum[r] = dot(r * kChunks, 0);
+#pragma unroll
+        for (int c = 1; c < kChunks; ++c) sum[r] += dot(r * kChunks + c, c);
+      }
+      advance();
+    }
+    // halves of the warp keep half of the rows each until one is left per lane
+    int row = group * kRowsPerStage, offset = 16;
+#pragma unroll
+    for (int held = kRowsPerStage; held > 1; held /= 2, offset /= 2) {
+      const bool upper = (lane & offset) != 0;
+      row += upper ? held / 2 : 0;
+#pragma unroll
+      for (int r = 0; r < held / 2; ++r) {
+        const float keep = upper ? sum[r + held / 2] : sum[r], give = upper ? sum[r] : sum[r + held / 2];
+        sum[r] = keep + __shfl_xor_sync(0xffffffffU, give, offset);
+      }
+    }
+#pragma unroll
+    for (int step = 16 / kRowsPerStage; step > 0; step /= 2) sum[0] += __shfl_xor_sync(0xffffffffU, sum[0], step);
+    if (lane % (32 / kRowsPerStage) == 0 && row < rows) partial[row * kWarps + warp] = sum[0];
+  }
+  __syncthreads();
+  const float alpha = p.row_scale != nullptr ? p.alpha * p.row_scale[blockIdx.y] : p.alpha;
+  for (int local = tid; local < columns; local += kThreads)
+    finish_column(p, 0, blockIdx.y, out_columns, column0 + local, alpha, local,
+                  [&](const int index) {  // (of a gated pair: 2 local, 2 local + 1)
+                    const int row = gated ? (index & 1) * columns + index / 2 : index;
+                    const float4 a = reinterpret_cast<const float4 *>(partial)[2 * row],
+                                 b = reinterpret_cast<const float4 *>(partial)[2 * row + 1];
+                    return ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
+                  });
+}
+
+// CTAs across the columns of each of `rows` output rows: together about kStreamCtas per SM.
+int stream_grid(const int out_columns, const int rows) {
+  const int wanted = std::max(1, kStreamCtas * kSmCount / rows);
+  return std::min(out_columns, wanted);
+}
+// Sizes that the one-row kernel has registers (K) and partial sums (N) for.
+template <bool kFp8>
+bool stream_applicable(const GemvParams &p) {
+  const int out_columns = p.gate_mode != 0 ? p.N / 2 : p.N, grid = stream_grid(out_columns, p.rows);
+  return p.K <= (kFp8 ? 6 * 16 : 8 * 8) * kWarps * 32 &&
+         ((out_columns - 1) / grid + 1) * (p.gate_mode != 0 ? 2 : 1) <= kStreamRows;
+}
+
+// One row, or grouped rows with a weight each.
+template <bool kFp8, class X>
+int launch_stream(const GemvParams &p, cudaStream_t stream) {
+  constexpr int kPer = kFp8 ? 16 : 8;
+  const int pieces = p.K / kPer, chunks = ((pieces + kWarps - 1) / kWarps + 31) / 32;
+  const dim3 grid(static_cast<unsigned int>(stream_grid(p.gate_mode != 0 ? p.N / 2 : p.N, p.rows)),
+                  static_cast<unsigned int>(p.rows));
+  const auto launch = [&](auto chunk_count, auto stage_rows) {
+    constexpr int kC = decltype(chunk_count)::value, kR = decltype(stage_rows)::value;
+    const auto kernel = gemv_stream_kernel<kFp8, X, kC, kR, kC >= 4 ? 1 : kC * kR>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamShared) != cudaSuccess)
+      return fail(kCuda, "cannot raise the shared-memory limit of the one-row projection kernel");
+    return launch_dependent("one-row projection kernel", kernel, grid, kThreads, kStreamShared, stream, p.dependent_launch != 0,
+                            1, p);
+  };
+  using std::integral_constant;
+  switch (chunks) {
+    case 1: return launch(integral_constant<int, 1>{}, integral_constant<int, 4>{});
+    case 2: return launch(integral_constant<int, 2>{}, integral_constant<int, 2>{});
+    case 3: return launch(integral_constant<int, 3>{}, integral_constant<int, 1>{});
+    case 4: return launch(integral_constant<int, 4>{}, integral_constant<int, 1>{});
+    case 5: return launch(integral_constant<int, 5>{}, integral_constant<int, 1>{});
+    case 6: return launch(integral_constant<int, 6>{}, integral_constant<int, 1>{});
+    default:
+      if constexpr (!kFp8) return launch(integral_constant<int, 8>{}, integral_constant<int, 1>{});
+      return fail(kInternal, "one-row projection kernel without registers for this K");
   }
 }
 
-// Four weight rows per CTA measured best at every width of the 7B and 40B
-// shapes (one row, BF16: 2.7 TB/s at 4096 x 4096, 5.3 TB/s at 22528 x 4096, with four
-// 16-byte loads per weight row in flight per thread);
-// a gated projection then produces two output columns per CTA.
+// 2..8 rows, sizes beyond the kernel above: four weight rows per CTA; a gated projection then produces two output columns
+// per CTA.
 constexpr int kColumnsPerCta = 4;
 
 template <bool kFp8>
 int launch_gemv(const GemvParams &p, cudaStream_t stream) {
+  if ((p.rows == 1 || p.row_group != nullptr) && stream_applicable<kFp8>(p))
+    return launch_stream<kFp8, std::conditional_t<kFp8, std::uint8_t, bf16>>(p, stream);
   const int out_columns = p.gate_mode != 0 ? p.N / 2 : p.N;
   const int per_cta = p.gate_mode != 0 ? kColumnsPerCta / 2 : kColumnsPerCta;
-  const unsigned int grid = static_cast<unsigned int>((out_columns + per_cta - 1) / per_cta);
-  if (p.row_group != nullptr || (p.rows == 1 && p.dependent_launch != 0)) {
-    const unsigned int rows = p.row_group != nullptr ? static_cast<unsigned int>(p.rows) : 1U;
-    GemvParams q = p;
-    q.rows = 1;
-    cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t config{};
-    config.gridDim = dim3(grid, rows);
-    config.blockDim = dim3(kThreads);
-    config.dynamicSmemBytes = 0;
-    config.stream = stream;
-    config.attrs = &attribute;
-    config.numAttrs = p.dependent_launch != 0 ? 1 : 0;
-    if (cudaLaunchKernelEx(&config, gemv_kernel<kFp8, 1, kColumnsPerCta>, q) != cudaSuccess)
-      return fail(kCuda, "cannot launch the small-batch projection kernel");
-  } else if (p.rows == 1)
-    gemv_kernel<kFp8, 1, kColumnsPerCta><<<grid, kThreads, 0, stream>>>(p);
-  else if (p.rows <= 2)
-    gemv_kernel<kFp8, 2, kColumnsPerCta><<<grid, kThreads, 0, stream>>>(p);
-  else if (p.rows <= 4)
-    gemv_kernel<kFp8, 4, kColumnsPerCta><<<grid, kThreads, 0, stream>>>(p);
-  else
-    gemv_kernel<kFp8, 8, kColumnsPerCta><<<grid, kThreads, 0, stream>>>(p);
-  return check_launch("small-batch projection kernel");
+  const dim3 grid(static_cast<unsigned int>((out_columns + per_cta - 1) / per_cta),
+                  p.row_group != nullptr ? static_cast<unsigned int>(p.rows) : 1U);
+  GemvParams q = p;
+  if (p.row_group != nullptr) q.rows = 1;
+  const auto kernel = q.rows == 1   ? gemv_kernel<kFp8, 1, kColumnsPerCta>
+                      : q.rows <= 2 ? gemv_kernel<kFp8, 2, kColumnsPerCta>
+                      : q.rows <= 4 ? gemv_kernel<kFp8, 4, kColumnsPerCta>
+                                    : gemv_kernel<kFp8, 8, kColumnsPerCta>;
+  return launch_dependent("small-batch projection kernel", kernel, grid, kThreads, 0, stream, p.dependent_launch != 0, 1, q);
 }
 
 }  // namespace
@@ -259,6 +474,34 @@ bool small_batch_linear_applicable(const LinearArgs &a) {
          (reinterpret_cast<std::uintptr_t>(a.weight) & 15U) == 0 &&
          a.out_features <= 0x7fffffffU && a.in_features <= 0x7fffffffU &&
          (a.gate_mode == 0 || a.out_features % 256 == 0);
+}
+
+bool one_row_linear_f32_applicable(const LinearF32Args &a) {
+  if (a.rows != 1 || a.row_group != nullptr || a.tile_group != nullptr || a.in_features % 8 != 0 || !aligned16(a.input) ||
+      !aligned16(a.weight) || a.in_features > 0x7fffffffU || a.out_features > 0x7fffffffU)
+    return false;
+  GemvParams p{};
+  p.rows = 1;
+  p.K = static_cast<int>(a.in_features);
+  p.N = static_cast<int>(a.out_features);
+  return stream_applicable<false>(p);
+}
+
+int one_row_linear_f32(const LinearF32Args &a, cudaStream_t stream) {
+  GemvParams p{};
+  p.x = a.input;
+  p.w = a.weight;
+  p.out_f32 = a.output;
+  p.bias_f32 = a.bias;
+  p.accumulate_f32 = a.accumulate ? 1 : 0;
+  p.rows = 1;
+  p.K = static_cast<int>(a.in_features);
+  p.N = static_cast<int>(a.out_features);
+  p.alpha = a.alpha;
+  p.softcap = a.softcap;
+  p.row_scale = a.row_scale;
+  p.dependent_launch = a.dependent_launch ? 1 : 0;
+  return a.input_type == Activation::kBf16 ? launch_stream<false, bf16>(p, stream) : launch_stream<false, float>(p, stream);
 }
 
 int small_batch_linear(const LinearArgs &a, cudaStream_t stream) {
@@ -282,6 +525,7 @@ int small_batch_linear(const LinearArgs &a, cudaStream_t stream) {
   p.softcap = a.softcap;
   p.row_group = a.row_group;
   p.row_fanout = static_cast<int>(a.row_fanout);
+  p.row_group_settled = a.row_group_settled && a.dependent_launch ? 1 : 0;
   p.row_scale = a.row_scale;
   return a.operand_type == OperandType::kE4m3 ? launch_gemv<true>(p, stream)
                                               : launch_gemv<false>(p, stream);

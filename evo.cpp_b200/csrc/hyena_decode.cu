@@ -40,9 +40,8 @@ __device__ __forceinline__ float filter_tap(const void *filter, const bool is_f3
 template <bool kModal>
 __global__ void __launch_bounds__(kThreads)
 mixer_decode_kernel(const Params p) {
-  // lets a one-row projection launched with programmatic stream serialisation start (and fetch its
-  // weights) under this kernel; it still waits for this grid to finish before it reads the result
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers();
+  release_dependents();
   const int channel = (blockIdx.x * kThreads + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   if (channel >= p.width) return;
@@ -152,10 +151,8 @@ int hyena_decode_mixer(const DecodeMixerArgs &a, cudaStream_t stream) {
   p.cross_correlation = a.cross_correlation;
   const unsigned int grid = ceil_div_u(a.width * 32, kThreads);
   if (modal)
-    mixer_decode_kernel<true><<<grid, kThreads, 0, stream>>>(p);
-  else
-    mixer_decode_kernel<false><<<grid, kThreads, 0, stream>>>(p);
-  return check_launch("decode mixer kernel");
+    return launch_dependent("decode mixer kernel", mixer_decode_kernel<true>, dim3(grid), kThreads, 0, stream, true, 1, p);
+  return launch_dependent("decode mixer kernel", mixer_decode_kernel<false>, dim3(grid), kThreads, 0, stream, true, 1, p);
 }
 
 }  // namespace evob

@@ -232,6 +232,8 @@ constexpr int kHistorySlotsPerLane = 8;  // cache_size <= 256
 __global__ void __launch_bounds__(kThreads)
 history_update_kernel(const bf16 *__restrict__ input, float *__restrict__ cache, const int length,
                       const int channels, const int cache_size, const bool fresh) {
+  wait_for_producers(input, cache);
+  release_dependents();
   const int channel = (blockIdx.x * kThreads + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   if (channel >= channels) return;
@@ -336,6 +338,8 @@ fir_rows_warp_kernel(const bf16 *__restrict__ input, const void *__restrict__ fi
                      bf16 *__restrict__ output, const std::size_t length, const std::size_t channels,
                      const std::size_t channels_per_group, const int taps, const int cached,
                      const bool cross_correlation) {
+  wait_for_producers(input, cache, output);
+  release_dependents();
   const std::size_t item = (static_cast<std::size_t>(blockIdx.x) * kThreads + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   if (item >= length * channels) return;
@@ -513,10 +517,9 @@ static int update_history(const void *input, float *cache, const std::size_t len
                           const std::size_t cache_size, const bool fresh, cudaStream_t stream) {
   if (cache_size > 32 * kHistorySlotsPerLane || channels > 0x3ffffffU || length > 0x7fffff00U)
     return fail(kInvalidArgument, "FIR history is longer than 256 entries or the tensor is too large");
-  history_update_kernel<<<ceil_div_u(channels * 32, kThreads), kThreads, 0, stream>>>(
-      static_cast<const bf16 *>(input), cache, static_cast<int>(length), static_cast<int>(channels),
-      static_cast<int>(cache_size), fresh);
-  return check_launch("FIR history kernel");
+  return launch_dependent("FIR history kernel", history_update_kernel, dim3(ceil_div_u(channels * 32, kThreads)), kThreads, 0,
+                          stream, true, 1, static_cast<const bf16 *>(input), cache, static_cast<int>(length),
+                          static_cast<int>(channels), static_cast<int>(cache_size), fresh);
 }
 
 int fill_fir_cache(const void *input, float *cache, const std::size_t length,
@@ -572,11 +575,11 @@ int fir_step(const void *input, const void *filter, const bool filter_is_f32,
   }
   const std::size_t warps = length * channels;
   if (warps > 0x3ffffffU || taps > 0x7fffffffU) return fail(kInvalidArgument, "FIR step is too large");
-  fir_rows_warp_kernel<<<ceil_div_u(warps * 32, kThreads), kThreads, 0, stream>>>(
-      static_cast<const bf16 *>(input), filter, filter_is_f32, static_cast<const bf16 *>(bias), multiply_bias,
-      cache, static_cast<bf16 *>(output), length, channels, channels / groups, static_cast<int>(taps),
-      static_cast<int>(cache_length), cross_correlation);
-  const int status = check_launch("FIR step kernel");
+  const int status =
+      launch_dependent("FIR step kernel", fir_rows_warp_kernel, dim3(ceil_div_u(warps * 32, kThreads)), kThreads, 0, stream, true, 1,
+                       static_cast<const bf16 *>(input), filter, filter_is_f32, static_cast<const bf16 *>(bias), multiply_bias,
+                       cache, static_cast<bf16 *>(output), length, channels, channels / groups, static_cast<int>(taps),
+                       static_cast<int>(cache_length), cross_correlation);
   if (status != kOk) return status;
   return update_history(input, cache, length, channels, taps - 1, false, stream);
 }

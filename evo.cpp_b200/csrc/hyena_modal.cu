@@ -54,6 +54,8 @@ modal_decode_warp_kernel(const bf16 *__restrict__ x2, const bf16 *__restrict__ x
                          const bf16 *__restrict__ direct, const float *__restrict__ log_poles,
                          const float *__restrict__ residues, float *__restrict__ state, bf16 *__restrict__ pregate,
                          bf16 *__restrict__ output, const int width, const int modes) {
+  wait_for_producers(x2, x1, value, state, pregate, output);
+  release_dependents();
   const int channel = (blockIdx.x * kDecodeThreads + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   if (channel >= width) return;
@@ -790,13 +792,11 @@ int modal_decode(const void *x2, const void *x1, const void *value,
       output == nullptr || width == 0 || modes == 0 || modes > 32)
     return fail(kInvalidArgument, "modal decode arguments are invalid");
   if (width > 0x3ffffffU) return fail(kInvalidArgument, "modal decode is too wide");
-  modal_decode_warp_kernel<<<ceil_div_u(width * 32, kDecodeThreads), kDecodeThreads, 0, stream>>>(
-      static_cast<const bf16 *>(x2), static_cast<const bf16 *>(x1),
-      static_cast<const bf16 *>(value), static_cast<const bf16 *>(direct),
-      log_poles, residues, state, static_cast<bf16 *>(pregate),
-      static_cast<bf16 *>(output), static_cast<int>(width),
-      static_cast<int>(modes));
-  return check_launch("modal decode kernel");
+  return launch_dependent("modal decode kernel", modal_decode_warp_kernel, dim3(ceil_div_u(width * 32, kDecodeThreads)),
+                          kDecodeThreads, 0, stream, true, 1, static_cast<const bf16 *>(x2), static_cast<const bf16 *>(x1),
+                          static_cast<const bf16 *>(value), static_cast<const bf16 *>(direct), log_poles, residues, state,
+                          static_cast<bf16 *>(pregate), static_cast<bf16 *>(output), static_cast<int>(width),
+                          static_cast<int>(modes));
 }
 
 int modal_taps(const void *gated, const float *log_poles, const float *residues, const std::size_t length,

@@ -19,8 +19,8 @@ constexpr int kWarps = kThreads / 32;
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 latent_norm_vector_kernel(const T *__restrict__ projection, const LatentNormArgs a) {
-  // a one-row projection launched with programmatic stream serialisation may start under this kernel
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(projection);
+  release_dependents();
   // a warp per (row, latent): neither waits for the rest of the CTA
   const std::size_t item = static_cast<std::size_t>(blockIdx.x) * kWarps + threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
@@ -74,8 +74,8 @@ latent_norm_vector_kernel(const T *__restrict__ projection, const LatentNormArgs
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 latent_norm_kernel(const T *__restrict__ projection, const LatentNormArgs a) {
-  // a one-row projection launched with programmatic stream serialisation may start under this kernel
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(projection);
+  release_dependents();
   __shared__ float scratch[kWarps];
   const std::size_t row = blockIdx.x;
   const bool is_query = blockIdx.y == 0;
@@ -109,6 +109,8 @@ template <typename T, int kVec, int kRows>
 __global__ void __launch_bounds__(kThreads)
 absorb_kernel(const T *__restrict__ query, const bf16 *__restrict__ key_up, T *__restrict__ absorbed, const int rows,
               const int heads, const int dim, const int rank) {
+  wait_for_producers(query, absorbed);
+  release_dependents();
   constexpr int kColumns = 8 * kVec;
   __shared__ float partial[kWarps][kRows][kColumns];
   const int head = blockIdx.x, part = threadIdx.x % 8, down = threadIdx.x / 8;
@@ -158,8 +160,8 @@ template <typename T, int kVec, int kRows>
 __global__ void __launch_bounds__(kThreads)
 expand_kernel(const T *__restrict__ mixed, const bf16 *__restrict__ value_up, T *__restrict__ output, const int rows,
               const int heads, const int value_dim, const int rank) {
-  // a one-row projection launched with programmatic stream serialisation may start under this kernel
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(mixed, output);
+  release_dependents();
   const int head = blockIdx.x, column = blockIdx.y * kWarps + threadIdx.x / 32, lane = threadIdx.x % 32;
   if (column >= value_dim) return;
   const bf16 *const w = value_up + (static_cast<std::size_t>(head) * value_dim + column) * rank;
@@ -243,6 +245,8 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const std::uint32_t (&a)
 template <int kBlocks>
 __global__ void __launch_bounds__(kThreads)
 latent_decode_kernel(const LatentDecodeParams p) {
+  wait_for_producers();
+  release_dependents();
   constexpr int kRank = 64 * kBlocks, kStride = latent_stride(kRank);
   extern __shared__ __align__(16) unsigned char latent_smem[];
   bf16 *const tiles = reinterpret_cast<bf16 *>(latent_smem);                    // [2][kTokens][kStride]
@@ -418,20 +422,8 @@ int launch_latent_decode(const LatentDecodeParams &p, const std::size_t rows, cu
   if (cudaFuncSetAttribute(latent_decode_kernel<kBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(kBytes)) != cudaSuccess)
     return fail(kCuda, "cannot raise the latent attention shared-memory limit");
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = kSplits;
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(kSplits, ceil_div_u(static_cast<std::size_t>(p.heads), kHeadGroup), static_cast<unsigned int>(rows));
-  config.blockDim = dim3(kThreads);
-  config.dynamicSmemBytes = kBytes;
-  config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  if (cudaLaunchKernelEx(&config, latent_decode_kernel<kBlocks>, p) != cudaSuccess)
-    return fail(kCuda, std::string("cannot launch the latent attention kernel: ") + cudaGetErrorString(cudaGetLastError()));
-  return check_launch("latent attention kernel");
+  const dim3 grid(kSplits, ceil_div_u(static_cast<std::size_t>(p.heads), kHeadGroup), static_cast<unsigned int>(rows));
+  return launch_dependent("latent attention kernel", latent_decode_kernel<kBlocks>, grid, kThreads, kBytes, stream, true, kSplits, p);
 }
 
 // f(T{}, kVec constant, kRows constant) for an activation type, vector width and a bound on the rows.
@@ -470,17 +462,17 @@ int latent_norm_append(const LatentNormArgs &a, cudaStream_t stream) {
       aligned16(a.cache)) {
     const unsigned int ctas = ceil_div_u(2 * a.rows, kWarps);
     if (a.type == Activation::kBf16)
-      latent_norm_vector_kernel<<<ctas, kThreads, 0, stream>>>(static_cast<const bf16 *>(a.projection), a);
-    else
-      latent_norm_vector_kernel<<<ctas, kThreads, 0, stream>>>(static_cast<const float *>(a.projection), a);
-    return check_launch("latent norm kernel");
+      return launch_dependent("latent norm kernel", latent_norm_vector_kernel<bf16>, dim3(ctas), kThreads, 0, stream, true, 1,
+                              static_cast<const bf16 *>(a.projection), a);
+    return launch_dependent("latent norm kernel", latent_norm_vector_kernel<float>, dim3(ctas), kThreads, 0, stream, true, 1,
+                            static_cast<const float *>(a.projection), a);
   }
   const dim3 grid(static_cast<unsigned int>(a.rows), 2);
   if (a.type == Activation::kBf16)
-    latent_norm_kernel<<<grid, kThreads, 0, stream>>>(static_cast<const bf16 *>(a.projection), a);
-  else
-    latent_norm_kernel<<<grid, kThreads, 0, stream>>>(static_cast<const float *>(a.projection), a);
-  return check_launch("latent norm kernel");
+    return launch_dependent("latent norm kernel", latent_norm_kernel<bf16>, grid, kThreads, 0, stream, true, 1,
+                            static_cast<const bf16 *>(a.projection), a);
+  return launch_dependent("latent norm kernel", latent_norm_kernel<float>, grid, kThreads, 0, stream, true, 1,
+                          static_cast<const float *>(a.projection), a);
 }
 
 int absorb_queries(const void *query, const void *key_up, const std::size_t rows, const std::size_t heads,
@@ -490,15 +482,17 @@ int absorb_queries(const void *query, const void *key_up, const std::size_t rows
     return fail(kInvalidArgument, "query absorption arguments are invalid");
   if (rows == 0) return kOk;
   const bool vector = latent_rank % 8 == 0 && aligned16(key_up);
+  int status = kOk;
   dispatch(type, vector, rows, [&](auto tag, auto vec, auto bound) {
     using T = decltype(tag);
     constexpr int kVec = decltype(vec)::value;
     const dim3 grid(static_cast<unsigned int>(heads), ceil_div_u(latent_rank, 8 * kVec));
-    absorb_kernel<T, kVec, decltype(bound)::value><<<grid, kThreads, 0, stream>>>(
-        static_cast<const T *>(query), static_cast<const bf16 *>(key_up), static_cast<T *>(absorbed),
-        static_cast<int>(rows), static_cast<int>(heads), static_cast<int>(dim), static_cast<int>(latent_rank));
+    status = launch_dependent("query absorption kernel", absorb_kernel<T, kVec, decltype(bound)::value>, grid, kThreads, 0, stream,
+                              true, 1, static_cast<const T *>(query), static_cast<const bf16 *>(key_up),
+                              static_cast<T *>(absorbed), static_cast<int>(rows), static_cast<int>(heads),
+                              static_cast<int>(dim), static_cast<int>(latent_rank));
   });
-  return check_launch("query absorption kernel");
+  return status;
 }
 
 int expand_values(const void *mixed, const void *value_up, const std::size_t rows, const std::size_t heads,
@@ -508,14 +502,16 @@ int expand_values(const void *mixed, const void *value_up, const std::size_t row
     return fail(kInvalidArgument, "value expansion arguments are invalid");
   if (rows == 0) return kOk;
   const bool vector = latent_rank % 8 == 0 && aligned16(mixed) && aligned16(value_up);
+  int status = kOk;
   dispatch(type, vector, rows, [&](auto tag, auto vec, auto bound) {
     using T = decltype(tag);
     const dim3 grid(static_cast<unsigned int>(heads), ceil_div_u(value_dim, kWarps));
-    expand_kernel<T, decltype(vec)::value, decltype(bound)::value><<<grid, kThreads, 0, stream>>>(
-        static_cast<const T *>(mixed), static_cast<const bf16 *>(value_up), static_cast<T *>(output),
-        static_cast<int>(rows), static_cast<int>(heads), static_cast<int>(value_dim), static_cast<int>(latent_rank));
+    status = launch_dependent("value expansion kernel", expand_kernel<T, decltype(vec)::value, decltype(bound)::value>, grid,
+                              kThreads, 0, stream, true, 1, static_cast<const T *>(mixed), static_cast<const bf16 *>(value_up),
+                              static_cast<T *>(output), static_cast<int>(rows), static_cast<int>(heads),
+                              static_cast<int>(value_dim), static_cast<int>(latent_rank));
   });
-  return check_launch("value expansion kernel");
+  return status;
 }
 
 bool latent_decode_applicable(const WindowAttentionArgs &a) {

@@ -31,12 +31,7 @@ int quantize_rows(const void *input, std::size_t rows, std::size_t width, void *
 int amax_bf16(const void *input, std::size_t elements, unsigned int *result_bits, cudaStream_t stream);
 int rms_norm(const void *input, const float *scale, std::size_t rows,
              std::size_t width, float epsilon, void *output, void *codes,
-             float quant_scale, cudaStream_t stream,
-             // few rows only: launch with programmatic stream serialisation (the gains are fetched under the
-             // kernel in front, the row after it has finished).  The decode step does not ask for it: with the
-             // norm released early the projection behind it starts two kernels ahead and its waiting CTAs take
-             // SM slots from the projection still running (2.63 against 2.59 ms per token).
-             bool dependent_launch = false);
+             float quant_scale, cudaStream_t stream);
 int gelu(const void *input, void *output, std::size_t elements,
          cudaStream_t stream);
 int gate(const void *first, const void *second, void *output,
@@ -80,9 +75,9 @@ struct LinearArgs {
   // is multiplied by alpha * row_scale[r] (dynamic per-row activation quantisation).
   const float *row_scale = nullptr;
   // One-row weight streams only: launch with programmatic stream serialisation, so that the kernel may
-  // start (and pull its weights into L2) while the kernel in front of it in the stream is still running;
-  // it waits for that kernel before it reads the input.  The caller promises that nothing this launch
-  // reads besides `weight` is still being written by work further back than the previous kernel.
+  // start (and fetch the first of its weights) while the kernel in front of it in the stream is still running;
+  // it waits for that kernel before it reads the input.  The caller promises that `weight` is not being written
+  // by earlier work in the stream.
   bool dependent_launch = false;
   int bias_mode = 0;   // 0 none, 1 fused F32 add, 2 separate BF16-rounded add
   // over 128-column halves (row-interleaved weights): 0 none, 1 a*b, 2 gelu(a)*b, 3 max(a, 0)*b, 4 clamped SwiGLU
@@ -118,6 +113,9 @@ struct LinearArgs {
   std::size_t tile_rows = 128;
   const int *row_group = nullptr;
   std::size_t row_fanout = 1;
+  // With dependent_launch: the kernel in front of this one is linear() with the same row_group, so row_group itself comes
+  // from work further back (which has completed when a grouped projection lets the kernel behind it start).
+  bool row_group_settled = false;
 };
 // Whether linear() takes the tile form of grouped weights at these sizes.
 bool grouped_linear_applicable(const LinearArgs &args);

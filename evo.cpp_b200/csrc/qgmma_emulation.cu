@@ -335,6 +335,7 @@ qgmma_emulation_rows_kernel(const std::uint8_t *__restrict__ input_codes,
                             const std::uint8_t *__restrict__ weight_codes,
                             bf16 *__restrict__ output, const std::size_t in_features,
                             const std::size_t out_features, const float output_scale) {
+  release_dependents();
   constexpr int kCodes = kGroup / kLanes, kWords = kCodes / 4;
   extern __shared__ __align__(16) unsigned char shared[];
   float *const x_magnitude = reinterpret_cast<float *>(shared);                                // [kRows][in_features]
@@ -511,6 +512,8 @@ int e4m3_emulated_gemm(const void *input_codes, const void *weight_codes,
                                    : (two_lanes ? qgmma_emulation_rows_kernel<2, 2, 8> : qgmma_emulation_rows_kernel<2, 4, 16>);
     const int status = allow_shared_memory(kernel, row_bytes);
     if (status != kOk) return status;
+    // (not a dependent launch: started beside a projection that still runs, its CTAs crowd on the SMs that are free
+    // first, and this kernel is bound by its arithmetic: 85 us against 41)
     kernel<<<blocks, kRowKernelThreads, row_bytes, stream>>>(
         static_cast<const std::uint8_t *>(input_codes),
         static_cast<const std::uint8_t *>(weight_codes), static_cast<bf16 *>(output),

@@ -623,8 +623,8 @@ decode_kernel(const T *__restrict__ projection, T *const history, const float *_
               const float *__restrict__ decay_rate, const float *__restrict__ decay_shift,
               const float *__restrict__ decay_weight, const float *__restrict__ decay_bias,
               const float *__restrict__ gain, float *const state, T *__restrict__ output, const DecodeParams p) {
-  // a one-row projection launched with programmatic stream serialisation may start under this kernel
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_for_producers(projection, output);
+  release_dependents();
   __shared__ float key[kDecoderMaxHeadDim], query[kDecoderMaxHeadDim], alpha[kDecoderMaxHeadDim];
   __shared__ float partial[2][kDecodeWarps][32], scratch[kDecodeWarps];
   __shared__ float squares[kDecodeMaxGroup];  // this CTA's part of every head's sum of squares
@@ -773,24 +773,12 @@ int launch_decode(const RecurrentArgs &a, cudaStream_t stream) {
   p.inverse_tau = 1.0F / a.tau;
   p.epsilon = a.epsilon;
   p.fresh = a.fresh ? 1 : 0;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = kDecodeRanks;
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(kDecodeRanks, static_cast<unsigned int>(kDelta ? a.kv_heads : a.heads));
-  config.blockDim = dim3(kDecodeThreads);
   const std::size_t columns = (kDelta ? a.heads / a.kv_heads : 1) * a.value_dim;
-  config.dynamicSmemBytes = (columns + kDecodeRanks - 1) / kDecodeRanks * sizeof(float);
-  config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  if (cudaLaunchKernelEx(&config, decode_kernel<kDelta, T>, static_cast<const T *>(a.projection),
-                         static_cast<T *>(a.conv_history), a.conv, a.decay_rate, a.decay_shift, a.decay_weight,
-                         a.decay_bias, a.output_norm, a.state, static_cast<T *>(a.output), p) != cudaSuccess)
-    return fail(kCuda, std::string("cannot launch the recurrent decode kernel: ") +
-                           cudaGetErrorString(cudaGetLastError()));
-  return check_launch("recurrent decode kernel");
+  return launch_dependent("recurrent decode kernel", decode_kernel<kDelta, T>,
+                          dim3(kDecodeRanks, static_cast<unsigned int>(kDelta ? a.kv_heads : a.heads)), kDecodeThreads,
+                          (columns + kDecodeRanks - 1) / kDecodeRanks * sizeof(float), stream, true, kDecodeRanks,
+                          static_cast<const T *>(a.projection), static_cast<T *>(a.conv_history), a.conv, a.decay_rate,
+                          a.decay_shift, a.decay_weight, a.decay_bias, a.output_norm, a.state, static_cast<T *>(a.output), p);
 }
 
 template <bool kDelta, int kElements, typename T>

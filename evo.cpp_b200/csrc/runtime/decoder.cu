@@ -185,6 +185,7 @@ int Context::decoder_linear(Stage &s, const DecoderProduct &p) {
     a.bias = p.bias;
     a.alpha = p.alpha;
     a.softcap = p.softcap;
+    a.dependent_launch = decode_dependent_launch_ && p.rows == 1;
     return linear_f32(a, s.stream);
   }
   LinearArgs a;
@@ -479,6 +480,7 @@ int Context::expert_feed_forward(Stage &s, const std::size_t i, const std::size_
     grouping(a, false);
     a.groups = b.experts;
     a.dependent_launch = decode_dependent_launch_ && rows == 1;
+    a.row_group_settled = pairwise && fused;
     a.output = s.expert_out;
     EVOB_OP(kCatGemmGrouped, linear(a, stream));
     norm->input_type = Activation::kBf16;

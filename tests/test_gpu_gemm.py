@@ -220,3 +220,44 @@ def _check_split_k_gated(ops, rows, inner, hidden):
         assert bool(((split.float() - reference).abs() <= 0.05 + 0.02 * reference.abs()).all())
         assert bool(((split.float() - fused.float()).abs() <= 0.05 + 0.02 * fused.float().abs()).all())
         assert float((split != fused).float().mean()) < 0.05
+
+
+@pytest.mark.parametrize("columns", [1, 37, 256, 1184, 5000])
+@pytest.mark.parametrize("inner", [64, 264, 1920, 2056, 4104, 8448, 11264, 16384, 16392])
+def test_one_row_streams(ops, inner, columns):
+    """One row at the edges of the weight stream's split: fewer columns than CTAs, pieces of 8 (16) values that leave
+    lanes or whole warps without work, every number of pieces per thread, and an inner size beyond its registers.  A
+    result passes through at most 32 roundings (16 products, 8 pieces, 5 + 3 sums)."""
+    generator = torch.Generator("cuda").manual_seed(inner + columns)
+    x, w = (torch.randn(n, inner, device="cuda", generator=generator) for n in (1, columns))
+    xb, wb = x.bfloat16(), w.bfloat16()
+    base = torch.randn(1, columns, device="cuda", generator=generator)
+
+    def check(out, left, right, add):
+        left, right = left.double(), right.double()
+        bound = 32 * 2.0 ** -24 * (left.abs() @ right.abs().T + add.double().abs())
+        assert bool(((out.double() - (left @ right.T + add)).abs() <= bound).all())
+
+    out = base.clone()
+    ops.call("f32_linear", p(x), p(wb), 1, inner, columns, 1, p(out), stream())
+    check(out, x, wb, base)
+    work = torch.empty(1 << 20, device="cuda")
+    ops.call("bf16_linear_f32_result", p(xb), p(wb), 1, inner, columns, 0, p(work), work.numel() * 4, p(out), stream())
+    check(out, xb, wb, torch.zeros_like(base))
+    bits = torch.empty(1, columns, dtype=torch.bfloat16, device="cuda")
+    if inner % 16 == 0:
+        codes, weights = (t.to(torch.float8_e4m3fn) for t in (x, w))
+        ops.call("e4m3_codes_linear", p(codes.view(torch.uint8)), None, p(weights.view(torch.uint8)), None, None, 1, inner,
+                 columns, 1.0, 0, 0, p(bits), stream())
+        expected = codes.double() @ weights.double().T
+        bound = 2.0 ** -8 * expected.abs() + 32 * 2.0 ** -24 * (codes.double().abs() @ weights.double().abs().T)
+        assert bool(((bits.double() - expected).abs() <= bound).all())
+    if columns % 128 == 0:
+        pair = torch.randn(2 * columns, inner, device="cuda", generator=generator).bfloat16()
+        ops.call("bf16_gated_up_projection", p(xb), p(pair), 1, inner, columns, 0, p(bits), stream())
+        first, second = (xb.double() @ pair.view(-1, 2, 128, inner)[:, i].reshape(columns, inner).double().T for i in (0, 1))
+        # both factors and the product are rounded to BF16 (2^-8 each), behind F32 sums with the bound above
+        slack = 32 * 2.0 ** -24 * inner
+        bound = 3.1 * 2.0 ** -8 * (first * second).abs() + slack * (first.abs() + second.abs())
+        assert bool(((bits.double() - first * second).abs() <= bound).all())
+    ops.call("check_async_errors", stream())
