@@ -35,6 +35,17 @@ int poly_norm(const void *input, const float *coefficients, std::size_t rows, st
 // table[h, d] = r1[h] ln(1 + r2[h] d), d < distances.
 int distance_bias_table(const float *r1, const float *r2, std::size_t heads, std::size_t distances, float *table,
                         cudaStream_t stream);
+// An operator in front of a one-row projection, computed by the projection's own kernel: the row norm
+// rms_norm_residual() of an F32 input (values: gains), or poly_norm() of an input in the activation type (values: its
+// four coefficients).
+struct RowFront {
+  const float *values = nullptr;
+  float epsilon = 0.0F;
+  bool poly = false;
+};
+// gemv.cu: whether one row of these sizes and buffers takes it.
+bool row_front_applicable(const RowFront &front, const void *input, const void *weight, std::size_t in_features,
+                          std::size_t out_features);
 // [rows, in] (F32 or BF16) x BF16 [out, in]^T in F32 fused multiply-adds.  output = [output +] alpha *
 // row_scale[r] * product + bias, then softcap tanh(output / softcap) where softcap > 0.  Grouped weights
 // [groups, out, in]: see LinearArgs (row_group / row_fanout, or tile_group / tile_count / tile_rows).
@@ -52,6 +63,7 @@ struct LinearF32Args {
   const int *tile_group = nullptr, *tile_count = nullptr;
   std::size_t tile_rows = 128;
   bool dependent_launch = false;  // one row: as LinearArgs::dependent_launch
+  RowFront front;                 // one row
 };
 int linear_f32(const LinearF32Args &args, cudaStream_t stream);
 // gemv.cu: the weight-streaming kernel for one row, which linear_f32() uses where it applies.

@@ -587,6 +587,7 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
     return fail(kInvalidArgument, "F32 linear arguments are invalid");
   if (a.rows == 0) return kOk;
   if (one_row_linear_f32_applicable(a)) return one_row_linear_f32(a, stream);
+  if (a.front.values != nullptr) return fail(kUnsupported, "operators in front of a projection take one row");
   F32Params p{};
   p.weight = static_cast<const bf16 *>(a.weight);
   p.output = a.output;

@@ -1268,6 +1268,12 @@ int linear(const LinearArgs &args, cudaStream_t stream) {
   if (args.output_f32 != nullptr &&
       (fp8 || args.gate_mode != 0 || args.bias_mode != 0 || args.residual != nullptr))
     return fail(kInvalidArgument, "the F32-result mode takes BF16 operands and no BF16 epilogue");
+  if (args.front.values != nullptr)
+    return args.rows == 1 && !fp8 && args.row_group == nullptr && args.tile_group == nullptr &&
+                   args.weight_wrap_features == 0 && args.row_scale == nullptr && small_batch_linear_applicable(args) &&
+                   row_front_applicable(args.front, args.input, args.weight, args.in_features, args.out_features)
+               ? small_batch_linear(args, stream)
+               : fail(kUnsupported, "operators in front of a projection take one row of BF16 products");
   if (args.row_group != nullptr)
     return small_batch_linear_applicable(args) ? small_batch_linear(args, stream)
                                                : fail(kUnsupported, "grouped rows do not take these sizes");

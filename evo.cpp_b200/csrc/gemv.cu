@@ -40,6 +40,9 @@ struct GemvParams {
   int row_fanout;
   int row_group_settled;   // LinearArgs::row_group_settled
   const float *row_scale;  // grouped weights only
+  const float *front;      // RowFront::values
+  float epsilon;
+  bool poly_front;
 };
 
 template <bool kFp8>
@@ -240,9 +243,13 @@ constexpr int kRingBytes = 48 * 1024, kStreamCtas = 2;
 constexpr int kStreamShared = 54 * 1024;
 constexpr int kStreamRows = (kStreamShared - kRingBytes) / (kWarps * static_cast<int>(sizeof(float)));  // per CTA
 
+// What is done to x on the way in.  A norm's statistics are those of the whole row: every CTA takes them itself, which
+// costs it a barrier against a launch and a round trip through memory.
+enum class Front { kNone, kRms, kPoly };
+
 // kUnit: pieces per thread that are copied and waited for at a time, whole rows (kRowsPerStage of kChunks pieces) or, of
 // long rows, single pieces.
-template <bool kFp8, class X, int kChunks, int kRowsPerStage, int kUnit>
+template <bool kFp8, class X, Front kFront, int kChunks, int kRowsPerStage, int kUnit>
 __global__ void __launch_bounds__(kThreads, kChunks >= 5 ? 2 : 3)
 gemv_stream_kernel(const GemvParams p) {
   constexpr int kPer = kFp8 ? 16 : 8;  // elements per 16-byte piece
@@ -310,7 +317,8 @@ gemv_stream_kernel(const GemvParams p) {
 #pragma unroll
     for (int unit = 0; unit < kUnits; ++unit) fetch(unit);
   };
-  const X *x = static_cast<const X *>(p.x);
+  using Source = std::conditional_t<kFront == Front::kRms, float, X>;
+  const Source *x = static_cast<const Source *>(p.x);
   if (grouped) {
     // which weights these are is a result of the kernel in front, or of one further back
     const int *row_group = p.row_group;
@@ -329,12 +337,65 @@ gemv_stream_kernel(const GemvParams p) {
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     if (piece0 + 32 * c < piece_end) {
-      const X *const source = x + static_cast<std::size_t>(piece0 + 32 * c) * kPer;
-      if constexpr (std::is_same_v<X, float>) load_floats<8>(source, xv[c]);
+      const Source *const source = x + static_cast<std::size_t>(piece0 + 32 * c) * kPer;
+      if constexpr (std::is_same_v<Source, float>) load_floats<8>(source, xv[c]);
       else unpack16<kFp8>(*reinterpret_cast<const uint4 *>(source), xv[c]);
     } else {
 #pragma unroll
       for (int i = 0; i < kPer; ++i) xv[c][i] = 0.0F;
+    }
+  }
+  if constexpr (kFront != Front::kNone) {
+    __shared__ float scratch[3][kWarps];
+    constexpr int kSums = kFront == Front::kPoly ? 3 : 1;
+    float sums[3] = {0.0F, 0.0F, 0.0F};  // of squares, fourth and sixth powers
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const float v = xv[c][i], square = v * v;
+        if constexpr (kFront == Front::kPoly) {
+          sums[0] += square;
+          sums[1] = fmaf(square, square, sums[1]);
+          sums[2] = fmaf(square * square, square, sums[2]);
+        } else {
+          sums[0] = fmaf(v, v, sums[0]);
+        }
+      }
+#pragma unroll
+    for (int k = 0; k < kSums; ++k) {
+      sums[k] = warp_sum(sums[k]);
+      if (lane == 0) scratch[k][warp] = sums[k];
+    }
+    __syncthreads();
+    const float inverse_width = 1.0F / static_cast<float>(p.K);
+#pragma unroll
+    for (int k = 0; k < kSums; ++k) {
+      sums[k] = 0.0F;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) sums[k] += scratch[k][w];
+      sums[k] = sums[k] * inverse_width + p.epsilon;
+    }
+    const auto rounded = [](const float v) { return to_float(from_float<X>(v)); };
+    if constexpr (kFront == Front::kRms) {
+      const float factor = 1.0F / sqrtf(sums[0]);
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c)
+        if (piece0 + 32 * c < piece_end) {
+          float gain[8];
+          load_floats<8>(p.front + static_cast<std::size_t>(piece0 + 32 * c) * 8, gain);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) xv[c][i] = rounded(xv[c][i] * factor * gain[i]);
+        }
+    } else {
+      const float a = p.front[0] * rsqrtf(sums[0]), b = p.front[1] * rsqrtf(sums[1]), c3 = p.front[2] * rsqrtf(sums[2]);
+      const float e = p.front[3];
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c)
+        if (piece0 + 32 * c < piece_end) {
+#pragma unroll
+          for (int i = 0; i < kPer; ++i) xv[c][i] = rounded(fmaf(fmaf(fmaf(c3, xv[c][i], b), xv[c][i], a), xv[c][i], e));
+        }
     }
   }
   int unit = 0;
@@ -414,7 +475,7 @@ bool stream_applicable(const GemvParams &p) {
 }
 
 // One row, or grouped rows with a weight each.
-template <bool kFp8, class X>
+template <bool kFp8, class X, Front kFront = Front::kNone>
 int launch_stream(const GemvParams &p, cudaStream_t stream) {
   constexpr int kPer = kFp8 ? 16 : 8;
   const int pieces = p.K / kPer, chunks = ((pieces + kWarps - 1) / kWarps + 31) / 32;
@@ -422,7 +483,7 @@ int launch_stream(const GemvParams &p, cudaStream_t stream) {
                   static_cast<unsigned int>(p.rows));
   const auto launch = [&](auto chunk_count, auto stage_rows) {
     constexpr int kC = decltype(chunk_count)::value, kR = decltype(stage_rows)::value;
-    const auto kernel = gemv_stream_kernel<kFp8, X, kC, kR, kC >= 4 ? 1 : kC * kR>;
+    const auto kernel = gemv_stream_kernel<kFp8, X, kFront, kC, kR, kC >= 4 ? 1 : kC * kR>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamShared) != cudaSuccess)
       return fail(kCuda, "cannot raise the shared-memory limit of the one-row projection kernel");
     return launch_dependent("one-row projection kernel", kernel, grid, kThreads, kStreamShared, stream, p.dependent_launch != 0,
@@ -448,6 +509,9 @@ constexpr int kColumnsPerCta = 4;
 
 template <bool kFp8>
 int launch_gemv(const GemvParams &p, cudaStream_t stream) {
+  if constexpr (!kFp8)
+    if (p.front != nullptr)
+      return p.poly_front ? launch_stream<false, bf16, Front::kPoly>(p, stream) : launch_stream<false, bf16, Front::kRms>(p, stream);
   if ((p.rows == 1 || p.row_group != nullptr) && stream_applicable<kFp8>(p))
     return launch_stream<kFp8, std::conditional_t<kFp8, std::uint8_t, bf16>>(p, stream);
   const int out_columns = p.gate_mode != 0 ? p.N / 2 : p.N;
@@ -476,6 +540,18 @@ bool small_batch_linear_applicable(const LinearArgs &a) {
          (a.gate_mode == 0 || a.out_features % 256 == 0);
 }
 
+bool row_front_applicable(const RowFront &front, const void *const input, const void *const weight,
+                          const std::size_t in_features, const std::size_t out_features) {
+  if (in_features % 8 != 0 || in_features == 0 || !aligned16(input) || !aligned16(weight) || (!front.poly && !aligned16(front.values)) || in_features > 0x7fffffffU ||
+      out_features > 0x7fffffffU)
+    return false;
+  GemvParams p{};
+  p.rows = 1;
+  p.K = static_cast<int>(in_features);
+  p.N = static_cast<int>(out_features);
+  return stream_applicable<false>(p);
+}
+
 bool one_row_linear_f32_applicable(const LinearF32Args &a) {
   if (a.rows != 1 || a.row_group != nullptr || a.tile_group != nullptr || a.in_features % 8 != 0 || !aligned16(a.input) ||
       !aligned16(a.weight) || a.in_features > 0x7fffffffU || a.out_features > 0x7fffffffU)
@@ -501,6 +577,10 @@ int one_row_linear_f32(const LinearF32Args &a, cudaStream_t stream) {
   p.softcap = a.softcap;
   p.row_scale = a.row_scale;
   p.dependent_launch = a.dependent_launch ? 1 : 0;
+  p.front = a.front.values;
+  p.epsilon = a.front.epsilon;
+  if (a.front.values != nullptr)
+    return a.front.poly ? launch_stream<false, float, Front::kPoly>(p, stream) : launch_stream<false, float, Front::kRms>(p, stream);
   return a.input_type == Activation::kBf16 ? launch_stream<false, bf16>(p, stream) : launch_stream<false, float>(p, stream);
 }
 
@@ -527,6 +607,9 @@ int small_batch_linear(const LinearArgs &a, cudaStream_t stream) {
   p.row_fanout = static_cast<int>(a.row_fanout);
   p.row_group_settled = a.row_group_settled && a.dependent_launch ? 1 : 0;
   p.row_scale = a.row_scale;
+  p.front = a.front.values;
+  p.epsilon = a.front.epsilon;
+  p.poly_front = a.front.poly;
   return a.operand_type == OperandType::kE4m3 ? launch_gemv<true>(p, stream)
                                               : launch_gemv<false>(p, stream);
 }

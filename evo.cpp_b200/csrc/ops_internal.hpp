@@ -8,6 +8,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "decoder_ops.hpp"
+
 namespace evob {
 
 // ---- fp8_codec.cpp: host E4M3FN codec (upstream include/evo/fp8.hpp)
@@ -108,6 +110,7 @@ struct LinearArgs {
   // (128 or 256), tile t belongs to group tile_group[t], *tile_count tiles are in use (both on the device; `rows`
   // is the capacity, unused tiles are not touched).  Row form (a few rows): output row r is input row
   // r / row_fanout times the weight of group row_group[r].
+  RowFront front;  // one row of BF16 products without groups or row_scale; the input is the operator's
   std::size_t groups = 0;
   const int *tile_group = nullptr, *tile_count = nullptr;
   std::size_t tile_rows = 128;

@@ -24,6 +24,7 @@ struct DecoderProduct {
   bool accumulate = false;
   const float *bias = nullptr;
   float alpha = 1.0F, softcap = 0.0F;
+  RowFront front;
 };
 
 namespace {
@@ -186,6 +187,7 @@ int Context::decoder_linear(Stage &s, const DecoderProduct &p) {
     a.alpha = p.alpha;
     a.softcap = p.softcap;
     a.dependent_launch = decode_dependent_launch_ && p.rows == 1;
+    a.front = p.front;
     return linear_f32(a, s.stream);
   }
   LinearArgs a;
@@ -203,6 +205,7 @@ int Context::decoder_linear(Stage &s, const DecoderProduct &p) {
   a.rows = p.rows;
   a.in_features = p.in_features;
   a.out_features = p.out_features;
+  a.front = p.front;
   return linear(a, s.stream);
 }
 
@@ -220,6 +223,9 @@ int Context::decoder_embed(Stage &s, const std::uint32_t *device_tokens, const s
 
 int Context::decoder_head(Stage &s, const std::size_t rows) {
   const ModelConfig &c = weights_->config;
+  DecoderProduct p;
+  p.input = s.normalized;
+  const RowFront norm{s.weights->final_norm, c.epsilon, false};
   if (c.output_norms) {
     LayerNormArgs n;
     n.input = s.hidden;
@@ -230,12 +236,13 @@ int Context::decoder_head(Stage &s, const std::size_t rows) {
     n.width = c.width;
     n.epsilon = c.epsilon;
     EVOB_OP(kCatNorm, layer_norm(n, s.stream));
+  } else if (rows == 1 && row_front_applicable(norm, s.hidden, s.weights->head, c.width, c.vocab)) {
+    p.input = s.hidden;
+    p.front = norm;
   } else {
     EVOB_OP(kCatNorm, rms_norm_residual(static_cast<const float *>(s.hidden), s.weights->final_norm, rows, c.width,
                                         c.epsilon, s.normalized, activation_type(profile_), s.stream));
   }
-  DecoderProduct p;
-  p.input = s.normalized;
   p.weight = s.weights->head;
   p.rows = rows;
   p.in_features = c.width;
@@ -516,8 +523,10 @@ int Context::run_decoder_stage(Stage &s, const std::size_t rows, const Mode mode
   if (c.output_norms && type == Activation::kBf16 && s.weights->layer_begin != 0)
     EVOB_OP(kCatElementwise, convert_rows(hidden, rows * D, s.normalized, type, stream));  // (the embedding leaves it too)
   const auto product = [&](const void *input, const void *weight, const std::size_t in_features,
-                           const std::size_t out_features, void *output, float *output_f32, const bool accumulate) {
+                           const std::size_t out_features, void *output, float *output_f32, const bool accumulate,
+                           const RowFront &front = {}) {
     DecoderProduct p;
+    p.front = front;
     p.input = input;
     p.weight = weight;
     p.rows = rows;
@@ -542,14 +551,23 @@ int Context::run_decoder_stage(Stage &s, const std::size_t rows, const Mode mode
     const DecoderBlock &b = c.blocks[layer];
     const DumpPlan *const tap = dumps != nullptr && dumps->wants_layer(layer) ? dumps : nullptr;
     const void *input = stream_input;
-    if (!c.output_norms) {
+    const std::size_t stride = b.projection_width();
+    // one row: a norm (or the activation) in front of a projection is part of its kernel
+    const auto fused = [&](const RowFront &front, const void *const values, const void *const weight,
+                           const std::size_t in_features, const std::size_t out_features) {
+      return rows == 1 && tap == nullptr && row_front_applicable(front, values, weight, in_features, out_features);
+    };
+    RowFront front;
+    if (!c.output_norms && fused(RowFront{w.pre_norm, c.epsilon, false}, hidden, w.projection, D, stride)) {
+      front = RowFront{w.pre_norm, c.epsilon, false};
+      input = hidden;
+    } else if (!c.output_norms) {
       EVOB_OP(kCatNorm, rms_norm_residual(hidden, w.pre_norm, rows, D, c.epsilon, s.normalized, type, stream));
       if (tap != nullptr)
         EVOB_TRY(emit_activation(stream, *tap, layer, DumpPoint::kPreNorm, s.normalized, rows, D, type));
       input = s.normalized;
     }
-    const std::size_t stride = b.projection_width();
-    EVOB_OP(kCatGemmBf16, product(input, w.projection, D, stride, s.projection, nullptr, false));
+    EVOB_OP(kCatGemmBf16, product(input, w.projection, D, stride, s.projection, nullptr, false, front));
     if (tap != nullptr)
       EVOB_TRY(emit_activation(stream, *tap, layer, DumpPoint::kMixerInputProjection, s.projection, rows, stride, type));
     if (b.mixer == MixerType::kWindowAttention) {
@@ -647,16 +665,22 @@ int Context::run_decoder_stage(Stage &s, const std::size_t rows, const Mode mode
     if (tap != nullptr) EVOB_TRY(emit_f32(stream, *tap, layer, DumpPoint::kMixerResidual, hidden, rows, D, D));
     if (b.feed_forward == FeedForward::kPolyNorm) {
       const std::size_t I = b.inner_width;
-      EVOB_OP(kCatNorm, rms_norm_residual(hidden, w.post_norm, rows, D, c.epsilon, s.normalized, type, stream));
+      const RowFront norm{w.post_norm, c.epsilon, false}, poly{w.activation, c.epsilon, true};
+      const bool norm_fused = fused(norm, hidden, w.l1, D, I), poly_fused = fused(poly, s.mlp_first, w.l3, I, D);
+      if (!norm_fused)
+        EVOB_OP(kCatNorm, rms_norm_residual(hidden, w.post_norm, rows, D, c.epsilon, s.normalized, type, stream));
       if (tap != nullptr)
         EVOB_TRY(emit_activation(stream, *tap, layer, DumpPoint::kPostNorm, s.normalized, rows, D, type));
-      EVOB_OP(kCatGemmBf16, product(s.normalized, w.l1, D, I, s.mlp_first, nullptr, false));
-      EVOB_OP(kCatPolyNorm, poly_norm(s.mlp_first, w.activation, rows, I, c.epsilon, s.gated, type, stream));
+      EVOB_OP(kCatGemmBf16, product(norm_fused ? s.hidden : s.normalized, w.l1, D, I, s.mlp_first, nullptr, false,
+                                    norm_fused ? norm : RowFront{}));
+      if (!poly_fused)
+        EVOB_OP(kCatPolyNorm, poly_norm(s.mlp_first, w.activation, rows, I, c.epsilon, s.gated, type, stream));
       if (tap != nullptr) {
         EVOB_TRY(emit_activation(stream, *tap, layer, DumpPoint::kMlpL1, s.mlp_first, rows, I, type));
         EVOB_TRY(emit_activation(stream, *tap, layer, DumpPoint::kMlpActivation, s.gated, rows, I, type));
       }
-      EVOB_OP(kCatGemmBf16, product(s.gated, w.l3, I, D, nullptr, hidden, true));
+      EVOB_OP(kCatGemmBf16, product(poly_fused ? s.mlp_first : s.gated, w.l3, I, D, nullptr, hidden, true,
+                                    poly_fused ? poly : RowFront{}));
     } else if (b.feed_forward != FeedForward::kNone) {
       LayerNormArgs n = behind;
       n.gain = w.post_norm;
