@@ -114,6 +114,22 @@ def test_f32_results(ops, rows, inner, outer):
             assert_near(out, xv @ wv.T + accumulate * base, 1)
 
 
+@pytest.mark.parametrize("rows", [2, 31, 33, 48, 90, 97, 128, 161])
+@pytest.mark.parametrize("inner, outer", [(8, 5), (100, 129), (130, 127), (264, 128), (520, 260), (1111, 40), (2056, 150)])
+def test_f32_products(ops, rows, inner, outer):
+    """Every height of the F32 tile and every split of the inner size, whole and ragged: the chains have at most
+    16 (ceil(inner / 256) + 4) additions, each rounded to 2^-24 of sums below the sum of the magnitudes."""
+    rng = np.random.default_rng(rows * 1000 + inner)
+    w, wv = activation(rng.normal(0, 1, (outer, inner)), 0)
+    x, base = (rng.normal(0, 1, shape).astype(np.float32) for shape in ((rows, inner), (rows, outer)))
+    exact = cuda(x)
+    out = cuda(base)
+    ops.call("f32_linear", exact.data_ptr(), w.data_ptr(), rows, inner, outer, 1, out.data_ptr(), stream())
+    error = np.abs(out.double().cpu().numpy() - (x.astype(np.float64) @ wv.T + base))
+    chain = 16 * (-(-inner // 256) + 4)
+    assert np.all(error <= chain * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(wv).T + np.abs(base)))
+
+
 # ---------------------------------------------------------------- attention
 def window_case(pkg, ops, *, rows, position, heads, kv_heads, dim, vdim, window, keep_first, kernel, float32=0, softcap=15.0,
                 sink=1, gated=True, biased=True, seed=0, edit=None):
