@@ -11,6 +11,8 @@
 
 #include <algorithm>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "ops_internal.hpp"
 
@@ -546,6 +548,26 @@ __global__ void add_bias_kernel(bf16 *__restrict__ output,
     output[i] = f2bf(bf2f(output[i]) + bf2f(bias[i % width]));
 }
 
+// Result rows as F32 straight into pinned host memory, and behind them the device's error word: one launch and one wait
+// where a copy, a widening loop on the host and a second copy stood.  Bound by the host link (3,001 x 512 logits: 6 MB).
+template <class T>
+__global__ void publish_kernel(const T *__restrict__ rows, const std::size_t elements, float *__restrict__ host,
+                               const int *error_word, int *host_error) {
+  wait_for_producers(rows, error_word);
+  release_dependents();
+  const std::size_t stride = static_cast<std::size_t>(blockDim.x) * gridDim.x;
+  const std::size_t tid = static_cast<std::size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (tid == 0) *host_error = *error_word;
+  const auto value = [](const T v) {
+    if constexpr (std::is_same_v<T, float>) return v;
+    else return bf2f(v);
+  };
+  for (std::size_t i = tid; i < elements / 4; i += stride)
+    reinterpret_cast<float4 *>(host)[i] =
+        make_float4(value(rows[4 * i]), value(rows[4 * i + 1]), value(rows[4 * i + 2]), value(rows[4 * i + 3]));
+  for (std::size_t i = elements / 4 * 4 + tid; i < elements; i += stride) host[i] = value(rows[i]);
+}
+
 // An id outside the table is never used as an index: its row is written as
 // zeros and bit 1 of the per-device error word is raised, which the next
 // gemm_error_state() reports as an invalid argument.
@@ -800,6 +822,21 @@ int embedding(const std::uint32_t *tokens, const void *table,
   if (error_word == nullptr) return status;
   return launch_dependent("embedding kernel", embedding_kernel, dim3(grid_for(rows * width)), kThreads, 0, stream, true, 1, tokens,
                           static_cast<const bf16 *>(table), static_cast<bf16 *>(output), rows, width, vocabulary, error_word);
+}
+
+int publish_rows(const void *rows, const bool f32, const std::size_t elements, float *host, int *host_error,
+                 cudaStream_t stream) {
+  if (rows == nullptr || host == nullptr || host_error == nullptr || !aligned16(host))
+    return fail(kInvalidArgument, "publishing arguments are invalid");
+  int status = kOk;
+  int *const error_word = device_error_word(&status);
+  if (error_word == nullptr) return status;
+  const dim3 grid(grid_for(elements / 4 + 1));
+  if (f32)
+    return launch_dependent("publishing kernel", publish_kernel<float>, grid, kThreads, 0, stream, true, 1,
+                            static_cast<const float *>(rows), elements, host, error_word, host_error);
+  return launch_dependent("publishing kernel", publish_kernel<bf16>, grid, kThreads, 0, stream, true, 1,
+                          static_cast<const bf16 *>(rows), elements, host, error_word, host_error);
 }
 
 int split_triples(const void *projection, const std::size_t rows,

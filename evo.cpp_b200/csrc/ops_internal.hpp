@@ -47,6 +47,9 @@ int add_bias(void *output, const void *bias, std::size_t rows,
 int embedding(const std::uint32_t *tokens, const void *table, std::size_t rows,
               std::size_t width, std::size_t vocabulary, void *output,
               cudaStream_t stream);
+// `elements` BF16 (F32) values as F32 into pinned host memory (16-byte aligned) and the per-device error word into
+// *host_error (pinned too); both are there when the stream has got this far.
+int publish_rows(const void *rows, bool f32, std::size_t elements, float *host, int *host_error, cudaStream_t stream);
 int split_triples(const void *projection, std::size_t rows, std::size_t width,
                   void *x2, void *x1, void *value, cudaStream_t stream);
 int transpose(const void *input, std::size_t rows, std::size_t columns,

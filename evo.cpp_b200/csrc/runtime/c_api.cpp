@@ -289,7 +289,7 @@ evo_status evo_context_prefill(evo_context *context, const evo_batch *batch,
     context->failed = true;  // cleared only if every chunk and callback succeeds
     const std::size_t capacity = context->context->activation_capacity();
     const std::size_t columns = context->context->config().vocab;
-    std::vector<float> logits;
+    evob::HostRows logits;
     for (std::size_t offset = 0; offset < tokens.size();) {
       const std::size_t rows = std::min(capacity, tokens.size() - offset);
       const std::vector<std::uint32_t> chunk(tokens.begin() + offset, tokens.begin() + offset + rows);
@@ -316,7 +316,7 @@ evo_status evo_context_decode(evo_context *context, uint32_t token, evo_logits_c
       return fail(evob::kInvalidArgument, "context and callback are required");
     if (context->failed || context->context->poisoned())
       return fail(evob::kInvalidArgument, "context was invalidated by an earlier failure");
-    std::vector<float> logits;
+    evob::HostRows logits;
     const std::size_t offset = context->context->position();
     int status = context->context->decode(token, &logits);
     if (status != kOk) {
@@ -579,7 +579,7 @@ evo_status evo_b200_context_prefill_with_dumps(evo_context *context, const evo_b
     if (tokens.size() > context->context->activation_capacity())
       return fail(evob::kUnsupported, "a prefill with dumps must fit one activation chunk");
     context->failed = true;
-    std::vector<float> logits;
+    evob::HostRows logits;
     status = context->context->prefill_with_dumps(tokens, plan, cached_attention != 0, &logits);
     if (status != kOk) return status;
     const evo_status callback_status =
@@ -604,7 +604,7 @@ evo_status evo_b200_context_decode_with_dumps(evo_context *context, uint32_t tok
     evob::DumpPlan plan;
     int status = make_dump_plan(requests, request_count, dump_callback, user_data, &plan);
     if (status != kOk) return status;
-    std::vector<float> logits;
+    evob::HostRows logits;
     const std::size_t offset = context->context->position();
     status = context->context->decode_with_dumps(token, plan, &logits);
     if (status != kOk) {
@@ -900,7 +900,7 @@ evo_status evo_b200_context_prefill_tokens(evo_context *context, const uint32_t 
       return fail(evob::kInvalidArgument, "sequence exceeds the context capacity");
     if (mode != EVO_B200_PREFILL_FRESH && token_count > capacity)
       return fail(evob::kInvalidArgument, "this prefill form takes at most one activation chunk of tokens");
-    std::vector<float> logits;
+    evob::HostRows logits;
     for (std::size_t offset = 0; offset < token_count;) {
       const std::size_t rows = std::min(capacity, token_count - offset);
       const std::vector<std::uint32_t> chunk(tokens + offset, tokens + offset + rows);

@@ -202,7 +202,74 @@ int Context::dump_mlp_taps(Stage &s, const std::size_t i, const std::size_t rows
   return kOk;
 }
 
+HostPool::~HostPool() {
+  for (const Block &b : free_) cudaFreeHost(b.data);
+}
+
+void *HostPool::take(const std::size_t bytes, std::size_t *const capacity) {
+  std::size_t wanted = std::size_t{64} << 10;
+  while (wanted < bytes) wanted *= 2;  // few sizes, so that blocks find their next user
+  {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    for (std::size_t i = 0; i < free_.size(); ++i)
+      if (free_[i].capacity >= wanted) {
+        const Block b = free_[i];
+        free_.erase(free_.begin() + static_cast<std::ptrdiff_t>(i));
+        *capacity = b.capacity;
+        return b.data;
+      }
+  }
+  void *data = nullptr;
+  if (cudaHostAlloc(&data, wanted, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  *capacity = wanted;
+  return data;
+}
+
+void HostPool::give(void *const block, const std::size_t capacity) {
+  Block dropped{block, capacity};
+  if (capacity <= kLargest) {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    free_.push_back(dropped);
+    if (free_.size() <= kKept) return;
+    const auto smallest = std::min_element(free_.begin(), free_.end(),
+                                           [](const Block &a, const Block &b) { return a.capacity < b.capacity; });
+    dropped = *smallest;
+    free_.erase(smallest);
+  }
+  cudaFreeHost(dropped.data);
+}
+
+void HostRows::release() {
+  if (block_ != nullptr) pool_->give(block_, capacity_);
+  block_ = nullptr;
+  pool_.reset();
+}
+
+void HostRows::resize(const std::shared_ptr<HostPool> &pool, const std::size_t count) {
+  if (block_ == nullptr || pool_ != pool || capacity_ < count * sizeof(float)) {
+    release();
+    block_ = count * sizeof(float) <= HostPool::kLargest ? pool->take(count * sizeof(float), &capacity_) : nullptr;
+    if (block_ != nullptr) pool_ = pool;
+  }
+  if (block_ == nullptr) own_.resize(count);
+  count_ = count;
+}
+
+void HostRows::assign(const float *const values, const std::size_t count) {
+  release();
+  own_.assign(values, values + count);
+  count_ = count;
+}
+
 Context::~Context() {
+  if (!stages_.empty()) {
+    DeviceGuard guard(stages_.front()->device);
+    cudaStreamSynchronize(stages_.front()->stream);  // nothing writes the pinned memory any more
+  }
+  if (host_step_ != nullptr) weights_->host_pool->give(host_step_, host_step_bytes_);
   if (decode_graph_ != nullptr) cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(decode_graph_));
 }
 
@@ -218,10 +285,9 @@ int Context::decode_step_graph(const std::uint32_t *host_token, bool *launched) 
   Stage &first = *stages_.front();
   DeviceGuard guard(first.device);
   cudaStream_t stream = first.stream;
-  decode_position_host_ = static_cast<int>(position_);
-  if (cudaMemcpyAsync(first.tokens, host_token, 4, cudaMemcpyHostToDevice, stream) != cudaSuccess ||
-      cudaMemcpyAsync(device_position_, &decode_position_host_, 4, cudaMemcpyHostToDevice, stream) != cudaSuccess)
-    return fail(kCuda, "token upload failed");
+  // (the stream is idle here: every step waits for its results)
+  host_step_[0] = *host_token;
+  host_step_[1] = static_cast<std::uint32_t>(position_);
   if (decode_graph_ == nullptr) {
     if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
@@ -229,8 +295,12 @@ int Context::decode_step_graph(const std::uint32_t *host_token, bool *launched) 
       return kOk;
     }
     dynamic_position_ = device_position_;
-    int status = c.decoder() ? decoder_embed(first, first.tokens, 1, position_)
-                             : embedding(first.tokens, first.weights->embedding, 1, c.width, c.vocab, first.hidden, stream);
+    int status = cudaMemcpyAsync(device_step_, host_step_, 2 * sizeof(std::uint32_t), cudaMemcpyHostToDevice, stream) == cudaSuccess
+                     ? kOk
+                     : fail(kCuda, "token upload failed");
+    if (status == kOk)
+      status = c.decoder() ? decoder_embed(first, device_step_, 1, position_)
+                           : embedding(device_step_, first.weights->embedding, 1, c.width, c.vocab, first.hidden, stream);
     if (status == kOk)
       status = c.decoder() ? run_decoder_stage(first, 1, Mode::kDecode, position_, -1, nullptr, nullptr)
                            : run_stage(first, 1, Mode::kDecode, -1, nullptr);
@@ -252,6 +322,9 @@ int Context::decode_step_graph(const std::uint32_t *host_token, bool *launched) 
       a.out_features = c.vocab;
       status = linear(a, stream);
     }
+    if (status == kOk)
+      status = publish_rows(first.logits, c.decoder(), c.vocab, reinterpret_cast<float *>(host_step_ + kStepRow),
+                            reinterpret_cast<int *>(host_step_ + 2), stream);
     dynamic_position_ = nullptr;
     cudaGraph_t graph = nullptr;
     const cudaError_t ended = cudaStreamEndCapture(stream, &graph);
@@ -391,7 +464,11 @@ int Context::create(std::shared_ptr<ModelWeights> weights, const std::size_t con
     DeviceGuard guard(first.device);
     void *p = nullptr;
     EVOB_TRY(first.allocate(&p, 16, &first.arena_bytes));
-    context->device_position_ = static_cast<int *>(p);
+    context->device_step_ = static_cast<std::uint32_t *>(p);
+    context->device_position_ = reinterpret_cast<const int *>(context->device_step_ + 1);
+    context->host_step_ = static_cast<std::uint32_t *>(weights->host_pool->take(
+        kStepRow * sizeof(std::uint32_t) + c.vocab * sizeof(float), &context->host_step_bytes_));
+    if (context->host_step_ == nullptr) return fail(kCuda, "cannot allocate the context's pinned memory");
     const char *const graphs = std::getenv("EVO_B200_DECODE_GRAPH");
     context->decode_graph_allowed_ = (graphs == nullptr || std::string(graphs) != "0") && !q8_kv;
     const char *const dependent = std::getenv("EVO_B200_DECODE_PDL");
@@ -902,7 +979,7 @@ int Context::run_wavefront(const std::size_t rows, const Mode /*mode*/, const lo
 }
 
 int Context::forward(const std::uint32_t *host_tokens, const std::uint32_t *device_tokens,
-                     const std::size_t rows, const Mode mode, std::vector<float> *logits,
+                     const std::size_t rows, const Mode mode, HostRows *logits,
                      const long capture_layer, std::vector<float> *captured, const DumpPlan *const dumps) {
   const ModelConfig &c = weights_->config;
   if (!healthy_) return fail(kInvalidArgument, "context was invalidated by an earlier failure");
@@ -1011,23 +1088,41 @@ int Context::forward(const std::uint32_t *host_tokens, const std::uint32_t *devi
       status = linear(a, first.stream);
     }
     if (status == kOk && logits != nullptr) {
-      // BF16 logits are widened here; decoders' heads leave F32
-      std::vector<std::uint16_t> raw(c.decoder() ? 0 : rows * c.vocab);
-      logits->resize(rows * c.vocab);
-      void *const host = c.decoder() ? static_cast<void *>(logits->data()) : static_cast<void *>(raw.data());
-      if (cudaMemcpyAsync(host, first.logits, logits->size() * (c.decoder() ? 4 : 2), cudaMemcpyDeviceToHost,
-                          first.stream) != cudaSuccess ||
-          cudaStreamSynchronize(first.stream) != cudaSuccess) {
-        status = fail(kCuda, std::string("logits read-back failed: ") +
-                                 cudaGetErrorString(cudaGetLastError()));
-      } else {
-        for (std::size_t j = 0; j < raw.size(); ++j) {
-          const std::uint32_t bits = static_cast<std::uint32_t>(raw[j]) << 16U;
-          std::memcpy(&(*logits)[j], &bits, 4);
+      const std::size_t elements = rows * c.vocab;
+      int *const error = reinterpret_cast<int *>(host_step_ + 2);
+      if (!graph_step) {
+        *error = 0;
+        logits->resize(weights_->host_pool, elements);
+        if (logits->pinned()) {
+          status = publish_rows(first.logits, c.decoder(), elements, logits->data(), error, first.stream);
+        } else {
+          // more than the pool holds; BF16 logits land in the upper half of the result and are widened from there
+          unsigned char *const target = reinterpret_cast<unsigned char *>(logits->data()) + (c.decoder() ? 0 : elements * 2);
+          if (cudaMemcpyAsync(target, first.logits, elements * (c.decoder() ? 4 : 2), cudaMemcpyDeviceToHost, first.stream) !=
+              cudaSuccess)
+            status = fail(kCuda, std::string("logits read-back failed: ") + cudaGetErrorString(cudaGetLastError()));
         }
+      }
+      if (status == kOk && cudaStreamSynchronize(first.stream) != cudaSuccess) {
+        status = fail(kCuda, std::string("logits read-back failed: ") + cudaGetErrorString(cudaGetLastError()));
+      } else if (status == kOk) {
+        if (graph_step) {
+          logits->assign(reinterpret_cast<const float *>(host_step_ + kStepRow), elements);
+        } else if (!logits->pinned() && !c.decoder()) {
+          const unsigned char *const source = reinterpret_cast<const unsigned char *>(logits->data()) + elements * 2;
+          for (std::size_t j = 0; j < elements; ++j) {
+            std::uint16_t raw;
+            std::memcpy(&raw, source + 2 * j, 2);
+            const std::uint32_t bits = static_cast<std::uint32_t>(raw) << 16U;
+            std::memcpy(logits->data() + j, &bits, 4);
+          }
+        }
+        const bool published = graph_step || logits->pinned();
         for (const auto &stage : stages_) {
           DeviceGuard stage_guard(stage->device);
-          if (status == kOk) status = gemm_error_state(stage->stream);
+          // (the first stage's error word has come with the logits)
+          const bool clean = stage == stages_.front() && published && *error == 0;
+          if (status == kOk && !clean) status = gemm_error_state(stage->stream);
           stage->collect_profile();
         }
       }
@@ -1126,25 +1221,25 @@ int Context::slice_head(const std::size_t position, const std::size_t rows) {
   return linear(a, stage.stream);
 }
 
-int Context::prefill(const std::vector<std::uint32_t> &tokens, std::vector<float> *logits) {
+int Context::prefill(const std::vector<std::uint32_t> &tokens, HostRows *logits) {
   if (logits == nullptr) return fail(kInvalidArgument, "logits output is null");
   return forward(tokens.data(), nullptr, tokens.size(), Mode::kPrefill, logits, -1, nullptr);
 }
-int Context::prefill_stateless(const std::vector<std::uint32_t> &tokens, std::vector<float> *logits) {
+int Context::prefill_stateless(const std::vector<std::uint32_t> &tokens, HostRows *logits) {
   if (logits == nullptr) return fail(kInvalidArgument, "logits output is null");
   return forward(tokens.data(), nullptr, tokens.size(), Mode::kStateless, logits, -1, nullptr);
 }
-int Context::prefill_cached(const std::vector<std::uint32_t> &tokens, std::vector<float> *logits) {
+int Context::prefill_cached(const std::vector<std::uint32_t> &tokens, HostRows *logits) {
   if (logits == nullptr) return fail(kInvalidArgument, "logits output is null");
   return forward(tokens.data(), nullptr, tokens.size(), Mode::kCachedPrefill, logits, -1, nullptr);
 }
-int Context::prefill_chunk(const std::vector<std::uint32_t> &tokens, std::vector<float> *logits) {
+int Context::prefill_chunk(const std::vector<std::uint32_t> &tokens, HostRows *logits) {
   if (logits == nullptr) return fail(kInvalidArgument, "logits output is null");
   if (state_valid_ && cached_attention_)
     return fail(kInvalidArgument, "a cached prefill continues through exact token decode only, not through another chunk");
   return forward(tokens.data(), nullptr, tokens.size(), Mode::kContinue, logits, -1, nullptr);
 }
-int Context::decode(const std::uint32_t token, std::vector<float> *logits) {
+int Context::decode(const std::uint32_t token, HostRows *logits) {
   if (logits == nullptr) return fail(kInvalidArgument, "logits output is null");
   return forward(&token, nullptr, 1, Mode::kDecode, logits, -1, nullptr);
 }
@@ -1152,7 +1247,7 @@ int Context::prefill_embedding(const std::vector<std::uint32_t> &tokens, const s
                                std::vector<float> *hidden) {
   if (hidden == nullptr || layer >= weights_->config.layers)
     return fail(kInvalidArgument, "layer capture index or output is invalid");
-  std::vector<float> logits;
+  HostRows logits;
   return forward(tokens.data(), nullptr, tokens.size(), Mode::kStateless, &logits,
                  static_cast<long>(layer), hidden);
 }
@@ -1162,12 +1257,12 @@ int Context::prefill_chunk_embedding(const std::vector<std::uint32_t> &tokens, c
     return fail(kInvalidArgument, "layer capture index or output is invalid");
   if (!first && state_valid_ && cached_attention_)
     return fail(kInvalidArgument, "a cached prefill continues through exact token decode only, not through another chunk");
-  std::vector<float> logits;
+  HostRows logits;
   return forward(tokens.data(), nullptr, tokens.size(), first ? Mode::kPrefill : Mode::kContinue, &logits,
                  static_cast<long>(layer), hidden);
 }
 int Context::prefill_with_dumps(const std::vector<std::uint32_t> &tokens, const DumpPlan &plan,
-                                const bool cached, std::vector<float> *logits) {
+                                const bool cached, HostRows *logits) {
   if (logits == nullptr) return fail(kInvalidArgument, "logits output is null");
   for (const DumpPlan::Request &request : plan.requests)
     if (request.layer >= weights_->config.layers || static_cast<int>(request.point) < 0 ||
@@ -1176,7 +1271,7 @@ int Context::prefill_with_dumps(const std::vector<std::uint32_t> &tokens, const 
   return forward(tokens.data(), nullptr, tokens.size(), cached ? Mode::kCachedPrefill : Mode::kPrefill, logits, -1,
                  nullptr, &plan);
 }
-int Context::decode_with_dumps(const std::uint32_t token, const DumpPlan &plan, std::vector<float> *logits) {
+int Context::decode_with_dumps(const std::uint32_t token, const DumpPlan &plan, HostRows *logits) {
   if (logits == nullptr) return fail(kInvalidArgument, "logits output is null");
   for (const DumpPlan::Request &request : plan.requests)
     if (request.layer >= weights_->config.layers || static_cast<int>(request.point) < 0 ||

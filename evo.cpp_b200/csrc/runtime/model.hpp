@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -231,8 +232,50 @@ struct StageWeights {
   ~StageWeights();
 };
 
+// Pinned host memory that results come back through, shared by the contexts of a model (any thread, any device).
+// kKept free blocks of up to kLargest bytes stay for the next user, the rest is given back.
+class HostPool {
+ public:
+  static constexpr std::size_t kLargest = std::size_t{64} << 20, kKept = 4;
+  ~HostPool();
+  void *take(std::size_t bytes, std::size_t *capacity);  // nullptr: not to be had
+  void give(void *block, std::size_t capacity);
+
+ private:
+  struct Block {
+    void *data;
+    std::size_t capacity;
+  };
+  std::mutex mutex_;
+  std::vector<Block> free_;
+};
+
+// Rows of F32 results on the host: a pool's block until the next use or the end of the object, or memory of its own.
+class HostRows {
+ public:
+  HostRows() = default;
+  HostRows(const HostRows &) = delete;
+  HostRows &operator=(const HostRows &) = delete;
+  ~HostRows() { release(); }
+  // Room for `count` values, pinned if the pool has it.
+  void resize(const std::shared_ptr<HostPool> &pool, std::size_t count);
+  void assign(const float *values, std::size_t count);
+  bool pinned() const { return block_ != nullptr; }
+  float *data() { return block_ != nullptr ? static_cast<float *>(block_) : own_.data(); }
+  const float *data() const { return block_ != nullptr ? static_cast<const float *>(block_) : own_.data(); }
+  std::size_t size() const { return count_; }
+
+ private:
+  void release();
+  std::shared_ptr<HostPool> pool_;
+  void *block_ = nullptr;
+  std::size_t capacity_ = 0, count_ = 0;
+  std::vector<float> own_;
+};
+
 struct ModelWeights {
   ModelConfig config;
+  std::shared_ptr<HostPool> host_pool = std::make_shared<HostPool>();
   std::vector<std::shared_ptr<StageWeights>> stages;
   // Per-process pipelines: this process holds stage `slice_index` of
   // `slice_count` (one StageWeights); 0 / 1 for a model held by one process.
@@ -265,12 +308,12 @@ class Context {
                     ExecutionProfile profile, bool full_arena_for_fixtures,
                     std::unique_ptr<Context> *out, bool q8_kv = false);
 
-  // logits: rows * vocab floats (converted from BF16).
-  int prefill(const std::vector<std::uint32_t> &tokens, std::vector<float> *logits);
-  int prefill_stateless(const std::vector<std::uint32_t> &tokens, std::vector<float> *logits);
-  int prefill_cached(const std::vector<std::uint32_t> &tokens, std::vector<float> *logits);
-  int prefill_chunk(const std::vector<std::uint32_t> &tokens, std::vector<float> *logits);
-  int decode(std::uint32_t token, std::vector<float> *logits);
+  // logits: rows * vocab floats (converted from BF16), valid until *logits is used again or destroyed.
+  int prefill(const std::vector<std::uint32_t> &tokens, HostRows *logits);
+  int prefill_stateless(const std::vector<std::uint32_t> &tokens, HostRows *logits);
+  int prefill_cached(const std::vector<std::uint32_t> &tokens, HostRows *logits);
+  int prefill_chunk(const std::vector<std::uint32_t> &tokens, HostRows *logits);
+  int decode(std::uint32_t token, HostRows *logits);
   // Block output of `layer` ([rows, width] floats) for a fresh stateless prefill.
   int prefill_embedding(const std::vector<std::uint32_t> &tokens, std::size_t layer,
                         std::vector<float> *hidden);
@@ -286,8 +329,8 @@ class Context {
   // next to the fused kernels, so that every intermediate exists as a buffer;
   // the block's own results still come from the ordinary path.
   int prefill_with_dumps(const std::vector<std::uint32_t> &tokens, const DumpPlan &plan, bool cached,
-                         std::vector<float> *logits);
-  int decode_with_dumps(std::uint32_t token, const DumpPlan &plan, std::vector<float> *logits);
+                         HostRows *logits);
+  int decode_with_dumps(std::uint32_t token, const DumpPlan &plan, HostRows *logits);
 
   // Device-resident variant used by the benchmark: tokens already on the
   // device of stage 0, logits left on the device (BF16 [rows, vocab]).
@@ -334,7 +377,7 @@ class Context {
   enum class Mode { kPrefill, kStateless, kCachedPrefill, kContinue, kDecode, kWindow };
   Context() = default;
   int forward(const std::uint32_t *host_tokens, const std::uint32_t *device_tokens,
-              std::size_t rows, Mode mode, std::vector<float> *logits, long capture_layer,
+              std::size_t rows, Mode mode, HostRows *logits, long capture_layer,
               std::vector<float> *captured, const DumpPlan *dumps = nullptr);
   int run_stage(Stage &stage, std::size_t rows, Mode mode, long capture_layer,
                 std::vector<float> *captured, std::size_t window_begin = 0,
@@ -367,9 +410,14 @@ class Context {
   // 128, history full; EVO_B200_DECODE_GRAPH=0 turns it off).
   int decode_step_graph(const std::uint32_t *host_token, bool *launched);
   void *decode_graph_ = nullptr;          // cudaGraphExec_t
-  int *device_position_ = nullptr;        // position of the decoded token, read by replayed kernels
+  // A step's token and position, and where replayed kernels read them; pinned: the same two, then the error word behind
+  // the step, and from kStepRow on its logits.
+  std::uint32_t *device_step_ = nullptr;
+  const int *device_position_ = nullptr;
+  std::uint32_t *host_step_ = nullptr;
+  std::size_t host_step_bytes_ = 0;
+  static constexpr std::size_t kStepRow = 4;
   const int *dynamic_position_ = nullptr; // == device_position_ while the graph is being recorded
-  int decode_position_host_ = 0;
   bool decode_graph_allowed_ = true;
   // one-row projections are launched with programmatic stream serialisation (EVO_B200_DECODE_PDL=0: plain launches)
   bool decode_dependent_launch_ = true;

@@ -72,7 +72,7 @@ struct Scheduler::Impl {
       result->error = last_error();
       return;
     }
-    std::vector<float> logits;
+    HostRows logits;
     std::vector<std::uint32_t> tokens;
     for (std::size_t offset = 0; offset < prompt.size(); offset += chunk) {
       if (work.cancelled.load(std::memory_order_relaxed)) {
@@ -103,7 +103,7 @@ struct Scheduler::Impl {
     }
     Sampler sampler(request.sampling);
     const float *last_row = logits.data() + (logits.size() / vocab - 1) * vocab;
-    std::vector<float> step;
+    HostRows step;
     for (std::size_t produced = 0; produced < request.new_tokens; ++produced) {
       if (work.cancelled.load(std::memory_order_relaxed)) {
         result->cancelled = true;

@@ -360,10 +360,13 @@ class Context:
 
         @LOGITS_CALLBACK
         def on_rows(data, rows, cols, offset, _user):
-            chunks.append((offset, np.ctypeslib.as_array(data, shape=(rows, cols)).copy()))
+            values = (ctypes.c_float * (rows * cols)).from_address(ctypes.addressof(data.contents))
+            chunks.append((offset, np.frombuffer(values, np.float32).reshape(rows, cols).copy()))
             return 0
 
         self.library.check(call(on_rows))
+        if len(chunks) == 1:
+            return chunks[0][1]
         chunks.sort(key=lambda c: c[0])
         return np.concatenate([c[1] for c in chunks], axis=0) if chunks else np.zeros((0, columns), np.float32)
 
