@@ -231,17 +231,16 @@ gemv_kernel(const GemvParams p) {
 // copies its 16-byte pieces of the weight rows into its own slots of a ring in shared memory
 // (cp.async) and reads only what it copied itself: no barrier in the loop, and the ring is filled before the thread
 // waits for the producer of x (the weights do not depend on it).  The warps' partial sums of all columns meet in
-// shared memory once, at the end.  The CTAs of two such kernels fit an SM, so the next projection of a decode step
-// fills its ring while this one drains.
+// shared memory once, at the end.  A CTA is two such teams, and its shared memory keeps a second CTA off the SM: where a
+// kernel starts beside others, CTAs that fit twice are packed on half of the SMs (observed: four small CTAs on each of 74),
+// and a stream is as slow as its fullest SM.
 // Grouped rows (blockIdx.y) take their weights' rows the same way, once they know their group.
-// Bound: HBM.  Back to back in a graph, weights beyond L2 (us; in brackets one CTA per four rows with registers and
-// prefetches into L2): 8448 x 2048 6.2 (8.3), 4096 x 4096 5.9 (7.4), gated 22528 x 4096 26.9 = 6.9 TB/s (29.3),
-// 4096 x 11264 15.0 (19.0), 5760 x 1920 4.5 (6.2).  One CTA per SM with twice the ring is up to 20 % slower (its eight
-// warps do not keep up), four with half of it as fast but 15 % slower at K = 11264.
-constexpr int kRingBytes = 48 * 1024, kStreamCtas = 2;
-// Four CTAs fit an SM and no fifth: where a kernel starts beside others, none of its SMs gets more than two extra.
-constexpr int kStreamShared = 54 * 1024;
-constexpr int kStreamRows = (kStreamShared - kRingBytes) / (kWarps * static_cast<int>(sizeof(float)));  // per CTA
+// Bound: HBM, and in a step the way from one kernel's end to the next one's first data.  48 decode steps of Gigusun:
+// 12.3 ms, 12.8 with two CTAs of one team each that pack; of Kikepel 11.4 and 11.9.
+constexpr int kTeams = 2, kRingBytes = 48 * 1024;
+constexpr int kStreamShared = 116 * 1024;  // more than half of an SM's
+constexpr int kTeamShared = kStreamShared / kTeams;
+constexpr int kStreamRows = (kTeamShared - kRingBytes) / (kWarps * static_cast<int>(sizeof(float)));  // per team
 
 // What is done to x on the way in.  A norm's statistics are those of the whole row: every CTA takes them itself, which
 // costs it a barrier against a launch and a round trip through memory.
@@ -250,20 +249,23 @@ enum class Front { kNone, kRms, kPoly };
 // kUnit: pieces per thread that are copied and waited for at a time, whole rows (kRowsPerStage of kChunks pieces) or, of
 // long rows, single pieces.
 template <bool kFp8, class X, Front kFront, int kChunks, int kRowsPerStage, int kUnit>
-__global__ void __launch_bounds__(kThreads, kChunks >= 5 ? 2 : 3)
+__global__ void __launch_bounds__(kTeams *kThreads, 1)
 gemv_stream_kernel(const GemvParams p) {
   constexpr int kPer = kFp8 ? 16 : 8;  // elements per 16-byte piece
   constexpr int kUnits = kRingBytes / (kUnit * kThreads * 16);
   static_assert(kUnits >= 3 && (kUnit == 1 ? kRowsPerStage == 1 : kUnit == kRowsPerStage * kChunks), "ring");
-  extern __shared__ __align__(16) uint4 ring[];  // [kUnits][kUnit][kThreads]
+  extern __shared__ __align__(16) unsigned char stream_smem[];
+  const int team = threadIdx.x / kThreads, tid = threadIdx.x % kThreads, warp = tid / 32, lane = tid % 32;
+  uint4 *const ring = reinterpret_cast<uint4 *>(stream_smem + team * kTeamShared);     // [kUnits][kUnit][kThreads]
   float *const partial = reinterpret_cast<float *>(ring + kUnits * kUnit * kThreads);  // [rows][kWarps]
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const auto team_barrier = [&] { asm volatile("barrier.cta.sync %0, %1;" ::"r"(team + 1), "n"(kThreads) : "memory"); };
   const bool gated = p.gate_mode != 0, grouped = p.row_group != nullptr;
   const int out_columns = gated ? p.N / 2 : p.N;
-  const auto share = [&](const unsigned int cta) {
-    return static_cast<int>(static_cast<unsigned long long>(out_columns) * cta / gridDim.x);
+  const auto share = [&](const unsigned int index) {
+    return static_cast<int>(static_cast<unsigned long long>(out_columns) * index / (kTeams * gridDim.x));
   };
-  const int column0 = share(blockIdx.x), columns = share(blockIdx.x + 1) - column0;
+  const unsigned int team_index = kTeams * blockIdx.x + team;
+  const int column0 = share(team_index), columns = share(team_index + 1) - column0;
   const int rows = gated ? 2 * columns : columns;  // gated: all first rows, then their partners
   const int groups = (rows + kRowsPerStage - 1) / kRowsPerStage;
   const std::size_t row_bytes = static_cast<std::size_t>(p.K) * (kFp8 ? 1 : 2);
@@ -346,7 +348,8 @@ gemv_stream_kernel(const GemvParams p) {
     }
   }
   if constexpr (kFront != Front::kNone) {
-    __shared__ float scratch[3][kWarps];
+    __shared__ float team_scratch[kTeams][3][kWarps];
+    auto &scratch = team_scratch[team];
     constexpr int kSums = kFront == Front::kPoly ? 3 : 1;
     float sums[3] = {0.0F, 0.0F, 0.0F};  // of squares, fourth and sixth powers
 #pragma unroll
@@ -367,7 +370,7 @@ gemv_stream_kernel(const GemvParams p) {
       sums[k] = warp_sum(sums[k]);
       if (lane == 0) scratch[k][warp] = sums[k];
     }
-    __syncthreads();
+    team_barrier();
     const float inverse_width = 1.0F / static_cast<float>(p.K);
 #pragma unroll
     for (int k = 0; k < kSums; ++k) {
@@ -449,7 +452,7 @@ gemv_stream_kernel(const GemvParams p) {
     for (int step = 16 / kRowsPerStage; step > 0; step /= 2) sum[0] += __shfl_xor_sync(0xffffffffU, sum[0], step);
     if (lane % (32 / kRowsPerStage) == 0 && row < rows) partial[row * kWarps + warp] = sum[0];
   }
-  __syncthreads();
+  team_barrier();
   const float alpha = p.row_scale != nullptr ? p.alpha * p.row_scale[blockIdx.y] : p.alpha;
   for (int local = tid; local < columns; local += kThreads)
     finish_column(p, 0, blockIdx.y, out_columns, column0 + local, alpha, local,
@@ -461,15 +464,15 @@ gemv_stream_kernel(const GemvParams p) {
                   });
 }
 
-// CTAs across the columns of each of `rows` output rows: together about kStreamCtas per SM.
+// CTAs across the columns of each of `rows` output rows: together about one per SM.
 int stream_grid(const int out_columns, const int rows) {
-  const int wanted = std::max(1, kStreamCtas * kSmCount / rows);
-  return std::min(out_columns, wanted);
+  const int wanted = std::max(1, kSmCount / rows);
+  return std::min((out_columns + kTeams - 1) / kTeams, wanted);
 }
 // Sizes that the one-row kernel has registers (K) and partial sums (N) for.
 template <bool kFp8>
 bool stream_applicable(const GemvParams &p) {
-  const int out_columns = p.gate_mode != 0 ? p.N / 2 : p.N, grid = stream_grid(out_columns, p.rows);
+  const int out_columns = p.gate_mode != 0 ? p.N / 2 : p.N, grid = kTeams * stream_grid(out_columns, p.rows);
   return p.K <= (kFp8 ? 6 * 16 : 8 * 8) * kWarps * 32 &&
          ((out_columns - 1) / grid + 1) * (p.gate_mode != 0 ? 2 : 1) <= kStreamRows;
 }
@@ -486,7 +489,7 @@ int launch_stream(const GemvParams &p, cudaStream_t stream) {
     const auto kernel = gemv_stream_kernel<kFp8, X, kFront, kC, kR, kC >= 4 ? 1 : kC * kR>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamShared) != cudaSuccess)
       return fail(kCuda, "cannot raise the shared-memory limit of the one-row projection kernel");
-    return launch_dependent("one-row projection kernel", kernel, grid, kThreads, kStreamShared, stream, p.dependent_launch != 0,
+    return launch_dependent("one-row projection kernel", kernel, grid, kTeams * kThreads, kStreamShared, stream, p.dependent_launch != 0,
                             1, p);
   };
   using std::integral_constant;
