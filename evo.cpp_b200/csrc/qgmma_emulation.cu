@@ -26,8 +26,8 @@
 //     mma.sync's result layout is the thread's output tile.
 // What bounds it: the ALU (packing, signs, staging) and the half of the FMA pipe
 // that dp2a shares with the multiply-adds, each busy for 60 % of the time with 16
-// warps per SM; about 3 instructions per product.  509 rows at 12288 x 4096: 3.6
-// ms = 7.1 T products/s; integer shifts per product took 17.1 ms.
+// warps per SM; about 3 instructions per product.  509 rows at 12288 x 4096: 3.5
+// ms = 7.4 T products/s; integer shifts per product took 17.1 ms.
 #include "common.cuh"
 #include "ops_internal.hpp"
 
@@ -258,7 +258,7 @@ qgmma_emulation_kernel(const std::uint8_t *__restrict__ input_codes,
           sum[m][n][q] = 0;
         }
 
-#pragma unroll 2
+#pragma unroll  // (two steps at a time: 3 % slower, four 16 %; with all of them the packing mixes with the multiply-adds)
     for (int k = 0; k < kGroup; k += 4) {
       std::uint64_t a_value[kM][2][2], b_value[kN][2][2];
       std::uint32_t a_sign[kM][2], b_sign[kN][2];
