@@ -750,15 +750,17 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 // rows x one K slice, and K is split until enough CTAs pull on the stream.  The
 // CTAs leave raw F32 partial sums [split][token][weight row]; the finishing
 // kernel adds them in split order and applies the epilogue.
-constexpr int kSwapStages = 6;
-
+// Up to 64 tokens the ring leaves room for a second CTA on the SM: of more CTAs than SMs all run at once and share the
+// stream, where a second wave of a few took as long as the first (61 tokens, 176 tiles of 22528 x 4096: 50 us with six
+// stages and one CTA, 38 with four and two).
 template <int BT>
 struct SwapLayout {
+  static constexpr int kStages = BT <= 16 ? 6 : BT <= 32 ? 5 : BT <= 64 ? 4 : 6;
   static constexpr int kWBytes = kBlockM * kBlockKBytes;  // 128 weight rows x 128 bytes of K
   static constexpr int kXBytes = BT * kBlockKBytes;
   static constexpr int kStageBytes = kWBytes + kXBytes;
-  static constexpr int kBarrierOffset = kSwapStages * kStageBytes;
-  static constexpr int kBarrierCount = 2 * kSwapStages + 1;  // full[], empty[], accumulator ready
+  static constexpr int kBarrierOffset = kStages * kStageBytes;
+  static constexpr int kBarrierCount = 2 * kStages + 1;  // full[], empty[], accumulator ready
   static constexpr int kTmemPtrOffset = kBarrierOffset + kBarrierCount * 8;
   static constexpr int kAbortOffset = kTmemPtrOffset + 8;
   static constexpr int kTotal = kAbortOffset + 8 + 1024;  // + alignment slack
@@ -775,8 +777,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   const std::uint32_t smem_base = smem_u32(smem);
   const std::uint32_t bar_base = smem_base + L::kBarrierOffset;
   auto full_bar = [&](const int s) { return bar_base + 8U * s; };
-  auto empty_bar = [&](const int s) { return bar_base + 8U * (kSwapStages + s); };
-  const std::uint32_t ready_bar = bar_base + 8U * (2 * kSwapStages);
+  auto empty_bar = [&](const int s) { return bar_base + 8U * (L::kStages + s); };
+  const std::uint32_t ready_bar = bar_base + 8U * (2 * L::kStages);
   volatile std::uint32_t *const tmem_ptr = reinterpret_cast<volatile std::uint32_t *>(smem + L::kTmemPtrOffset);
   volatile int *const abort_flag = reinterpret_cast<volatile int *>(smem + L::kAbortOffset);
   const int warp = threadIdx.x / 32;
@@ -784,7 +786,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   constexpr std::uint32_t kTmemColumns = BT < 32 ? 32 : BT;  // power of two, at least 32
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kSwapStages; ++s) {
+    for (int s = 0; s < L::kStages; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
     }
@@ -803,6 +805,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  release_dependents();
   const std::uint32_t tmem_base = *tmem_ptr;
 
   const int tile_n = blockIdx.x % tiles_n;
@@ -814,14 +817,23 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     if (lane == 0) {
       int stage = 0;
       std::uint32_t phase = 0;
+      const auto k_of = [&](const int kb) { return kFp8 ? kb * kBlockKBytes : kb * (kBlockKBytes / 2); };
+      // the first weights do not depend on the kernel that writes the tokens
+      const int early = k_per_split < L::kStages ? k_per_split : L::kStages;
+      for (int s = 0; s < early; ++s) {
+        mbar_expect_tx(full_bar(s), L::kStageBytes);
+        tma_load_2d(smem_base + s * L::kStageBytes, &map_w, full_bar(s), k_of(kb_begin + s), n0);
+      }
+      wait_for_producers();
       for (int kb = kb_begin; kb < kb_begin + k_per_split; ++kb) {
-        if (!mbar_wait(empty_bar(stage), phase ^ 1U, abort_flag)) break;
         const std::uint32_t w_dst = smem_base + stage * L::kStageBytes;
-        mbar_expect_tx(full_bar(stage), L::kStageBytes);
-        const int k_elem = kFp8 ? kb * kBlockKBytes : kb * (kBlockKBytes / 2);
-        tma_load_2d(w_dst, &map_w, full_bar(stage), k_elem, n0);
-        tma_load_2d(w_dst + L::kWBytes, &map_x, full_bar(stage), k_elem, 0);
-        if (++stage == kSwapStages) {
+        if (kb - kb_begin >= early) {
+          if (!mbar_wait(empty_bar(stage), phase ^ 1U, abort_flag)) break;
+          mbar_expect_tx(full_bar(stage), L::kStageBytes);
+          tma_load_2d(w_dst, &map_w, full_bar(stage), k_of(kb), n0);
+        }
+        tma_load_2d(w_dst + L::kWBytes, &map_x, full_bar(stage), k_of(kb), 0);
+        if (++stage == L::kStages) {
           stage = 0;
           phase ^= 1U;
         }
@@ -846,7 +858,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         for (int k = 0; k < kBlockKBytes / 32; ++k)
           tc_mma<kFp8>(tmem_base, w_desc + 2U * k, x_desc + 2U * k, idesc, (kb | k) != 0 ? 1U : 0U);
         tc_commit(empty_bar(stage));
-        if (++stage == kSwapStages) {
+        if (++stage == L::kStages) {
           stage = 0;
           phase ^= 1U;
         }
@@ -965,6 +977,8 @@ gemm_simt_kernel(const void *__restrict__ a_raw, const void *__restrict__ b_raw,
 __global__ void __launch_bounds__(256)
 splitk_finish_kernel(const float *__restrict__ partials, const int splits, const std::size_t partial_stride,
                      const EpilogueParams ep, const int M, const int N) {
+  wait_for_producers(partials);
+  release_dependents();
   const bool gated = ep.gate_mode != 0;
   const int out_columns = gated ? N / 2 : N;
   const std::size_t total = static_cast<std::size_t>(M) * out_columns;
@@ -1154,7 +1168,7 @@ int launch_tc_pair(const void *a, const void *b, const EpilogueParams &ep, const
 
 template <bool kFp8, int BT>
 int launch_swap(const void *x, const void *w, float *partials, const std::size_t M, const std::size_t N,
-                const std::size_t K, const int split, cudaStream_t stream) {
+                const std::size_t K, const int split, const bool dependent, cudaStream_t stream) {
   int status = kOk;
   DeviceState *const state = device_state(&status);
   if (state == nullptr) return status;
@@ -1175,10 +1189,10 @@ int launch_swap(const void *x, const void *w, float *partials, const std::size_t
   }
   const int tiles_n = static_cast<int>((N + kBlockM - 1) / kBlockM);
   const int k_blocks = static_cast<int>(K * (kFp8 ? 1 : 2) / kBlockKBytes);
-  gemm_swap_kernel<kFp8, BT><<<static_cast<unsigned int>(tiles_n * split), kGemmThreads, L::kTotal, stream>>>(
-      map_w, map_x, partials, M * N, static_cast<int>(M), static_cast<int>(N), tiles_n, k_blocks / split,
-      state->error_word);
-  return check_launch("tcgen05 few-token GEMM kernel");
+  return launch_dependent("tcgen05 few-token GEMM kernel", gemm_swap_kernel<kFp8, BT>,
+                          dim3(static_cast<unsigned int>(tiles_n * split)), kGemmThreads, L::kTotal, stream, dependent, 1, map_w,
+                          map_x, partials, M * N, static_cast<int>(M), static_cast<int>(N), tiles_n, k_blocks / split,
+                          state->error_word);
 }
 
 }  // namespace
@@ -1350,7 +1364,8 @@ int linear(const LinearArgs &args, cudaStream_t stream) {
       float *const partials = static_cast<float *>(args.split_workspace);
       const auto launch = [&](auto fp8_tag, auto bt_tag) {
         return launch_swap<decltype(fp8_tag)::value, decltype(bt_tag)::value>(
-            args.input, args.weight, partials, args.rows, args.out_features, args.in_features, split, stream);
+            args.input, args.weight, partials, args.rows, args.out_features, args.in_features, split,
+            args.dependent_launch, stream);
       };
       using F = std::false_type;
       using T = std::true_type;
@@ -1361,10 +1376,10 @@ int linear(const LinearArgs &args, cudaStream_t stream) {
       else status = fp8 ? launch(T{}, std::integral_constant<int, 128>{}) : launch(F{}, std::integral_constant<int, 128>{});
       if (status != kOk) return status;
       const std::size_t outputs = args.rows * out_columns;
-      splitk_finish_kernel<<<static_cast<unsigned int>((outputs + 255) / 256 > 2048 ? 2048 : (outputs + 255) / 256),
-                             256, 0, stream>>>(partials, split, args.rows * args.out_features, ep,
-                                               static_cast<int>(args.rows), static_cast<int>(args.out_features));
-      return check_launch("split-K finishing kernel");
+      return launch_dependent("split-K finishing kernel", splitk_finish_kernel,
+                              dim3(static_cast<unsigned int>((outputs + 255) / 256 > 2048 ? 2048 : (outputs + 255) / 256)), 256,
+                              0, stream, true, 1, static_cast<const float *>(partials), split, args.rows * args.out_features, ep,
+                              static_cast<int>(args.rows), static_cast<int>(args.out_features));
     }
   }
   // (measured: pays off up to a few dozen rows; at 128 rows the partial-sum traffic outweighs it)

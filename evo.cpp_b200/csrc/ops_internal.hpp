@@ -79,7 +79,7 @@ struct LinearArgs {
   // Optional per-row factor [rows] F32 (tile kernel only): the accumulator of row r
   // is multiplied by alpha * row_scale[r] (dynamic per-row activation quantisation).
   const float *row_scale = nullptr;
-  // One-row weight streams only: launch with programmatic stream serialisation, so that the kernel may
+  // Weight streams (one row; up to 128 rows with a split_workspace): launch with programmatic stream serialisation, so that the kernel may
   // start (and fetch the first of its weights) while the kernel in front of it in the stream is still running;
   // it waits for that kernel before it reads the input.  The caller promises that `weight` is not being written
   // by earlier work in the stream.

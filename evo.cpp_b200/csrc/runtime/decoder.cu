@@ -193,7 +193,7 @@ int Context::decoder_linear(Stage &s, const DecoderProduct &p) {
   LinearArgs a;
   a.split_workspace = s.split_workspace;
   a.split_workspace_bytes = kSplitWorkspaceBytes;
-  a.dependent_launch = decode_dependent_launch_ && p.rows == 1;
+  a.dependent_launch = decode_dependent_launch_ && p.rows <= 128;
   a.input = p.input;
   a.weight = p.weight;
   a.output = p.output;

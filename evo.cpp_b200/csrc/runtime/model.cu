@@ -605,7 +605,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       LinearArgs a;
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
-      a.dependent_launch = decode_dependent_launch_ && rows == 1;
+      a.dependent_launch = decode_dependent_launch_ && rows <= 128;
       a.input = fp8 ? s.codes : s.normalized;
       a.weight = w.projection;
       a.output = s.projection;
@@ -814,7 +814,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       LinearArgs a;
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
-      a.dependent_launch = decode_dependent_launch_ && rows == 1;
+      a.dependent_launch = decode_dependent_launch_ && rows <= 128;
       a.input = s.mixer_out;
       a.weight = w.out_weight;
       a.bias = w.out_bias;
@@ -856,7 +856,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       LinearArgs a;
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
-      a.dependent_launch = decode_dependent_launch_ && rows == 1;
+      a.dependent_launch = decode_dependent_launch_ && rows <= 128;
       a.input = s.normalized;
       a.weight = w.l12;
       a.output = s.gated;
@@ -897,7 +897,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       LinearArgs a;
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
-      a.dependent_launch = decode_dependent_launch_ && rows == 1;
+      a.dependent_launch = decode_dependent_launch_ && rows <= 128;
       a.input = s.gated;
       a.weight = w.l3;
       a.residual = s.residual;
@@ -1078,7 +1078,7 @@ int Context::forward(const std::uint32_t *host_tokens, const std::uint32_t *devi
       LinearArgs a;
       a.split_workspace = first.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
-      a.dependent_launch = decode_dependent_launch_ && rows == 1;
+      a.dependent_launch = decode_dependent_launch_ && rows <= 128;
       a.input = first.normalized;
       a.weight = first.weights->embedding;  // tied head
       a.output = first.logits;
