@@ -364,7 +364,8 @@ rms_norm_kernel(const bf16 *__restrict__ input, const float *__restrict__ scale,
 // in a row (gains, row, next row) and the generic one two.  A thread owns columns t, t + 256, ... in
 // registers: exactly the terms of its partial sum in row_denominator's order, and the columns it
 // normalises and stores (neighbouring threads write neighbouring columns).
-template <int kPerThread>
+// kWhole: the width is kPerThread x 256; otherwise less, and the columns past it count as zeros.
+template <int kPerThread, bool kWhole>
 __global__ void __launch_bounds__(kThreads)
 rms_norm_few_rows_kernel(const bf16 *__restrict__ input, const float *__restrict__ scale,
                          bf16 *__restrict__ output, std::uint8_t *__restrict__ codes, const int width,
@@ -377,9 +378,15 @@ rms_norm_few_rows_kernel(const bf16 *__restrict__ input, const float *__restrict
   unsigned short raw[kPerThread];
   float gain[kPerThread];
 #pragma unroll
-  for (int k = 0; k < kPerThread; ++k) gain[k] = scale[threadIdx.x + k * kThreads];
+  for (int k = 0; k < kPerThread; ++k) {
+    const int column = threadIdx.x + k * kThreads;
+    gain[k] = kWhole || column < width ? scale[column] : 0.0F;
+  }
 #pragma unroll
-  for (int k = 0; k < kPerThread; ++k) raw[k] = in[threadIdx.x + k * kThreads];
+  for (int k = 0; k < kPerThread; ++k) {
+    const int column = threadIdx.x + k * kThreads;
+    raw[k] = kWhole || column < width ? in[column] : static_cast<unsigned short>(0);
+  }
   float sum = 0.0F;
 #pragma unroll
   for (int k = 0; k < kPerThread; ++k) {
@@ -405,6 +412,7 @@ rms_norm_few_rows_kernel(const bf16 *__restrict__ input, const float *__restrict
 #pragma unroll
   for (int k = 0; k < kPerThread; ++k) {
     const std::size_t column = threadIdx.x + k * kThreads;
+    if (!kWhole && column >= static_cast<std::size_t>(width)) break;
     const bf16 result = f2bf(rbf(__fdiv_rn(bits2f_bf16(raw[k]), denominator)) * rbf(gain[k]));
     if (output != nullptr) output[row * width + column] = result;
     if (codes != nullptr) codes[row * width + column] = e4m3_code(bf2f(result) * quant_scale);
@@ -717,21 +725,26 @@ int rms_norm(const void *input, const float *scale, const std::size_t rows,
   };
   const bool vectors = width % 8 == 0 && aligned(input, 15) && aligned(scale, 15) &&
                        (output == nullptr || aligned(output, 15)) && (codes == nullptr || aligned(codes, 7));
-  if (rows <= 8 && width % kThreads == 0) {
+  // (61 rows of 4096: 3.4 us against 5.5 with the streaming kernel, one row of 1920: 2.5 against 5.3; beyond a block per SM
+  // the streaming kernel's prefetch wins)
+  if (rows <= kSmCount && width <= 32 * kThreads) {
     const auto launch_few = [&](auto kernel) {
       return launch_dependent("RMSNorm kernel", kernel, dim3(static_cast<unsigned int>(rows)), kThreads, 0, stream, true, 1,
                               static_cast<const bf16 *>(input), scale, static_cast<bf16 *>(output),
                               static_cast<std::uint8_t *>(codes), static_cast<int>(width), epsilon, quant_scale);
     };
-    switch (width / kThreads) {
-      case 1: return launch_few(rms_norm_few_rows_kernel<1>);
-      case 2: return launch_few(rms_norm_few_rows_kernel<2>);
-      case 4: return launch_few(rms_norm_few_rows_kernel<4>);
-      case 8: return launch_few(rms_norm_few_rows_kernel<8>);     // 2048
-      case 16: return launch_few(rms_norm_few_rows_kernel<16>);   // 4096
-      case 32: return launch_few(rms_norm_few_rows_kernel<32>);   // 8192
-      default: break;
-    }
+    const auto launch_width = [&](auto per_thread) {
+      constexpr int kPer = decltype(per_thread)::value;
+      return width == static_cast<std::size_t>(kPer) * kThreads ? launch_few(rms_norm_few_rows_kernel<kPer, true>)
+                                                                : launch_few(rms_norm_few_rows_kernel<kPer, false>);
+    };
+    const std::size_t per_thread = (width + kThreads - 1) / kThreads;
+    if (per_thread <= 1) return launch_width(std::integral_constant<int, 1>{});
+    if (per_thread <= 2) return launch_width(std::integral_constant<int, 2>{});
+    if (per_thread <= 4) return launch_width(std::integral_constant<int, 4>{});
+    if (per_thread <= 8) return launch_width(std::integral_constant<int, 8>{});     // 1920, 2048
+    if (per_thread <= 16) return launch_width(std::integral_constant<int, 16>{});   // 4096
+    return launch_width(std::integral_constant<int, 32>{});                         // 8192
   }
   if (vectors) {
     const std::size_t smem = 3 * width * sizeof(unsigned short);
