@@ -13,8 +13,9 @@
 //   lane 0       direct term, post-gate, store.
 // Every product, sum and rounding is the one the unfused kernels make, in the
 // same order (upstream pins them: src/cuda/hyena.cu:275-416 for the FIR steps,
-// :718-761 for the modal step), so the results are bit-identical.  Histories
-// must be full (position >= taps - 1); shorter histories take the unfused path.
+// :718-761 for the modal step), so the results are bit-identical.  A history that
+// is not full yet holds its entries at its end; its oldest one is entry 0 of the
+// sums and meets tap 0 (cross-correlation) or the last tap in reach.
 #include "common.cuh"
 #include "ops_internal.hpp"
 
@@ -30,6 +31,7 @@ struct Params {
   float *short_cache, *inner_cache, *modal_state;
   bf16 *output;
   int width, channels_per_group, taps, modes;
+  int short_cached, inner_cached;  // valid entries of the histories, at their ends
   bool filter_is_f32, cross_correlation;
 };
 
@@ -54,10 +56,11 @@ mixer_decode_kernel(const Params p) {
     const float older = row[0], newer = row[1];
     const bf16 *const w = p.short_filter + column * 3;
     // slots 0 and 1 of the 32-slot tree; the other slots are +0 and only matter for the sign of zero
-    const float t0 = __fadd_rn(0.0F, __fmul_rn(older, bf2f(w[0])));
-    const float t1 = __fadd_rn(0.0F, __fmul_rn(newer, bf2f(w[1])));
+    const float entry0 = p.short_cached == 2 ? older : newer;
+    const float t0 = p.short_cached > 0 ? __fadd_rn(0.0F, __fmul_rn(entry0, bf2f(w[0]))) : 0.0F;
+    const float t1 = p.short_cached == 2 ? __fadd_rn(0.0F, __fmul_rn(newer, bf2f(w[1]))) : 0.0F;
     const float current = bf2f(p.projection[column]);
-    z = rbf(__fadd_rn(__fmul_rn(current, bf2f(w[2])), __fadd_rn(t0, t1)));
+    z = rbf(__fadd_rn(__fmul_rn(current, bf2f(w[p.short_cached])), __fadd_rn(t0, t1)));
     row[0] = newer;
     row[1] = current;
   }
@@ -87,14 +90,15 @@ mixer_decode_kernel(const Params p) {
     const int cache_size = p.taps - 1;
     const std::size_t group = channel / p.channels_per_group;
     float *const row = p.inner_cache + static_cast<std::size_t>(channel) * cache_size;
+    const int active = p.inner_cached, first = cache_size - active;  // (the entries in front are zeros and stay)
     float history[4];  // taps <= 128
     float term = 0.0F;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int a = 32 * k + lane;
-      history[k] = a < cache_size ? row[a] : 0.0F;
-      if (a < cache_size) {
-        const int tap = p.cross_correlation ? a : cache_size - a;
+      history[k] = a < active ? row[first + a] : 0.0F;
+      if (a < active) {
+        const int tap = p.cross_correlation ? a : active - a;
         term = __fadd_rn(term, __fmul_rn(history[k], filter_tap(p.filter, p.filter_is_f32, group * p.taps + tap)));
       }
     }
@@ -107,11 +111,11 @@ mixer_decode_kernel(const Params p) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int a = 32 * k + lane;
-      if (a >= 1 && a < cache_size) row[a - 1] = history[k];
+      if (first + a >= 1 && a < active) row[first + a - 1] = history[k];
     }
     if (lane == 0) {
       row[cache_size - 1] = gated;
-      const int current_tap = p.cross_correlation ? cache_size : 0;
+      const int current_tap = p.cross_correlation ? active : 0;
       float total =
           __fadd_rn(__fmul_rn(gated, filter_tap(p.filter, p.filter_is_f32, group * p.taps + current_tap)), term);
       if (p.direct != nullptr) total = __fadd_rn(total, __fmul_rn(bf2f(p.direct[channel]), gated));
@@ -147,6 +151,8 @@ int hyena_decode_mixer(const DecodeMixerArgs &a, cudaStream_t stream) {
   p.channels_per_group = modal ? 1 : static_cast<int>(a.width / a.groups);
   p.taps = static_cast<int>(a.taps);
   p.modes = static_cast<int>(a.modes);
+  p.short_cached = static_cast<int>(a.position < 2 ? a.position : 2);
+  p.inner_cached = modal ? 0 : static_cast<int>(a.position < a.taps - 1 ? a.position : a.taps - 1);
   p.filter_is_f32 = a.filter_is_f32;
   p.cross_correlation = a.cross_correlation;
   const unsigned int grid = ceil_div_u(a.width * 32, kThreads);

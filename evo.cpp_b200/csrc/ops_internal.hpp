@@ -242,6 +242,7 @@ struct DecodeMixerArgs {
   float *modal_state = nullptr;        // [width, modes] F32, advanced
   void *output = nullptr;              // [width] BF16
   std::size_t width = 0;
+  std::size_t position = ~std::size_t{0};  // tokens seen: what the histories hold until they are full
 };
 int hyena_decode_mixer(const DecodeMixerArgs &args, cudaStream_t stream);
 int modal_decode(const void *x2, const void *x1, const void *value,

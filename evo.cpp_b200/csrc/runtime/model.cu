@@ -739,10 +739,10 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
           return fail(kCuda, "projection history save failed");
       }
     } else if (mode == Mode::kDecode && rows == 1 && c.short_taps == 3 && tap == nullptr &&
-               position_ >= std::max({c.short_taps, c.hcs_taps, c.hcm_taps}) &&
                (w.type == MixerType::kHcl ? c.state_size <= 32 : (w.type == MixerType::kHcs ? c.hcs_taps : c.hcm_taps) <= 128)) {
-      // one token against full histories: the whole mixer in one launch
+      // one token against the histories: the whole mixer in one launch
       DecodeMixerArgs a;
+      a.position = position_;
       a.projection = s.projection;
       a.short_filter = w.short_filter;
       a.short_cache = state.short_cache;

@@ -162,3 +162,17 @@ def test_decode_taps_and_error_paths(rt, model):
     assert aborted.value.code == 3
     with pytest.raises(rt.EvoError):
         failing.prefill(sequence)
+
+
+@pytest.mark.parametrize("prompt", [1, 2, 3, 7])
+def test_steps_on_histories_that_fill(rt, model, prompt):
+    """The one-launch mixers against the separate operators (which tapped blocks take), bit for bit, from the first step
+    behind a short prompt until the longest history (127 rows) is full."""
+    rng = np.random.default_rng(prompt)
+    tokens = [int(t) for t in rng.choice(np.frombuffer(b"ACGT", np.uint8), prompt + 134)]
+    whole, tapped = model.context(512), model.context(512)
+    assert np.array_equal(whole.prefill_tokens(tokens[:prompt]), tapped.prefill_tokens(tokens[:prompt]))
+    taps = [(layer, "mixer_output") for layer in range(LAYERS)]
+    for at, token in enumerate(tokens[prompt:]):
+        step, _ = tapped.decode_with_dumps(token, taps)
+        assert np.array_equal(whole.decode(token), step), at
