@@ -164,9 +164,9 @@ gemv_kernel(const GemvParams p) {
   // instructions do nothing.
   const bool grouped = p.row_group != nullptr;
   if (grouped) {
-    // which weights these are is a result of the kernel in front
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // which weights these are is a result of the kernel in front; the one behind may rely on it (row_group_settled)
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     wb += static_cast<std::size_t>(p.row_group[blockIdx.y]) * p.N * row_bytes;
     xb += static_cast<std::size_t>(blockIdx.y / p.row_fanout) * row_bytes;
   } else if (p.dependent_launch != 0) {

@@ -419,7 +419,7 @@ class Context {
   static constexpr std::size_t kStepRow = 4;
   const int *dynamic_position_ = nullptr; // == device_position_ while the graph is being recorded
   bool decode_graph_allowed_ = true;
-  // one-row projections are launched with programmatic stream serialisation (EVO_B200_DECODE_PDL=0: plain launches)
+  // projections of up to 128 rows are launched with programmatic stream serialisation (EVO_B200_DECODE_PDL=0: plainly)
   bool decode_dependent_launch_ = true;
 
   std::shared_ptr<ModelWeights> weights_;
