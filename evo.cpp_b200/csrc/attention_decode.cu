@@ -59,7 +59,7 @@ attention_decode_kernel(const bf16 *__restrict__ query, const bf16 *__restrict__
                         const bf16 *__restrict__ value_cache, const Q8PageTable pages, bf16 *__restrict__ output,
                         const int rows, const int static_total_keys, const int heads,
                         const int *__restrict__ dynamic_prefix) {
-  wait_for_producers(query, key_cache, value_cache, output, dynamic_prefix);
+  wait_for_producers(query, key_cache, value_cache, dynamic_prefix);
   release_dependents();
   // replayed launches (CUDA graphs) read the number of keys already cached from device memory
   const int total_keys = dynamic_prefix != nullptr ? *dynamic_prefix + rows : static_total_keys;

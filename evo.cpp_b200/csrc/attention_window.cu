@@ -29,7 +29,7 @@ head_norm_append_kernel(const T *__restrict__ projection, const std::size_t stri
                         T *__restrict__ value_cache, const int static_position,
                         const int *__restrict__ dynamic_position, const int capacity, const int heads,
                         const int kv_heads, const int dim, const int value_dim, const float epsilon) {
-  wait_for_producers(projection, query, key_cache, value_cache, dynamic_position);
+  wait_for_producers(projection, dynamic_position);
   release_dependents();
   const std::size_t row = blockIdx.x;
   const std::size_t at = (dynamic_position != nullptr ? *dynamic_position : static_position) + row;
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kRowThreads)
 window_attention_row_kernel(const T *__restrict__ query, const T *__restrict__ key_cache,
                             const T *__restrict__ value_cache, const T *__restrict__ gate, T *__restrict__ output,
                             const RowParams p) {
-  wait_for_producers(query, key_cache, value_cache, gate, output);
+  wait_for_producers(query, key_cache, value_cache, gate);
   release_dependents();
   constexpr int kWidth = kElements * kLanes, kGroups = 32 / kLanes;  // keys that a warp takes at once
   __shared__ float warp_partials[kRowWarps][kWidth + 2];

@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kThreads)
 rms_norm_few_rows_kernel(const bf16 *__restrict__ input, const float *__restrict__ scale,
                          bf16 *__restrict__ output, std::uint8_t *__restrict__ codes, const int width,
                          const float epsilon, const float quant_scale) {
-  wait_for_producers(input, scale, output, codes);
+  wait_for_producers(input, scale);
   release_dependents();
   __shared__ float partial[32];
   const std::size_t row = blockIdx.x;
@@ -432,7 +432,7 @@ rms_norm_stream_kernel(const bf16 *__restrict__ input, const float *__restrict__
   extern __shared__ __align__(16) unsigned short row_cache[];  // 2 x width BF16 values, then width BF16 scales
   __shared__ float partial[32];
   const std::size_t width = kWidth != 0 ? static_cast<std::size_t>(kWidth) : runtime_width;
-  wait_for_producers(input, scale, output, codes);
+  wait_for_producers(input, scale);
   release_dependents();
   std::uint32_t *const scale_pairs = reinterpret_cast<std::uint32_t *>(row_cache + 2 * width);
   for (std::size_t i = threadIdx.x; i < width / 2; i += kThreads)
@@ -518,7 +518,7 @@ __global__ void pointwise_kernel(const bf16 *__restrict__ first,
                                  const bf16 *__restrict__ second,
                                  bf16 *__restrict__ output,
                                  const std::size_t elements) {
-  wait_for_producers(first, second, output);
+  wait_for_producers(first, second);
   release_dependents();
   const std::size_t vectors = elements / 8;
   const std::size_t stride = static_cast<std::size_t>(blockDim.x) * gridDim.x;
@@ -586,7 +586,7 @@ __global__ void embedding_kernel(const std::uint32_t *__restrict__ tokens,
                                  const std::size_t width,
                                  const std::size_t vocabulary,
                                  int *const error_word) {
-  wait_for_producers(tokens, output);
+  wait_for_producers(tokens);
   release_dependents();
   const std::size_t elements = rows * width;
   const std::size_t stride = static_cast<std::size_t>(blockDim.x) * gridDim.x;
@@ -609,7 +609,7 @@ __global__ void embedding_kernel(const std::uint32_t *__restrict__ tokens,
 __global__ void __launch_bounds__(kThreads)
 embedding_vector_kernel(const std::uint32_t *__restrict__ tokens, const uint4 *__restrict__ table, uint4 *__restrict__ output,
                         const std::size_t rows, const std::uint32_t vectors, const std::size_t vocabulary, int *const error_word) {
-  wait_for_producers(tokens, output);
+  wait_for_producers(tokens);
   release_dependents();
   for (std::size_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const std::size_t id = tokens[row];
@@ -625,7 +625,7 @@ __global__ void split_triples_kernel(const bf16 *__restrict__ projection,
                                      bf16 *__restrict__ x1,
                                      bf16 *__restrict__ value,
                                      const std::size_t elements) {
-  wait_for_producers(projection, x2, x1, value);
+  wait_for_producers(projection);
   release_dependents();
   const std::size_t stride = static_cast<std::size_t>(blockDim.x) * gridDim.x;
   for (std::size_t i = static_cast<std::size_t>(blockIdx.x) * blockDim.x +
