@@ -73,7 +73,7 @@ split_rope_append_vec_kernel(const bf16 *__restrict__ qkv, const float *__restri
                              const std::size_t heads, const std::size_t head_dim,
                              const std::size_t static_position_offset, const float position_scale,
                              const bool head_major, const int *__restrict__ dynamic_position) {
-  wait_for_producers(qkv, dynamic_position);
+  wait_for_producers(qkv, inverse_frequency, dynamic_position);
   release_dependents();
   // replayed launches (CUDA graphs) read the position from device memory
   const std::size_t position_offset =

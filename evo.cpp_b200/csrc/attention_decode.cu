@@ -81,7 +81,7 @@ attention_decode_kernel(const bf16 *__restrict__ query, const bf16 *__restrict__
   {
     const uint4 *const source = reinterpret_cast<const uint4 *>(
         query + static_cast<std::size_t>(row) * width + head * kHeadDim + part * 16);
-    unpack16(__ldg(source), __ldg(source + 1), q);
+    unpack16(source[0], source[1], q);
   }
   float running_max = -INFINITY, running_sum = 0.0F;
   float acc[16];
@@ -96,14 +96,14 @@ attention_decode_kernel(const bf16 *__restrict__ query, const bf16 *__restrict__
       if constexpr (kQ8) {
         const std::size_t page = static_cast<std::size_t>(key) / pages.page_tokens;
         const std::size_t slot = (static_cast<std::size_t>(key) % pages.page_tokens) * heads + head;
-        const uint4 kc = __ldg(reinterpret_cast<const uint4 *>(pages.key[page] + slot * kHeadDim + part * 16));
-        const uint4 vc = __ldg(reinterpret_cast<const uint4 *>(pages.value[page] + slot * kHeadDim + part * 16));
-        unpack16_q8(kc, __ldg(pages.key_scale[page] + slot), k);
-        unpack16_q8(vc, __ldg(pages.value_scale[page] + slot), v);
+        const uint4 kc = *reinterpret_cast<const uint4 *>(pages.key[page] + slot * kHeadDim + part * 16);
+        const uint4 vc = *reinterpret_cast<const uint4 *>(pages.value[page] + slot * kHeadDim + part * 16);
+        unpack16_q8(kc, pages.key_scale[page][slot], k);
+        unpack16_q8(vc, pages.value_scale[page][slot], v);
       } else {
         const uint4 *const kp = reinterpret_cast<const uint4 *>(key_cache + static_cast<std::size_t>(key) * width + lane_offset);
         const uint4 *const vp = reinterpret_cast<const uint4 *>(value_cache + static_cast<std::size_t>(key) * width + lane_offset);
-        const uint4 k0 = __ldg(kp), k1 = __ldg(kp + 1), v0 = __ldg(vp), v1 = __ldg(vp + 1);
+        const uint4 k0 = kp[0], k1 = kp[1], v0 = vp[0], v1 = vp[1];
         unpack16(k0, k1, k);
         unpack16(v0, v1, v);
       }

@@ -29,7 +29,7 @@ head_norm_append_kernel(const T *__restrict__ projection, const std::size_t stri
                         T *__restrict__ value_cache, const int static_position,
                         const int *__restrict__ dynamic_position, const int capacity, const int heads,
                         const int kv_heads, const int dim, const int value_dim, const float epsilon) {
-  wait_for_producers(projection, dynamic_position);
+  wait_for_producers(projection, query_gain, key_gain, dynamic_position);
   release_dependents();
   const std::size_t row = blockIdx.x;
   const std::size_t at = (dynamic_position != nullptr ? *dynamic_position : static_position) + row;
@@ -108,7 +108,7 @@ struct ScoreParams {
 __device__ __forceinline__ float capped_score(const float dot, const ScoreParams &p, const int distance) {
   float s = dot * p.scale;
   if (p.softcap > 0.0F) s = p.softcap * tanhf(s / p.softcap);
-  if (p.bias != nullptr) s -= __ldg(p.bias + distance);
+  if (p.bias != nullptr) s -= p.bias[distance];
   return s;
 }
 

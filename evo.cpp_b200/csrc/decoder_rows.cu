@@ -80,7 +80,7 @@ embed_positions_kernel(const std::uint32_t *__restrict__ tokens, const bf16 *__r
                        const bf16 *__restrict__ positions, const float *__restrict__ gain, const int width,
                        const std::uint32_t vocabulary, const int position, const int *__restrict__ dynamic_position,
                        const float epsilon, float *__restrict__ output, int *const error_word) {
-  wait_for_producers(tokens, dynamic_position);
+  wait_for_producers(tokens, table, positions, gain, dynamic_position);
   release_dependents();
   __shared__ float scratch[kThreads / 32];
   const std::size_t row = blockIdx.x;
@@ -117,7 +117,7 @@ template <typename T, bool kVector>
 __global__ void __launch_bounds__(kThreads)
 rms_norm_residual_kernel(const float *__restrict__ input, const float *__restrict__ gain, const int width,
                          const float epsilon, T *__restrict__ output) {
-  wait_for_producers(input);
+  wait_for_producers(input, gain);
   release_dependents();
   __shared__ float scratch[kThreads / 32];
   const float *const x = input + static_cast<std::size_t>(blockIdx.x) * width;
@@ -138,7 +138,7 @@ template <typename T, bool kVector>
 __global__ void __launch_bounds__(kThreads)
 poly_norm_kernel(const T *input, const float *__restrict__ coefficients, const int width, const float epsilon,
                  T *output) {
-  wait_for_producers(input, output);
+  wait_for_producers(input, coefficients, output);
   release_dependents();
   __shared__ float scratch[kThreads / 32];
   const T *const z = input + static_cast<std::size_t>(blockIdx.x) * width;
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kThreads)
 embed_rows_kernel(const std::uint32_t *__restrict__ tokens, const bf16 *__restrict__ table, const int width,
                   const std::uint32_t vocabulary, float *__restrict__ stream_rows, T *__restrict__ copy,
                   int *const error_word) {
-  wait_for_producers(tokens);
+  wait_for_producers(tokens, table);
   release_dependents();
   const std::size_t row = blockIdx.x;
   const std::uint32_t token = tokens[row];

@@ -262,8 +262,8 @@ __device__ __forceinline__ void store_normalized_row(const unsigned short *row_c
   const float reciprocal = __frcp_rn(denominator);
   const auto load = [&](const int v, Bf16x8 &values, float (&scales)[8]) {
     values.raw = reinterpret_cast<const uint4 *>(row_cache)[v];
-    const float4 s0 = __ldg(reinterpret_cast<const float4 *>(scale) + 2 * v);
-    const float4 s1 = __ldg(reinterpret_cast<const float4 *>(scale) + 2 * v + 1);
+    const float4 s0 = reinterpret_cast<const float4 *>(scale)[2 * v];
+    const float4 s1 = reinterpret_cast<const float4 *>(scale)[2 * v + 1];
     scales[0] = s0.x; scales[1] = s0.y; scales[2] = s0.z; scales[3] = s0.w;
     scales[4] = s1.x; scales[5] = s1.y; scales[6] = s1.z; scales[7] = s1.w;
   };
@@ -586,7 +586,7 @@ __global__ void embedding_kernel(const std::uint32_t *__restrict__ tokens,
                                  const std::size_t width,
                                  const std::size_t vocabulary,
                                  int *const error_word) {
-  wait_for_producers(tokens);
+  wait_for_producers(tokens, table);
   release_dependents();
   const std::size_t elements = rows * width;
   const std::size_t stride = static_cast<std::size_t>(blockDim.x) * gridDim.x;
@@ -609,7 +609,7 @@ __global__ void embedding_kernel(const std::uint32_t *__restrict__ tokens,
 __global__ void __launch_bounds__(kThreads)
 embedding_vector_kernel(const std::uint32_t *__restrict__ tokens, const uint4 *__restrict__ table, uint4 *__restrict__ output,
                         const std::size_t rows, const std::uint32_t vectors, const std::size_t vocabulary, int *const error_word) {
-  wait_for_producers(tokens);
+  wait_for_producers(tokens, table);
   release_dependents();
   for (std::size_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const std::size_t id = tokens[row];

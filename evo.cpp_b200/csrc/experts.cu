@@ -79,7 +79,7 @@ route_logits_kernel(const float *__restrict__ logits, const std::size_t stride, 
 template <typename T, bool kVector, int kPerLane>
 __global__ void __launch_bounds__(32 * kRouteWarps)
 route_rows_kernel(const T *__restrict__ input, const bf16 *__restrict__ router, const int width, const Choice c) {
-  wait_for_producers(input);
+  wait_for_producers(input, router);
   release_dependents();
   __shared__ float logits[kDecoderMaxExperts / kRouterSplits + kRouteWarps];  // of this CTA's experts
   cg::cluster_group cluster = cg::this_cluster();

@@ -165,9 +165,10 @@ gemv_kernel(const GemvParams p) {
   const bool grouped = p.row_group != nullptr;
   if (grouped) {
     // which weights these are is a result of the kernel in front; the one behind may rely on it (row_group_settled)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    wb += static_cast<std::size_t>(p.row_group[blockIdx.y]) * p.N * row_bytes;
+    const int *row_group = p.row_group;
+    wait_for_producers(xb, row_group);
+    release_dependents();
+    wb += static_cast<std::size_t>(row_group[blockIdx.y]) * p.N * row_bytes;
     xb += static_cast<std::size_t>(blockIdx.y / p.row_fanout) * row_bytes;
   } else if (p.dependent_launch != 0) {
     for (int chunk = threadIdx.x * 8; chunk < chunks; chunk += kThreads * 8) {  // one request per 128-byte line
@@ -175,8 +176,8 @@ gemv_kernel(const GemvParams p) {
       for (int c = 0; c < kColumns; ++c)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(wb + weight_row[c] * row_bytes + static_cast<std::size_t>(chunk) * 16));
     }
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    release_dependents();
+    wait_for_producers(xb);
   }
 #pragma unroll(kRows == 1 ? 4 : (kRows == 2 ? 2 : 1))
   for (int chunk = threadIdx.x; chunk < chunks; chunk += kThreads) {
@@ -188,7 +189,7 @@ gemv_kernel(const GemvParams p) {
     for (int r = 0; r < kRows; ++r) {
       if (r < p.rows) {
         float xv[kPerChunk];
-        unpack16<kFp8>(__ldg(reinterpret_cast<const uint4 *>(xb + r * row_bytes) + chunk), xv);
+        unpack16<kFp8>(reinterpret_cast<const uint4 *>(xb + r * row_bytes)[chunk], xv);
 #pragma unroll
         for (int c = 0; c < kColumns; ++c) {
           float wv[kPerChunk];

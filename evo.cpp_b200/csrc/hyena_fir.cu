@@ -338,7 +338,7 @@ fir_rows_warp_kernel(const bf16 *__restrict__ input, const void *__restrict__ fi
                      bf16 *__restrict__ output, const std::size_t length, const std::size_t channels,
                      const std::size_t channels_per_group, const int taps, const int cached,
                      const bool cross_correlation) {
-  wait_for_producers(input, cache);
+  wait_for_producers(input, filter, bias, cache);
   release_dependents();
   const std::size_t item = (static_cast<std::size_t>(blockIdx.x) * kThreads + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;

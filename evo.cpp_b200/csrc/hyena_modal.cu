@@ -54,7 +54,7 @@ modal_decode_warp_kernel(const bf16 *__restrict__ x2, const bf16 *__restrict__ x
                          const bf16 *__restrict__ direct, const float *__restrict__ log_poles,
                          const float *__restrict__ residues, float *__restrict__ state, bf16 *__restrict__ pregate,
                          bf16 *__restrict__ output, const int width, const int modes) {
-  wait_for_producers(x2, x1, value, state);
+  wait_for_producers(x2, x1, value, direct, log_poles, residues, state);
   release_dependents();
   const int channel = (blockIdx.x * kDecodeThreads + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;

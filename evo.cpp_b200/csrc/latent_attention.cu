@@ -109,7 +109,7 @@ template <typename T, int kVec, int kRows>
 __global__ void __launch_bounds__(kThreads)
 absorb_kernel(const T *__restrict__ query, const bf16 *__restrict__ key_up, T *__restrict__ absorbed, const int rows,
               const int heads, const int dim, const int rank) {
-  wait_for_producers(query);
+  wait_for_producers(query, key_up);
   release_dependents();
   constexpr int kColumns = 8 * kVec;
   __shared__ float partial[kWarps][kRows][kColumns];
@@ -160,7 +160,7 @@ template <typename T, int kVec, int kRows>
 __global__ void __launch_bounds__(kThreads)
 expand_kernel(const T *__restrict__ mixed, const bf16 *__restrict__ value_up, T *__restrict__ output, const int rows,
               const int heads, const int value_dim, const int rank) {
-  wait_for_producers(mixed);
+  wait_for_producers(mixed, value_up);
   release_dependents();
   const int head = blockIdx.x, column = blockIdx.y * kWarps + threadIdx.x / 32, lane = threadIdx.x % 32;
   if (column >= value_dim) return;

@@ -623,7 +623,7 @@ decode_kernel(const T *__restrict__ projection, T *const history, const float *_
               const float *__restrict__ decay_rate, const float *__restrict__ decay_shift,
               const float *__restrict__ decay_weight, const float *__restrict__ decay_bias,
               const float *__restrict__ gain, float *const state, T *__restrict__ output, const DecodeParams p) {
-  wait_for_producers(projection);
+  wait_for_producers(projection, conv, decay_rate, decay_shift, decay_weight, decay_bias, gain);
   release_dependents();
   __shared__ float key[kDecoderMaxHeadDim], query[kDecoderMaxHeadDim], alpha[kDecoderMaxHeadDim];
   __shared__ float partial[2][kDecodeWarps][32], scratch[kDecodeWarps];
