@@ -487,7 +487,7 @@ linear_f32_tile_kernel(const T *__restrict__ input, const F32Params p) {
   cluster.sync();  // remote shared memory stays alive until every CTA has read it
 }
 
-// Few rows of grouped weights: a warp per (row, output).
+// Few rows: a warp per (row, output).
 template <typename T, bool kVector>
 __global__ void __launch_bounds__(256)
 linear_f32_rows_kernel(const T *__restrict__ input, const F32Params p) {
@@ -495,7 +495,7 @@ linear_f32_rows_kernel(const T *__restrict__ input, const F32Params p) {
   if (column >= p.out_features) return;
   const std::size_t row = blockIdx.y;
   const T *const x = input + row / p.row_fanout * p.in_features;
-  const std::size_t group = static_cast<std::size_t>(p.row_group[row]);
+  const std::size_t group = p.row_group != nullptr ? static_cast<std::size_t>(p.row_group[row]) : 0;
   const bf16 *const w = p.weight + (group * p.out_features + column) * p.in_features;
   float sum = 0.0F;
   if constexpr (kVector) {
@@ -691,10 +691,17 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
   p.tile_count = a.tile_count;
   p.tile_rows = static_cast<int>(a.tile_rows);
   const bool vector = a.in_features % 8 == 0 && aligned16(a.input) && aligned16(a.weight);
+  // Every row of the few-row kernel fetches the weights again, from L2 where they fit.  The tile kernel fetches them once,
+  // for 32 rows or more, and its steps wait for memory: 2 rows of 2048 x 8448 take 18 us against 90, 12 rows 72 against 90,
+  // 16 rows of 8448 x 2048 90 against 136, of 2048 x 8448 92 against 91; but 16 rows of 4096 x 22528 (185 MB) 520 against 397.
+  constexpr std::size_t kL2Weights = std::size_t{96} << 20;
+  const bool few_rows = a.row_group != nullptr ||
+                        (a.tile_group == nullptr &&
+                         (a.rows <= 12 || (a.rows <= 16 && a.in_features * a.out_features * 2 <= kL2Weights)));
   const auto launch = [&](auto tag) {
     using T = decltype(tag);
     const T *const input = static_cast<const T *>(a.input);
-    if (a.row_group != nullptr) {
+    if (few_rows) {
       const auto kernel = vector ? linear_f32_rows_kernel<T, true> : linear_f32_rows_kernel<T, false>;
       return launch_dependent("F32 linear kernel (few rows)", kernel,
                               dim3(ceil_div_u(a.out_features, 8), static_cast<unsigned int>(a.rows)), 256, 0, stream, false, 1,

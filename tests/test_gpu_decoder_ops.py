@@ -130,6 +130,43 @@ def test_f32_products(ops, rows, inner, outer):
     assert np.all(error <= chain * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(wv).T + np.abs(base)))
 
 
+@pytest.mark.parametrize("rows, inner, outer", [(1, 1001, 40), (1, 16400, 9), (2, 8, 5), (3, 1111, 70), (12, 2056, 150), (13, 2056, 150),
+                                                (16, 100, 129), (16, 520, 260), (17, 520, 260), (13, 8192, 6400), (12, 8192, 6400)])
+def test_few_f32_rows(ops, rows, inner, outer):
+    """Both sides of the line between a warp per output and the tiles, whole and ragged, and weights on either side of L2.
+    A lane of the former adds 8 ceil(inner / 256) products (single ones: ceil(inner / 32)), five lanes' sums and the base."""
+    rng = np.random.default_rng(rows * 1000 + inner)
+    w, wv = activation(rng.normal(0, 1, (outer, inner)), 0)
+    x, base = (rng.normal(0, 1, shape).astype(np.float32) for shape in ((rows, inner), (rows, outer)))
+    exact, out = cuda(x), cuda(base)
+    ops.call("f32_linear", exact.data_ptr(), w.data_ptr(), rows, inner, outer, 1, out.data_ptr(), stream())
+    error = np.abs(out.double().cpu().numpy() - (x.astype(np.float64) @ wv.T + base))
+    chain = 16 * (-(-inner // 256) + 4)  # of the tiles; the lanes' is shorter
+    assert np.all(error <= chain * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(wv).T + np.abs(base)))
+
+
+def test_few_f32_rows_cost_less_than_a_tile(ops):
+    """Two rows are a stream of the weights; a tile pads them to 32 (18 us against 90 at this size)."""
+    import torch
+
+    w = torch.randn(8448, 2048, device="cuda").bfloat16()
+
+    def microseconds(rows):
+        x, out = torch.randn(rows, 2048, device="cuda"), torch.empty(rows, 8448, device="cuda")
+        times = []
+        for _ in range(12):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            begin.record()
+            for _ in range(10):
+                ops.call("f32_linear", x.data_ptr(), w.data_ptr(), rows, 2048, 8448, 0, out.data_ptr(), stream())
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times)
+
+    assert microseconds(2) < 0.5 * microseconds(32)
+
+
 # ---------------------------------------------------------------- attention
 def window_case(pkg, ops, *, rows, position, heads, kv_heads, dim, vdim, window, keep_first, kernel, float32=0, softcap=15.0,
                 sink=1, gated=True, biased=True, seed=0, edit=None):
