@@ -63,6 +63,7 @@ struct LinearF32Args {
   const int *tile_group = nullptr, *tile_count = nullptr;
   std::size_t tile_rows = 128;
   bool dependent_launch = false;  // one row: as LinearArgs::dependent_launch
+  bool weight_stream = false;     // as LinearArgs::weight_stream
   RowFront front;                 // one row
 };
 int linear_f32(const LinearF32Args &args, cudaStream_t stream);

@@ -672,7 +672,11 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
       (a.row_group != nullptr && a.rows > 65535U))
     return fail(kInvalidArgument, "F32 linear arguments are invalid");
   if (a.rows == 0) return kOk;
-  if (one_row_linear_f32_applicable(a)) return one_row_linear_f32(a, stream);
+  // One row: outside a pass's chain of launches the weight stream's ring and its one large CTA per SM have to be set up
+  // first, which short rows do not repay (264 x 5000: 8.3 us, 4.5 with a warp per output; 512 x 2048: 5.9 and 4.6; 1024 x
+  // 1024: 5.8 and 5.9; 4096 x 4096: 10.6 and 14.3).
+  if ((a.weight_stream || a.front.values != nullptr || a.in_features >= 1024) && one_row_linear_f32_applicable(a))
+    return one_row_linear_f32(a, stream);
   if (a.front.values != nullptr) return fail(kUnsupported, "operators in front of a projection take one row");
   F32Params p{};
   p.weight = static_cast<const bf16 *>(a.weight);

@@ -34,6 +34,7 @@ struct GemvParams {
   float alpha;
   int bias_mode, gate_mode;
   int dependent_launch;  // launched with programmatic stream serialisation: see the kernel
+  bool weight_stream;    // LinearArgs::weight_stream
   float gate_limit, softcap;
   // grouped weights [groups, N, K]: blockIdx.y = output row r, x row r / row_fanout, weight of group row_group[r]
   const int *row_group;
@@ -516,7 +517,13 @@ int launch_gemv(const GemvParams &p, cudaStream_t stream) {
   if constexpr (!kFp8)
     if (p.front != nullptr)
       return p.poly_front ? launch_stream<false, bf16, Front::kPoly>(p, stream) : launch_stream<false, bf16, Front::kRms>(p, stream);
-  if ((p.rows == 1 || p.row_group != nullptr) && stream_applicable<kFp8>(p))
+  // Single calls start behind everything else, with their ring empty: of BF16 weights a CTA per four of them is then as
+  // fast or faster (alone: 64 x 64 4.2 us against 5.3, 11264 x 4096 20.5 against 22.2, 8192 x 8192 26.7 against 30.5), of
+  // E4M3 up to some thousand columns (8448 x 2048 8.3 and 10.3, 4096 x 4096 8.3 and 8.5; 4096 x 12288 16.5 and 14.3).
+  // Grouped rows read a weight each and start with a lookup either way: all but short ones take the stream (4 rows of
+  // 2048 x 2816 14.3 and 13.7, 16 rows 45 and 32; 2 rows of 256 x 512 4.4 and 6.1).
+  const bool stream_rows = p.weight_stream || (p.row_group != nullptr ? p.K >= 1024 : kFp8 && p.N >= 8192);
+  if (stream_rows && (p.rows == 1 || p.row_group != nullptr) && stream_applicable<kFp8>(p))
     return launch_stream<kFp8, std::conditional_t<kFp8, std::uint8_t, bf16>>(p, stream);
   const int out_columns = p.gate_mode != 0 ? p.N / 2 : p.N;
   const int per_cta = p.gate_mode != 0 ? kColumnsPerCta / 2 : kColumnsPerCta;
@@ -605,6 +612,7 @@ int small_batch_linear(const LinearArgs &a, cudaStream_t stream) {
   p.bias_mode = a.bias_mode;
   p.gate_mode = a.gate_mode;
   p.dependent_launch = a.dependent_launch && (a.rows == 1 || a.row_group != nullptr) ? 1 : 0;
+  p.weight_stream = a.weight_stream;
   p.gate_limit = a.gate_limit;
   p.softcap = a.softcap;
   p.row_group = a.row_group;

@@ -84,6 +84,9 @@ struct LinearArgs {
   // it waits for that kernel before it reads the input.  The caller promises that `weight` is not being written
   // by earlier work in the stream.
   bool dependent_launch = false;
+  // One row, grouped rows: one of a pass's chain of launches, which gains from the weight stream at any size.  (Not decided
+  // by dependent_launch: a pass gives the same bits with and without it.)
+  bool weight_stream = false;
   int bias_mode = 0;   // 0 none, 1 fused F32 add, 2 separate BF16-rounded add
   // over 128-column halves (row-interleaved weights): 0 none, 1 a*b, 2 gelu(a)*b, 3 max(a, 0)*b, 4 clamped SwiGLU
   // with gate_limit (gates.cuh).  3 and 4 work on the F32 accumulators (plus bias_f32 in the weight's row order)

@@ -187,6 +187,7 @@ int Context::decoder_linear(Stage &s, const DecoderProduct &p) {
     a.alpha = p.alpha;
     a.softcap = p.softcap;
     a.dependent_launch = decode_dependent_launch_ && p.rows == 1;
+    a.weight_stream = true;
     a.front = p.front;
     return linear_f32(a, s.stream);
   }
@@ -194,6 +195,7 @@ int Context::decoder_linear(Stage &s, const DecoderProduct &p) {
   a.split_workspace = s.split_workspace;
   a.split_workspace_bytes = kSplitWorkspaceBytes;
   a.dependent_launch = decode_dependent_launch_ && p.rows <= 128;
+  a.weight_stream = true;
   a.input = p.input;
   a.weight = p.weight;
   a.output = p.output;
@@ -351,6 +353,7 @@ int Context::gated_feed_forward(Stage &s, const std::size_t i, const std::size_t
     a.split_workspace = s.split_workspace;
     a.split_workspace_bytes = kSplitWorkspaceBytes;
     a.dependent_launch = decode_dependent_launch_ && rows == 1;
+    a.weight_stream = true;
     a.input = input;
     a.weight = w.l12;
     a.output = s.gated;
@@ -469,6 +472,7 @@ int Context::expert_feed_forward(Stage &s, const std::size_t i, const std::size_
     grouping(a, true);
     a.groups = b.experts;
     a.dependent_launch = decode_dependent_launch_ && rows == 1;
+    a.weight_stream = true;
     a.output = s.gated;
     a.gate_mode = kGateClamped;
     a.gate_limit = b.gate_limit;
@@ -487,6 +491,7 @@ int Context::expert_feed_forward(Stage &s, const std::size_t i, const std::size_
     grouping(a, false);
     a.groups = b.experts;
     a.dependent_launch = decode_dependent_launch_ && rows == 1;
+    a.weight_stream = true;
     a.row_group_settled = pairwise && fused;
     a.output = s.expert_out;
     EVOB_OP(kCatGemmGrouped, linear(a, stream));

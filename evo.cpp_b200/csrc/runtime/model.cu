@@ -167,6 +167,7 @@ int Context::dump_mlp_taps(Stage &s, const std::size_t i, const std::size_t rows
     EVOB_TRY(first.reserve(rows * I * 2));
     EVOB_TRY(second.reserve(rows * I * 2));
     LinearArgs a;
+    a.weight_stream = true;
     a.split_workspace = s.split_workspace;
     a.split_workspace_bytes = kSplitWorkspaceBytes;
     a.input = s.normalized;
@@ -314,6 +315,7 @@ int Context::decode_step_graph(const std::uint32_t *host_token, bool *launched) 
       a.split_workspace = first.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
       a.dependent_launch = decode_dependent_launch_ && true;
+      a.weight_stream = true;
       a.input = first.normalized;
       a.weight = first.weights->embedding;  // tied head
       a.output = first.logits;
@@ -606,6 +608,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
       a.dependent_launch = decode_dependent_launch_ && rows <= 128;
+      a.weight_stream = true;
       a.input = fp8 ? s.codes : s.normalized;
       a.weight = w.projection;
       a.output = s.projection;
@@ -815,6 +818,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
       a.dependent_launch = decode_dependent_launch_ && rows <= 128;
+      a.weight_stream = true;
       a.input = s.mixer_out;
       a.weight = w.out_weight;
       a.bias = w.out_bias;
@@ -857,6 +861,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
       a.dependent_launch = decode_dependent_launch_ && rows <= 128;
+      a.weight_stream = true;
       a.input = s.normalized;
       a.weight = w.l12;
       a.output = s.gated;
@@ -875,6 +880,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       EVOB_OP(up8 ? kCatGemmFp8Ffn : kCatGemmBf16, linear(a, stream));
     } else {
       LinearArgs a;
+      a.weight_stream = true;
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
       a.input = s.normalized;
@@ -898,6 +904,7 @@ int Context::run_stage(Stage &s, const std::size_t rows, const Mode mode,
       a.split_workspace = s.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
       a.dependent_launch = decode_dependent_launch_ && rows <= 128;
+      a.weight_stream = true;
       a.input = s.gated;
       a.weight = w.l3;
       a.residual = s.residual;
@@ -1079,6 +1086,7 @@ int Context::forward(const std::uint32_t *host_tokens, const std::uint32_t *devi
       a.split_workspace = first.split_workspace;
       a.split_workspace_bytes = kSplitWorkspaceBytes;
       a.dependent_launch = decode_dependent_launch_ && rows <= 128;
+      a.weight_stream = true;
       a.input = first.normalized;
       a.weight = first.weights->embedding;  // tied head
       a.output = first.logits;
@@ -1210,6 +1218,7 @@ int Context::slice_head(const std::size_t position, const std::size_t rows) {
                         1.0F, stage.stream);
   if (status != kOk) return status;
   LinearArgs a;
+  a.weight_stream = true;
   a.split_workspace = stage.split_workspace;
   a.split_workspace_bytes = kSplitWorkspaceBytes;
   a.input = normalized;

@@ -6,6 +6,8 @@ checked against an F32 matmul of the same BF16 operands (tolerance 0.02 abs +
 tests/test_cuda_ops.cu:252-369)."""
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -223,41 +225,84 @@ def _check_split_k_gated(ops, rows, inner, hidden):
 
 
 @pytest.mark.parametrize("columns", [1, 37, 256, 1184, 5000])
-@pytest.mark.parametrize("inner", [64, 264, 1920, 2056, 4104, 8448, 11264, 16384, 16392])
+@pytest.mark.parametrize("inner", [64, 264, 1920, 2056, 4104, 6152, 8192, 8448, 11264, 14336, 16384, 16392])
 def test_one_row_streams(ops, inner, columns):
-    """One row at the edges of the weight stream's split: fewer columns than CTAs, pieces of 8 (16) values that leave
-    lanes or whole warps without work, every number of pieces per thread, and an inner size beyond its registers.  A
-    result passes through at most 32 roundings (16 products, 8 pieces, 5 + 3 sums)."""
+    """One row at the edges of its kernels: fewer columns than CTAs, pieces of 8 (16) values that leave lanes or whole
+    warps without work, every number of pieces per thread of the F32 weight stream (1, 2, 3, 4, 5, 6 and 8), and an inner
+    size beyond its registers.  A result passes through as many roundings as the kernel that takes the size chains."""
+    lanes = 8 * (-(-inner // 256)) + 5 + 2                     # a warp per output: a lane's products, the lanes, the base
+    stream_chain = 8 + 7 + 5 + 3 + 2                           # a piece's products, the pieces, lanes, warps, the base
+    f32_chain = stream_chain if 1024 <= inner <= 16384 else lanes
+    bf16_chain = 8 * (-(-inner // 2048)) + 5 + 8 + 2           # a CTA per four outputs: a thread's products, lanes, warps
+    e4m3_chain = 16 * (-(-inner // 4096)) + 5 + 8 + 2
     generator = torch.Generator("cuda").manual_seed(inner + columns)
     x, w = (torch.randn(n, inner, device="cuda", generator=generator) for n in (1, columns))
     xb, wb = x.bfloat16(), w.bfloat16()
     base = torch.randn(1, columns, device="cuda", generator=generator)
 
-    def check(out, left, right, add):
+    def check(out, left, right, add, chain):
         left, right = left.double(), right.double()
-        bound = 32 * 2.0 ** -24 * (left.abs() @ right.abs().T + add.double().abs())
+        bound = chain * 2.0 ** -24 * (left.abs() @ right.abs().T + add.double().abs())
         assert bool(((out.double() - (left @ right.T + add)).abs() <= bound).all())
 
     out = base.clone()
     ops.call("f32_linear", p(x), p(wb), 1, inner, columns, 1, p(out), stream())
-    check(out, x, wb, base)
+    check(out, x, wb, base, f32_chain)
     work = torch.empty(1 << 20, device="cuda")
     ops.call("bf16_linear_f32_result", p(xb), p(wb), 1, inner, columns, 0, p(work), work.numel() * 4, p(out), stream())
-    check(out, xb, wb, torch.zeros_like(base))
+    check(out, xb, wb, torch.zeros_like(base), bf16_chain)
     bits = torch.empty(1, columns, dtype=torch.bfloat16, device="cuda")
     if inner % 16 == 0:
         codes, weights = (t.to(torch.float8_e4m3fn) for t in (x, w))
         ops.call("e4m3_codes_linear", p(codes.view(torch.uint8)), None, p(weights.view(torch.uint8)), None, None, 1, inner,
                  columns, 1.0, 0, 0, p(bits), stream())
         expected = codes.double() @ weights.double().T
-        bound = 2.0 ** -8 * expected.abs() + 32 * 2.0 ** -24 * (codes.double().abs() @ weights.double().abs().T)
+        bound = 2.0 ** -8 * expected.abs() + e4m3_chain * 2.0 ** -24 * (codes.double().abs() @ weights.double().abs().T)
         assert bool(((bits.double() - expected).abs() <= bound).all())
     if columns % 128 == 0:
         pair = torch.randn(2 * columns, inner, device="cuda", generator=generator).bfloat16()
         ops.call("bf16_gated_up_projection", p(xb), p(pair), 1, inner, columns, 0, p(bits), stream())
         first, second = (xb.double() @ pair.view(-1, 2, 128, inner)[:, i].reshape(columns, inner).double().T for i in (0, 1))
         # both factors and the product are rounded to BF16 (2^-8 each), behind F32 sums with the bound above
-        slack = 32 * 2.0 ** -24 * inner
+        slack = bf16_chain * 2.0 ** -24 * inner
         bound = 3.1 * 2.0 ** -8 * (first * second).abs() + slack * (first.abs() + second.abs())
         assert bool(((bits.double() - first * second).abs() <= bound).all())
     ops.call("check_async_errors", stream())
+
+
+@pytest.mark.parametrize("columns", [8192, 8201])
+@pytest.mark.parametrize("inner", [528, 4224, 12288, 14336, 16400, 24576, 24592])
+def test_one_row_e4m3_streams(ops, inner, columns):
+    """Every number of pieces per thread of the E4M3 weight stream (1 to 6) and an inner size beyond it."""
+    generator = torch.Generator("cuda").manual_seed(inner + columns)
+    x, w = (torch.randn(n, inner, device="cuda", generator=generator).to(torch.float8_e4m3fn) for n in (1, columns))
+    out = torch.empty(1, columns, dtype=torch.bfloat16, device="cuda")
+    ops.call("e4m3_codes_linear", p(x.view(torch.uint8)), None, p(w.view(torch.uint8)), None, None, 1, inner, columns, 1.0, 0,
+             0, p(out), stream())
+    ops.call("check_async_errors", stream())
+    xd, wd = x.double(), w.double()
+    expected = xd @ wd.T
+    # a piece's products, the pieces, lanes and warps; beyond the stream a thread's products, lanes and warps
+    chain = 16 + 5 + 5 + 3 if inner <= 24576 else 16 * (-(-inner // 4096)) + 5 + 8
+    bound = 2.0 ** -8 * expected.abs() + chain * 2.0 ** -24 * (xd.abs() @ wd.abs().T)
+    assert bool(((out.double() - expected).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("columns", [5, 300, 1184])
+@pytest.mark.parametrize("inner", [264, 1032, 2056, 4104, 6152, 8200, 11264, 14336, 16384, 16392])
+def test_grouped_row_streams(pkg, ops, inner, columns):
+    """Rows with a weight each: every number of pieces per thread of the BF16 weight stream (1, 2, 3, 4, 5, 6 and 8), and
+    sizes on either side of it."""
+    generator = torch.Generator("cuda").manual_seed(inner + columns)
+    x = torch.randn(2, inner, device="cuda", generator=generator).bfloat16()
+    w = torch.randn(3, columns, inner, device="cuda", generator=generator).bfloat16()
+    group = torch.tensor([2, 0, 1, 2], dtype=torch.int32, device="cuda")
+    out = torch.empty(4, columns, device="cuda")
+    arguments = pkg.Projection(input=p(x), weight=p(w), output=p(out), rows=4, in_features=inner, out_features=columns, alpha=1.0,
+                               f32_result=1, row_group=p(group), row_fanout=2, groups=3)
+    ops.call("projection", ctypes.addressof(arguments), stream())
+    ops.call("check_async_errors", stream())
+    chain = 8 + 7 + 5 + 3 + 1 if 1024 <= inner <= 16384 else 8 * (-(-inner // 2048)) + 5 + 8 + 1
+    for r in range(4):
+        xd, wd = x[r // 2].double(), w[group[r]].double()
+        assert bool(((out[r].double() - wd @ xd).abs() <= chain * 2.0 ** -24 * (wd.abs() @ xd.abs())).all())
