@@ -39,7 +39,7 @@ KERNEL_SOURCES = [
 ]
 OPS_SOURCES = KERNEL_SOURCES + ["ops_api.cu"]
 RUNTIME_SOURCES = KERNEL_SOURCES + [
-    "runtime/safetensors.cpp", "runtime/model_load.cpp", "runtime/model_weights.cpp",
+    "runtime/safetensors.cpp", "runtime/host_pool.cpp", "runtime/model_load.cpp", "runtime/model_weights.cpp",
     "runtime/gigusun.cpp", "runtime/kikepel.cpp",
     "runtime/model.cu", "runtime/decoder.cu", "runtime/sampler.cpp", "runtime/variant.cpp", "runtime/variant_io.cpp", "runtime/scheduler.cpp", "runtime/c_api.cpp",
 ]

@@ -203,67 +203,15 @@ int Context::dump_mlp_taps(Stage &s, const std::size_t i, const std::size_t rows
   return kOk;
 }
 
-HostPool::~HostPool() {
-  for (const Block &b : free_) cudaFreeHost(b.data);
-}
-
-void *HostPool::take(const std::size_t bytes, std::size_t *const capacity) {
-  std::size_t wanted = std::size_t{64} << 10;
-  while (wanted < bytes) wanted *= 2;  // few sizes, so that blocks find their next user
-  {
-    const std::lock_guard<std::mutex> lock(mutex_);
-    for (std::size_t i = 0; i < free_.size(); ++i)
-      if (free_[i].capacity >= wanted) {
-        const Block b = free_[i];
-        free_.erase(free_.begin() + static_cast<std::ptrdiff_t>(i));
-        *capacity = b.capacity;
-        return b.data;
-      }
-  }
+void *pinned_allocate(const std::size_t bytes) {
   void *data = nullptr;
-  if (cudaHostAlloc(&data, wanted, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+  if (cudaHostAlloc(&data, bytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  *capacity = wanted;
   return data;
 }
-
-void HostPool::give(void *const block, const std::size_t capacity) {
-  Block dropped{block, capacity};
-  if (capacity <= kLargest) {
-    const std::lock_guard<std::mutex> lock(mutex_);
-    free_.push_back(dropped);
-    if (free_.size() <= kKept) return;
-    const auto smallest = std::min_element(free_.begin(), free_.end(),
-                                           [](const Block &a, const Block &b) { return a.capacity < b.capacity; });
-    dropped = *smallest;
-    free_.erase(smallest);
-  }
-  cudaFreeHost(dropped.data);
-}
-
-void HostRows::release() {
-  if (block_ != nullptr) pool_->give(block_, capacity_);
-  block_ = nullptr;
-  pool_.reset();
-}
-
-void HostRows::resize(const std::shared_ptr<HostPool> &pool, const std::size_t count) {
-  if (block_ == nullptr || pool_ != pool || capacity_ < count * sizeof(float)) {
-    release();
-    block_ = count * sizeof(float) <= HostPool::kLargest ? pool->take(count * sizeof(float), &capacity_) : nullptr;
-    if (block_ != nullptr) pool_ = pool;
-  }
-  if (block_ == nullptr) own_.resize(count);
-  count_ = count;
-}
-
-void HostRows::assign(const float *const values, const std::size_t count) {
-  release();
-  own_.assign(values, values + count);
-  count_ = count;
-}
+void pinned_free(void *const block) { cudaFreeHost(block); }
 
 Context::~Context() {
   if (!stages_.empty()) {

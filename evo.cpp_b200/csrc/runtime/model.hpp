@@ -11,10 +11,10 @@
 #include <cstdint>
 #include <functional>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <vector>
 
+#include "host_pool.hpp"
 #include "safetensors.hpp"
 
 namespace evob {
@@ -232,50 +232,13 @@ struct StageWeights {
   ~StageWeights();
 };
 
-// Pinned host memory that results come back through, shared by the contexts of a model (any thread, any device).
-// kKept free blocks of up to kLargest bytes stay for the next user, the rest is given back.
-class HostPool {
- public:
-  static constexpr std::size_t kLargest = std::size_t{64} << 20, kKept = 4;
-  ~HostPool();
-  void *take(std::size_t bytes, std::size_t *capacity);  // nullptr: not to be had
-  void give(void *block, std::size_t capacity);
-
- private:
-  struct Block {
-    void *data;
-    std::size_t capacity;
-  };
-  std::mutex mutex_;
-  std::vector<Block> free_;
-};
-
-// Rows of F32 results on the host: a pool's block until the next use or the end of the object, or memory of its own.
-class HostRows {
- public:
-  HostRows() = default;
-  HostRows(const HostRows &) = delete;
-  HostRows &operator=(const HostRows &) = delete;
-  ~HostRows() { release(); }
-  // Room for `count` values, pinned if the pool has it.
-  void resize(const std::shared_ptr<HostPool> &pool, std::size_t count);
-  void assign(const float *values, std::size_t count);
-  bool pinned() const { return block_ != nullptr; }
-  float *data() { return block_ != nullptr ? static_cast<float *>(block_) : own_.data(); }
-  const float *data() const { return block_ != nullptr ? static_cast<const float *>(block_) : own_.data(); }
-  std::size_t size() const { return count_; }
-
- private:
-  void release();
-  std::shared_ptr<HostPool> pool_;
-  void *block_ = nullptr;
-  std::size_t capacity_ = 0, count_ = 0;
-  std::vector<float> own_;
-};
+// Portable pinned memory; nullptr when there is none.
+void *pinned_allocate(std::size_t bytes);
+void pinned_free(void *block);
 
 struct ModelWeights {
   ModelConfig config;
-  std::shared_ptr<HostPool> host_pool = std::make_shared<HostPool>();
+  std::shared_ptr<HostPool> host_pool = std::make_shared<HostPool>(pinned_allocate, pinned_free);
   std::vector<std::shared_ptr<StageWeights>> stages;
   // Per-process pipelines: this process holds stage `slice_index` of
   // `slice_count` (one StageWeights); 0 / 1 for a model held by one process.

@@ -502,3 +502,118 @@ def test_reference_fasta_index_and_scoring_windows(evo, tmp_path):
     import gzip
     refused("packed.fa.gz", gzip.compress(b">a\nACGT\n"), 5, "gzip-compressed")
     assert _reference(evo, tmp_path / "absent.fa")[0] == 3
+
+
+# ---- pinned host memory of results (runtime/host_pool): plain C++ on a stand-in for the CUDA runtime's calls
+POOL_PROGRAM = r"""
+#include <cassert>
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+
+#include "runtime/host_pool.hpp"
+
+using evob::HostPool;
+using evob::HostRows;
+
+static std::map<void *, std::size_t> live;
+static std::size_t allocations = 0, refuse_above = ~std::size_t{0};
+static void *allocate(const std::size_t bytes) {
+  if (bytes > refuse_above) return nullptr;
+  ++allocations;
+  void *const p = std::malloc(bytes);
+  live[p] = bytes;
+  return p;
+}
+static void release(void *const p) {
+  assert(live.erase(p) == 1);
+  std::free(p);
+}
+static std::size_t live_bytes() {
+  std::size_t sum = 0;
+  for (const auto &[p, bytes] : live) sum += bytes;
+  return sum;
+}
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::exit(1); } } while (0)
+
+int main() {
+  constexpr std::size_t kMiB = std::size_t{1} << 20;
+  {
+    auto pool = std::make_shared<HostPool>(allocate, release);
+    std::size_t large = 0, medium = 0, small = 0, got = 0;
+    void *const l = pool->take(64 * kMiB, &large), *const m = pool->take(3 * kMiB, &medium), *const s = pool->take(2064, &small);
+    CHECK(l && m && s && large == 64 * kMiB && medium == 4 * kMiB && small >= 2064 && small <= kMiB);
+    // the smallest block that fits, whatever came back first; none that is far too large
+    pool->give(l, large);
+    pool->give(m, medium);
+    pool->give(s, small);
+    CHECK(pool->take(2064, &got) == s && got == small);
+    const std::size_t before = allocations;
+    void *const other = pool->take(2064, &got);
+    CHECK(other != nullptr && other != l && other != m && allocations == before + 1);
+    CHECK(pool->take(3 * kMiB, &got) == m && pool->take(40 * kMiB, &got) == l && allocations == before + 1);
+    CHECK(pool->take(64 * kMiB + 1, &got) == nullptr && allocations == before + 1);
+    pool->give(l, large);
+    pool->give(m, medium);
+    pool->give(s, small);
+    pool->give(other, small);
+  }
+  CHECK(live.empty());
+  {
+    // many small blocks stay, so that users who come and go together neither allocate nor free
+    HostPool pool(allocate, release);
+    std::vector<void *> blocks(12);
+    std::size_t capacity = 0;
+    for (void *&b : blocks) b = pool.take(2064, &capacity);
+    for (void *const b : blocks) pool.give(b, capacity);
+    const std::size_t before = allocations;
+    CHECK(live.size() == blocks.size());
+    for (void *&b : blocks) b = pool.take(2064, &capacity);
+    CHECK(allocations == before);
+    for (void *const b : blocks) pool.give(b, capacity);
+    // what is kept is bounded, in number and in bytes; what was used last stays
+    std::vector<void *> large(6);
+    for (void *&b : large) b = pool.take(64 * kMiB, &capacity);
+    for (void *const b : large) pool.give(b, capacity);
+    CHECK(live_bytes() <= HostPool::kKeptBytes && live.size() <= HostPool::kKept);
+    CHECK(live.count(large.back()) == 1);
+    blocks.resize(40);
+    for (void *&b : blocks) b = pool.take(2064, &capacity);
+    for (void *const b : blocks) pool.give(b, capacity);
+    CHECK(live_bytes() <= HostPool::kKeptBytes && live.size() <= HostPool::kKept);
+  }
+  CHECK(live.empty());
+  {
+    // rows: pinned where the pool has memory, their own where it has none
+    auto pool = std::make_shared<HostPool>(allocate, release);
+    HostRows rows;
+    rows.resize(pool, 1000);
+    CHECK(rows.pinned() && rows.size() == 1000);
+    const float *const first = rows.data();
+    rows.resize(pool, 900);
+    CHECK(rows.data() == first && rows.size() == 900);
+    refuse_above = 0;
+    rows.resize(pool, 100000);
+    CHECK(!rows.pinned() && rows.size() == 100000 && rows.data() != nullptr);
+    rows.data()[99999] = 1.0F;
+    rows.resize(nullptr, 10);
+    CHECK(!rows.pinned() && rows.size() == 10);
+    const float values[3] = {1.0F, 2.0F, 3.0F};
+    rows.resize(pool, 1000);
+    rows.assign(values, 3);
+    CHECK(!rows.pinned() && rows.size() == 3 && rows.data()[2] == 3.0F);
+  }
+  CHECK(live.empty());
+  std::puts("ok");
+}
+"""
+
+
+def test_pool_of_pinned_results(tmp_path):
+    source, program = tmp_path / "pool.cpp", tmp_path / "pool"
+    source.write_text(POOL_PROGRAM)
+    csrc = ROOT / "evo.cpp_b200" / "csrc"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-I", str(csrc), str(source),
+                    str(csrc / "runtime" / "host_pool.cpp"), "-o", str(program)], check=True)
+    done = subprocess.run([str(program)], capture_output=True, text=True)
+    assert done.returncode == 0 and done.stdout.strip() == "ok", done.stdout + done.stderr
