@@ -16,12 +16,17 @@ class HostPool {
   using Free = void (*)(void *);
   static constexpr std::size_t kLargest = std::size_t{64} << 20, kSmallest = std::size_t{64} << 10;
   static constexpr std::size_t kKept = 16, kKeptBytes = 4 * kLargest;
+  static constexpr std::size_t kSlabBytes = std::size_t{256} << 10;
   static constexpr std::size_t kWaste = 8;  // a block serves what takes an eighth of it or more
 
-  HostPool(Allocate allocate, Free free);
+  // Nothing above `largest` bytes is pinned.
+  HostPool(Allocate allocate, Free free, std::size_t largest = kLargest);
   HostPool(const HostPool &) = delete;
   HostPool &operator=(const HostPool &) = delete;
   ~HostPool();
+  // Up to `count` small blocks of `bytes` from one allocation, which lasts as long as the pool: an allocation takes 2 ms
+  // and more whatever its size, a context is made in as much.  Once, before the pool is shared; no memory, no blocks.
+  void reserve(std::size_t bytes, std::size_t count);
   void *take(std::size_t bytes, std::size_t *capacity);  // nullptr: not to be had
   void give(void *block, std::size_t capacity) noexcept;
 
@@ -32,6 +37,10 @@ class HostPool {
   };
   const Allocate allocate_;
   const Free free_memory_;
+  const std::size_t largest_;
+  void *slab_ = nullptr;
+  std::size_t small_bytes_ = 0;
+  std::vector<void *> small_;  // free blocks of the slab, small_bytes_ each (no other block has this capacity)
   std::mutex mutex_;
   std::vector<Block> idle_;  // in the order in which they came back
   std::size_t idle_bytes_ = 0;

@@ -416,11 +416,12 @@ int Context::create(std::shared_ptr<ModelWeights> weights, const std::size_t con
     EVOB_TRY(first.allocate(&p, 16, &first.arena_bytes));
     context->device_step_ = static_cast<std::uint32_t *>(p);
     context->device_position_ = reinterpret_cast<const int *>(context->device_step_ + 1);
-    context->host_step_ = static_cast<std::uint32_t *>(weights->host_pool->take(
-        kStepRow * sizeof(std::uint32_t) + c.vocab * sizeof(float), &context->host_step_bytes_));
-    if (context->host_step_ == nullptr) return fail(kCuda, "cannot allocate the context's pinned memory");
+    if (weights->slice_count < 2)
+      context->host_step_ =
+          static_cast<std::uint32_t *>(weights->host_pool->take(step_bytes(c), &context->host_step_bytes_));
     const char *const graphs = std::getenv("EVO_B200_DECODE_GRAPH");
-    context->decode_graph_allowed_ = (graphs == nullptr || std::string(graphs) != "0") && !q8_kv;
+    context->decode_graph_allowed_ = (graphs == nullptr || std::string(graphs) != "0") && !q8_kv &&
+                                     context->host_step_ != nullptr;
     const char *const dependent = std::getenv("EVO_B200_DECODE_PDL");
     context->decode_dependent_launch_ = dependent == nullptr || std::string(dependent) != "0";
   }
@@ -1045,14 +1046,14 @@ int Context::forward(const std::uint32_t *host_tokens, const std::uint32_t *devi
     }
     if (status == kOk && logits != nullptr) {
       const std::size_t elements = rows * c.vocab;
-      int *const error = reinterpret_cast<int *>(host_step_ + 2);
+      int *const error = host_step_ != nullptr ? reinterpret_cast<int *>(host_step_ + 2) : nullptr;
       if (!graph_step) {
-        *error = 0;
-        logits->resize(weights_->host_pool, elements);
+        logits->resize(error != nullptr ? weights_->host_pool : nullptr, elements);
         if (logits->pinned()) {
+          *error = 0;
           status = publish_rows(first.logits, c.decoder(), elements, logits->data(), error, first.stream);
         } else {
-          // more than the pool holds; BF16 logits land in the upper half of the result and are widened from there
+          // more than is pinned; BF16 logits land in the upper half of the result and are widened from there
           unsigned char *const target = reinterpret_cast<unsigned char *>(logits->data()) + (c.decoder() ? 0 : elements * 2);
           if (cudaMemcpyAsync(target, first.logits, elements * (c.decoder() ? 4 : 2), cudaMemcpyDeviceToHost, first.stream) !=
               cudaSuccess)

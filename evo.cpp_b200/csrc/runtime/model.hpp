@@ -271,6 +271,8 @@ class Context {
                     ExecutionProfile profile, bool full_arena_for_fixtures,
                     std::unique_ptr<Context> *out, bool q8_kv = false);
 
+  // Pinned bytes that a context keeps.
+  static std::size_t step_bytes(const ModelConfig &c) { return (kStepRow + c.vocab) * sizeof(float); }
   // logits: rows * vocab floats (converted from BF16), valid until *logits is used again or destroyed.
   int prefill(const std::vector<std::uint32_t> &tokens, HostRows *logits);
   int prefill_stateless(const std::vector<std::uint32_t> &tokens, HostRows *logits);
@@ -374,7 +376,7 @@ class Context {
   int decode_step_graph(const std::uint32_t *host_token, bool *launched);
   void *decode_graph_ = nullptr;          // cudaGraphExec_t
   // A step's token and position, and where replayed kernels read them; pinned: the same two, then the error word behind
-  // the step, and from kStepRow on its logits.
+  // the step, and from kStepRow on its logits.  Without pinned memory (null) there is no graph, and results are copied.
   std::uint32_t *device_step_ = nullptr;
   const int *device_position_ = nullptr;
   std::uint32_t *host_step_ = nullptr;

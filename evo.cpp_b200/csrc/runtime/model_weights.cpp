@@ -7,6 +7,7 @@
 // apply the gate in its epilogue.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <set>
 
@@ -377,6 +378,12 @@ int load_weights(const ModelFile &file, const std::vector<int> &devices,
       for (const ExpectedTensor &e : expected_model_tensors(c)) stage->weight_bytes += file.find(e.name)->bytes;
     for (const LayerWeights &w : stage->layers) stage->weight_bytes += w.payload_bytes;
     weights->stages.push_back(std::move(stage));
+  }
+  if (status == kOk && !sliced) {
+    std::size_t largest = HostPool::kLargest;
+    if (const char *const text = std::getenv("EVO_B200_PINNED_BYTES")) largest = std::strtoull(text, nullptr, 0);
+    weights->host_pool = std::make_shared<HostPool>(pinned_allocate, pinned_free, largest);
+    weights->host_pool->reserve(Context::step_bytes(c), 32);
   }
   cudaSetDevice(previous_device);
   if (status != kOk) return status;

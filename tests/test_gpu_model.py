@@ -380,3 +380,34 @@ def test_embedding_is_chunked_and_advances_the_context_like_upstream(rt, evo, bf
     evo.lib.evo_batch_free(batch)
     with pytest.raises(rt.EvoError):
         failing.prefill(sequence)
+
+
+@pytest.mark.parametrize("limit", [0, 4096])
+@pytest.mark.parametrize("decoder", [False, True], ids=["stripedhyena", "decoder"])
+def test_results_without_pinned_memory(rt, evo, pkg, fp8_fixture, tmp_path, monkeypatch, decoder, limit):
+    """Contexts need no pinned memory: without any, or with results above the limit, logits come back through pageable
+    copies (BF16 ones are widened in place), bit for bit the same, and errors are still reported."""
+    if decoder:
+        from gigusun_util import attention, delta, gla, make_model
+
+        path, flags = make_model(pkg, tmp_path / "m", [delta(), attention(), gla()])[0], 0
+    else:
+        path, flags = fp8_fixture, rt.MODEL_FLAG_ALLOW_SYNTHETIC
+    usual = evo.load(path, flags=flags)
+    monkeypatch.setenv("EVO_B200_PINNED_BYTES", str(limit))
+    limited = evo.load(path, flags=flags)
+    monkeypatch.delenv("EVO_B200_PINNED_BYTES")
+    tokens = np.random.default_rng(3).integers(0, usual.vocab, 150).tolist()
+    full = 0 if decoder else rt.CONTEXT_FLAG_FULL_ARENA
+    a, b = usual.context(256, full), limited.context(256, full)
+    for prompt in (tokens[:1], tokens[:7], tokens):
+        assert np.array_equal(a.prefill_tokens(prompt), b.prefill_tokens(prompt))
+    for token in tokens[:5]:
+        assert np.array_equal(a.decode(token), b.decode(token))
+    assert np.array_equal(a.embed_tokens(tokens[:20], 1), b.embed_tokens(tokens[:20], 1))
+    for context in (a, b):
+        with pytest.raises(rt.EvoError) as refused:
+            context.prefill_tokens([0, usual.vocab])
+        assert refused.value.code == 2
+    for closed in (a, b, usual, limited):
+        closed.close()

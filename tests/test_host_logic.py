@@ -584,6 +584,37 @@ int main() {
   }
   CHECK(live.empty());
   {
+    // blocks of a slab: one allocation for all, never given back alone, for small requests only
+    HostPool pool(allocate, release);
+    const std::size_t before = allocations;
+    pool.reserve(2064, 32);
+    CHECK(allocations == before + 1 && live_bytes() <= kMiB);
+    std::vector<void *> blocks(32);
+    std::size_t capacity = 0, other = 0;
+    for (void *&b : blocks) CHECK((b = pool.take(2064, &capacity)) != nullptr && capacity >= 2064);
+    CHECK(allocations == before + 1);
+    void *const more = pool.take(2064, &other), *const large = pool.take(kMiB, &other);
+    CHECK(more != nullptr && large != nullptr && allocations == before + 3);
+    pool.give(large, other);
+    for (void *const b : blocks) pool.give(b, capacity);
+    CHECK(pool.take(kMiB, &other) == large && pool.take(2064, &capacity) == blocks.back());
+    CHECK(allocations == before + 3);
+    release(more);
+    release(large);
+  }
+  CHECK(live.empty());
+  {
+    // no memory, or none allowed: no blocks, and nothing fails
+    refuse_above = 0;
+    HostPool pool(allocate, release), none(allocate, release, 0);
+    std::size_t capacity = 0;
+    pool.reserve(2064, 32);
+    CHECK(pool.take(2064, &capacity) == nullptr);
+    refuse_above = ~std::size_t{0};
+    none.reserve(2064, 32);
+    CHECK(none.take(1, &capacity) == nullptr && live.empty());
+  }
+  {
     // rows: pinned where the pool has memory, their own where it has none
     auto pool = std::make_shared<HostPool>(allocate, release);
     HostRows rows;
