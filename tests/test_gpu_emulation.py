@@ -31,7 +31,7 @@ def _codes(rng, kind, shape):
 @pytest.mark.parametrize("kind", ["any", "sparse", "subnormal", "extreme", "cancel"])
 @pytest.mark.parametrize("rows,inner,columns", [(1, 32, 33), (1, 544, 70), (2, 96, 31), (1, 64, 18944), (2, 32, 18950),
                                                (3, 32, 5), (16, 160, 65), (17, 96, 64), (33, 64, 129), (65, 32, 9409),
-                                               (128, 64, 9472)])
+                                               (128, 64, 9472), (125, 64, 9473), (509, 32, 2433)])
 def test_emulated_projection_at_kernel_edges(ops, oracle, rows, inner, columns, kind):
     rng = np.random.default_rng(rows * 31 + inner + columns)
     x, w = _codes(rng, kind, (rows, inner)), _codes(rng, kind, (columns, inner))

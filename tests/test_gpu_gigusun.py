@@ -335,3 +335,25 @@ def test_refusals(rt, made):
     with pytest.raises(rt.EvoError):
         c.decode(1)                                                 # the context is full
     c.close()
+
+
+@pytest.mark.parametrize("profile, limit", [("float32", 2e-5), ("exact", 2.0 ** -7)])
+@pytest.mark.parametrize("width, ff", [(40, 24), (264, 2056), (72, 4104), (72, 6152), (136, 8448), (72, 11264), (40, 14336), (2056, 72),
+                                       (4104, 24), (6152, 72), (8200, 40), (11264, 72), (14336, 24), (16384, 72)])
+def test_fronts_of_one_row_projections(pkg, rt, tmp_path, width, ff, profile, limit):
+    """The residual norm and the polynomial activation inside one-row projections against their own kernels, which tapped
+    blocks take: every number of pieces per thread (1, 2, 3, 4, 5, 6 and 8) on both sides, lanes and warps without work.
+    They differ by the order of F32 sums (some 50 roundings of 2^-24 in a factor); behind it BF16 activations may
+    round the other way, by 2^-8 of single values."""
+    blocks = [gla(heads=1, dim=8, vdim=16, ff=ff), attention(heads=2, kv_heads=1, dim=16, vdim=8, size=9, keep_first=1, ff=ff)]
+    directory, config, _ = make_model(pkg, tmp_path / "m", blocks, vocab=40, width=width, max_positions=64)
+    model = rt.EvoLibrary(pkg.EVO_LIBRARY).load(directory)
+    flags = rt.CONTEXT_FLAG_FLOAT32 if profile == "float32" else 0
+    fused, apart = model.context(32, flags), model.context(32, flags)
+    tokens = np.random.default_rng(width).integers(0, 40, 12).tolist()
+    assert np.array_equal(fused.prefill_tokens(tokens[:5]), apart.prefill_tokens(tokens[:5]))
+    for token in tokens[5:]:
+        step, taps = apart.decode_with_dumps(token, [(0, "mixer_output"), (1, "mixer_output")])
+        assert len(taps) == 2 and error(fused.decode(token), step) < limit
+    for closed in (fused, apart, model):
+        closed.close()
