@@ -600,7 +600,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
                        "l2_policy": "weights (12 GB) and activations exceed the 126 MB L2 every step; no flush needed",
                        "model_load_seconds": load_seconds},
             "e2e": {"value": e2e_value, "unit": "tokens/s", "h2d_bytes_per_step": 4 * tokens,
-                    "d2h_bytes_per_step": 2 * tokens * VOCAB},
+                    "d2h_bytes_per_step": 4 * tokens * VOCAB},  # F32 logits cross the host link
             "gpu_launches": launches_per_step * args.steps,
             "gflop_per_token": gemm_flops_per_token(tokens) / 1e9,
             "model_tflops": gemm_flops_per_token(tokens) * tokens / (ms_per_step * 1e-3) / 1e12,

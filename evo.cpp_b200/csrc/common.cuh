@@ -83,7 +83,8 @@ constexpr int kSmCount = 148;
 // rms_norm() of 1,000 x 8192: 8.5 and 13.7, where the pointers had lost their address space, too).
 // Kernels other than weight streams release after their wait: a projection that started earlier still would find the SMs
 // unevenly taken by the one in front of this kernel, and where its CTAs land is where they stay (a gated 11264 x 2048
-// projection took 12.4 us behind early releases, 7.8 with its CTAs spread evenly).
+// projection took 12.4 us behind early releases, 7.8 with its CTAs spread evenly).  A kernel that releases and never waits
+// has to be launched plainly.
 __device__ __forceinline__ void release_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class Pointer>
 __device__ __forceinline__ void make_opaque(Pointer &pointer) {

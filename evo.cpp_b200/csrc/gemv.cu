@@ -508,8 +508,8 @@ int launch_stream(const GemvParams &p, cudaStream_t stream) {
   }
 }
 
-// 2..8 rows, sizes beyond the kernel above: four weight rows per CTA; a gated projection then produces two output columns
-// per CTA.
+// 2..8 rows, single calls, sizes beyond the kernel above: four weight rows per CTA; a gated projection then produces two
+// output columns per CTA.
 constexpr int kColumnsPerCta = 4;
 
 template <bool kFp8>

@@ -116,7 +116,6 @@ struct LinearArgs {
   // (128 or 256), tile t belongs to group tile_group[t], *tile_count tiles are in use (both on the device; `rows`
   // is the capacity, unused tiles are not touched).  Row form (a few rows): output row r is input row
   // r / row_fanout times the weight of group row_group[r].
-  RowFront front;  // one row of BF16 products without groups or row_scale; the input is the operator's
   std::size_t groups = 0;
   const int *tile_group = nullptr, *tile_count = nullptr;
   std::size_t tile_rows = 128;
@@ -125,6 +124,7 @@ struct LinearArgs {
   // With dependent_launch: the kernel in front of this one is linear() with the same row_group, so row_group itself comes
   // from work further back (which has completed when a grouped projection lets the kernel behind it start).
   bool row_group_settled = false;
+  RowFront front;  // one row of BF16 products without groups or row_scale; the input is the operator's
 };
 // Whether linear() takes the tile form of grouped weights at these sizes.
 bool grouped_linear_applicable(const LinearArgs &args);

@@ -25,8 +25,8 @@
 //     (e is in [-9, 8], so the exponents stay within F32 and BF16).
 //     mma.sync's result layout is the thread's output tile.
 // What bounds it: the ALU (packing, signs, staging) and the half of the FMA pipe
-// that dp2a shares with the multiply-adds, each busy for 60 % of the time with 16
-// warps per SM; about 3 instructions per product.  509 rows at 12288 x 4096: 3.5
+// that dp2a shares with the multiply-adds, busy for 52 and 55 % of the time with 16
+// warps per SM, in bursts that meet each other; about 3 instructions per product.  509 rows at 12288 x 4096: 3.5
 // ms = 7.4 T products/s; integer shifts per product took 17.1 ms.
 #include "common.cuh"
 #include "ops_internal.hpp"
@@ -109,7 +109,6 @@ struct OperandTile {
   std::uint16_t power[kLines][kGroup + 8];  // BF16 2^(6 e) times a scale, 0 for a zero
 };
 
-// Eight codes of line `line`, K positions [k, k + 8) of the group.
 // Two BF16 values 2^(6 e) scale of two magnitudes (0 for a zero).
 __device__ __forceinline__ std::uint32_t powers_of(const float lo, const float hi, const std::uint64_t scale) {
   const std::uint64_t p = pair_of(__uint_as_float(__float_as_uint(lo) & 0x7f800000U),
@@ -335,6 +334,8 @@ qgmma_emulation_rows_kernel(const std::uint8_t *__restrict__ input_codes,
                             const std::uint8_t *__restrict__ weight_codes,
                             bf16 *__restrict__ output, const std::size_t in_features,
                             const std::size_t out_features, const float output_scale) {
+  // (it releases and never waits, so it has to be launched plainly: a dependent launch that completes says nothing about
+  // the kernels further back)
   release_dependents();
   constexpr int kCodes = kGroup / kLanes, kWords = kCodes / 4;
   extern __shared__ __align__(16) unsigned char shared[];
