@@ -8,26 +8,20 @@
 //   acc   = truncate_to_13_fraction_bits(sum u)
 // and finally out = bf16(acc * output_scale).
 //
-// No tensor-core product reproduces the per-group alignment, so the products
-// are CUDA-core work; the parts around them are arranged to cost little:
-//   * a product and its truncation are one FMA: |a||b| + 2^23 u rounded toward
-//     zero is 2^23 u + trunc(|a||b| / u) u, because the sum lies in a binade
-//     whose ulp is u (|a||b| < 2^(E + 2) = 2^15 u) and |a||b| has 8 significant
-//     bits.  The integer is then the low 16 bits of the result.  Two K values
-//     share a packed FMA (fma.rz.f32x2);
-//   * the integers of two K values are packed into one word and added with
-//     their signs by dp2a; the signs are +-1 bytes, four K values per word, and
-//     their product is an exclusive or of the operands' words (one of them
-//     stored with its bit 0 flipped);
-//   * the exponent maximum is a tensor-core product: with 2^(6 e) for every
-//     operand, a sum over 32 products lies in [2^(6 E), 2^(6 E + 5)], so its
-//     F32 exponent divided by 6 is E whatever the accumulator rounds away
+// mma.sync with an F32 accumulator C adds its 16 products in one alignment: each product's magnitude is cut at 2^-25 of the
+// largest exponent among C and the products (measured on the B200 for BF16 and F16 operands; every test of this file's
+// results depends on it), and the sum at 2^-23 of its own.  So the emulation's products are tensor-core products:
+//   * C = 1.5 2^25 u cuts every product at u, for every output its own u;
+//   * the sum in C keeps multiples of 4 u only, so every K value takes four of the 16 places, and the sum is 4 times the
+//     emulated one and exact;
+//   * an E4M3 code's bits in an F16 value's place are the code's value times 2^-8;
+//   * the exponent maximum is a product as well: with 2^(6 e) for every operand, a sum over 32 products lies in
+//     [2^(6 E), 2^(6 E + 5)], so its F32 exponent divided by 6 is E whatever the accumulator rounds away
 //     (e is in [-9, 8], so the exponents stay within F32 and BF16).
-//     mma.sync's result layout is the thread's output tile.
-// What bounds it: the ALU (packing, signs, staging) and the half of the FMA pipe
-// that dp2a shares with the multiply-adds, busy for 52 and 55 % of the time with 16
-// warps per SM, in bursts that meet each other; about 3 instructions per product.  509 rows at 12288 x 4096: 3.5
-// ms = 7.4 T products/s; integer shifts per product took 17.1 ms.
+// What bounds it: some 36 ALU instructions, 37 of the FMA pipe (copies of operands among them) and 10 MMAs of 8 cycles per
+// 16 x 8 outputs and group, none of them more than half of the time; with few rows the unpacking of the weights, of which no
+// step is shared.  509 rows at 12288 x 4096: 1.08 ms = 24 T products/s (F32 multiply-adds that truncate, one product in half
+// an instruction and its sign in two more: 3.48 ms), 200 rows 0.52 (1.72), 8 rows 0.053 (0.229).
 #include "common.cuh"
 #include "ops_internal.hpp"
 
@@ -69,13 +63,6 @@ __device__ __forceinline__ std::uint32_t low_halves(const std::uint64_t pair) {
   return __byte_perm(static_cast<std::uint32_t>(pair), static_cast<std::uint32_t>(pair >> 32U), 0x5410);
 }
 
-// 2^E as F32 bits.  `powers` is the sum over the group's products of 2^(6 e) times 2^5 (stored with one operand), so
-// its exponent field is 132 + 6 E + 0 .. 5.  Without a product this gives E = -22: products' E is at least -18, so an
-// accumulator is a multiple of 2^-31 and loses nothing to a unit of 2^-35.
-__device__ __forceinline__ std::uint32_t largest_bits(const float powers, const float acc) {
-  const std::uint32_t sixth = ((__float_as_uint(powers) >> 15U) * 43691U) >> 26U;  // floor(field / 6)
-  return max((sixth << 23U) + (105U << 23U), __float_as_uint(acc) & 0x7f800000U);
-}
 // One group's step of an accumulator: `sum` is the signed sum of the truncated products in units of u.  The
 // accumulator's own part is truncated the same way as a product; all of it is exact in F32 (below 2^24 u).
 __device__ __forceinline__ float advanced(const float acc, const int sum, const std::uint32_t largest) {
@@ -85,259 +72,238 @@ __device__ __forceinline__ float advanced(const float acc, const int sum, const 
   return __uint_as_float(__float_as_uint(total) & 0xfffffc00U);
 }
 
-__device__ __forceinline__ std::uint32_t shared_address(const void *pointer) {
-  return static_cast<std::uint32_t>(__cvta_generic_to_shared(pointer));
-}
-__device__ __forceinline__ void load_matrices(std::uint32_t (&r)[4], const std::uint32_t address) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(address));
-}
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const std::uint32_t (&a)[4], const std::uint32_t b0,
                                          const std::uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-               "{%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_bf16_first(float (&d)[4], const std::uint32_t (&a)[4], const std::uint32_t b0,
+                                               const std::uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0F));
+}
+__device__ __forceinline__ void mma_f16(float (&d)[4], const std::uint32_t (&a)[4], const std::uint32_t b0,
+                                        const std::uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Rows (or columns) of one operand's group in shared memory.  The strides keep the 16-byte accesses of eight
-// neighbouring lines on different banks.
-template <int kLines>
-struct OperandTile {
-  float magnitude[kLines][kGroup + 4];
-  std::uint32_t sign[kLines][kGroup / 4 + 4];
-  std::uint16_t power[kLines][kGroup + 8];  // BF16 2^(6 e) times a scale, 0 for a zero
+// Eight codes of a line as tensor-core operands.  An E4M3 code's bits in the place of an F16 value's are the code's value
+// times 2^-8, subnormals and the code 0x7f (480) included.
+struct Operands {
+  std::uint32_t copies[8];  // the value, in both halves
+  std::uint32_t powers[4];  // BF16 pairs 2^(6 (e + 15) - 127), times 2^85 for weights; 0 for a zero
 };
-
-// Two BF16 values 2^(6 e) scale of two magnitudes (0 for a zero).
-__device__ __forceinline__ std::uint32_t powers_of(const float lo, const float hi, const std::uint64_t scale) {
-  const std::uint64_t p = pair_of(__uint_as_float(__float_as_uint(lo) & 0x7f800000U),
-                                  __uint_as_float(__float_as_uint(hi) & 0x7f800000U));
-  std::uint64_t square, fourth, result;
-  asm("mul.f32x2 %0, %1, %1;" : "=l"(square) : "l"(p));
-  asm("mul.f32x2 %0, %1, %2;" : "=l"(fourth) : "l"(square), "l"(scale));
-  asm("mul.f32x2 %0, %1, %1;" : "=l"(result) : "l"(square));
-  asm("mul.f32x2 %0, %1, %2;" : "=l"(result) : "l"(result), "l"(fourth));
-  return __byte_perm(static_cast<std::uint32_t>(result), static_cast<std::uint32_t>(result >> 32U), 0x7632);
+template <bool kWeights>
+__device__ __forceinline__ Operands operands_of(const uint2 codes) {
+  Operands r;
+#pragma unroll
+  for (int word = 0; word < 2; ++word) {
+    const std::uint32_t c = word == 0 ? codes.x : codes.y;
+    const std::uint32_t upper = (c & 0x80808080U) | ((c >> 1U) & 0x3f3f3f3fU), lower = (c << 7U) & 0x80808080U;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r.copies[4 * word + i] = __byte_perm(lower, upper, 0x4040U + 0x1111U * i);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const std::uint32_t pair = __byte_perm(lower, upper, 0x5140U + 0x2222U * i);
+      std::uint32_t normal, power;  // (every E4M3 value but 0 is a normal F16 number)
+      asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(normal) : "r"(pair), "r"(0x5c005c00U));  // 2^8
+      power = ((normal >> 3U) & 0x0f800f80U) * 6U;
+      if constexpr (kWeights) asm("mul.rn.bf16x2 %0, %0, %1;" : "+r"(power) : "r"(0x6a006a00U));  // 2^85
+      r.powers[2 * word + i] = power;
+    }
+  }
+  return r;
 }
 
-// Eight codes of line `line`, K positions [k, k + 8) of the group.
-template <int kLines>
-__device__ __forceinline__ void unpack(OperandTile<kLines> &tile, const int line, const int k, const uint2 codes,
-                                       const std::uint32_t sign_flip, const float scale) {
-  const float4 lo = magnitudes_of(codes.x), hi = magnitudes_of(codes.y);
-  *reinterpret_cast<float4 *>(&tile.magnitude[line][k]) = lo;
-  *reinterpret_cast<float4 *>(&tile.magnitude[line][k + 4]) = hi;
-  *reinterpret_cast<uint2 *>(&tile.sign[line][k / 4]) =
-      make_uint2(signs_of(codes.x) ^ sign_flip, signs_of(codes.y) ^ sign_flip);
-  const std::uint64_t scales = pair_of(scale, scale);
-  *reinterpret_cast<uint4 *>(&tile.power[line][k]) =
-      make_uint4(powers_of(lo.x, lo.y, scales), powers_of(lo.z, lo.w, scales), powers_of(hi.x, hi.y, scales),
-                 powers_of(hi.z, hi.w, scales));
+// 16 weight rows' group as mma.sync's A operands: row g, row g + 8, and for the products the same again.
+struct WeightTile {
+  std::uint32_t copies[8][4], powers[2][4];
+};
+__device__ __forceinline__ WeightTile weight_tile_of(const uint2 upper, const uint2 lower) {
+  const Operands a = operands_of<true>(upper), b = operands_of<true>(lower);
+  WeightTile t;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    t.copies[k][0] = a.copies[k];
+    t.copies[k][1] = b.copies[k];
+    t.copies[k][2] = a.copies[k];
+    t.copies[k][3] = b.copies[k];
+  }
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    t.powers[half][0] = a.powers[2 * half];
+    t.powers[half][1] = b.powers[2 * half];
+    t.powers[half][2] = a.powers[2 * half + 1];
+    t.powers[half][3] = b.powers[2 * half + 1];
+  }
+  return t;
+}
+// 2^(E - 14) as F32 bits (E counts products; an accumulator's own exponent is in the same place) from the sum of the powers,
+// whose exponent field is 6 (E + 23) + 0 .. 5: floor(field / 6) + 90, the high word of bits * 2^32 / 6.  Without a product E
+// is -23: products' E is at least -18, so an accumulator is a multiple of 2^-31 and loses nothing to a unit of 2^-36.
+__device__ __forceinline__ std::uint32_t sixth_of(const std::uint32_t bits) {
+  std::uint32_t d;
+  asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(bits), "r"(0x2aaaaaabU), "r"(90U << 23U));
+  return d;
 }
 
-// A CTA of eight warps owns kTileRows x kTileCols outputs, a warp 16 kM x 8 kN of them in mma.sync's layout.
-template <int kTileRows, int kTileCols, int kM, int kN>
+// A row's group in shared memory: lane c of a quad reads its eight K values as pairs of copies (two K values per 16-byte
+// word, 64 j + 16 c bytes in) and their powers.  Eight lanes of neighbouring rows meet different banks.
+struct __align__(16) RowGroup {
+  uint4 copies[4][4];
+  uint4 powers[4];
+};
+static_assert(sizeof(RowGroup) % 128 == 64, "neighbouring rows are half of the banks apart");
+
+// One group's step of four accumulators (mma.sync's result layout; 2^-14 of the emulated ones): 16 weight rows and eight
+// rows.  Two chains of products halve the wait for each other; they start on either side of zero and meet there.
+__device__ __forceinline__ void advance(float (&acc)[4], const WeightTile &w, const RowGroup &x, const int c) {
+  float powers[4], sum[4], other[4];
+  const uint4 p = x.powers[c];
+  mma_bf16_first(powers, w.powers[0], p.x, p.y);
+  mma_bf16(powers, w.powers[1], p.z, p.w);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float largest = fmaxf(fabsf(acc[q]), __uint_as_float(sixth_of(__float_as_uint(powers[q]))));
+    const float unit = __uint_as_float(__float_as_uint(largest) & 0x7f800000U);
+    const float lift = __uint_as_float((__float_as_uint(acc[q]) & 0x80000000U) | 0x44c00000U);  // +-1536: 1.5 2^(12 - 2)
+    sum[q] = __fmaf_rz(unit, lift, acc[q]);  // the accumulator's own part, truncated like a product
+    other[q] = -(unit * lift);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {
+    const uint4 b = x.copies[k / 2][c];
+    mma_f16(sum, w.copies[k], b.x, b.y);
+    mma_f16(other, w.copies[k + 1], b.z, b.w);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) acc[q] = __uint_as_float(__float_as_uint(sum[q] + other[q]) & 0xfffffc00U);  // 13 fraction bits
+}
+
+// A CTA owns 16 kWarps output columns (weight rows, unpacked in registers by the one warp that uses them) x 8 kN rows
+// (unpacked in shared memory, kDepth groups at a time).
+template <int kNTiles, int kWarpCount, int kGroups, int kResident>
 struct EmulationShape {
-  static constexpr int kRows = kTileRows, kCols = kTileCols, kMTiles = kM, kNTiles = kN;
-  static constexpr int kRowWarps = kTileRows / (16 * kM);
-  static_assert(kRowWarps * (kTileCols / (8 * kN)) == 8, "eight warps");
-  struct Stage {
-    OperandTile<kTileRows> a;
-    OperandTile<kTileCols> b;
-  };
+  static constexpr int kN = kNTiles, kWarps = kWarpCount, kDepth = kGroups, kBlocks = kResident;
+  static constexpr int kThreads = 32 * kWarps, kRows = 8 * kN, kCols = 16 * kWarps;
+  using Stage = RowGroup[kDepth][kRows];
 };
-
-constexpr int kEmulationThreads = 256;
 
 template <class Shape>
-__global__ void __launch_bounds__(kEmulationThreads)
+__global__ void __launch_bounds__(Shape::kThreads, Shape::kBlocks)
 qgmma_emulation_kernel(const std::uint8_t *__restrict__ input_codes,
                        const std::uint8_t *__restrict__ weight_codes,
                        bf16 *__restrict__ output, const std::size_t rows,
                        const std::size_t in_features,
                        const std::size_t out_features,
                        const float output_scale) {
-  constexpr int kM = Shape::kMTiles, kN = Shape::kNTiles;
+  constexpr int kN = Shape::kN, kThreads = Shape::kThreads, kDepth = Shape::kDepth, kRows = Shape::kRows;
+  constexpr int kPieces = kRows * 4 * kDepth, kShare = (kPieces + kThreads - 1) / kThreads;
+  // (it releases and never waits, so it has to be launched plainly: a dependent launch that completes says nothing about
+  // the kernels further back)
+  if constexpr (kN == 1) release_dependents();
   using Stage = typename Shape::Stage;
   extern __shared__ __align__(16) unsigned char shared[];
   Stage *const stages = reinterpret_cast<Stage *>(shared);
-  const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
-  const int warp_row = warp % Shape::kRowWarps * (16 * kM), warp_col = warp / Shape::kRowWarps * (8 * kN);
-  const std::size_t row0 = static_cast<std::size_t>(blockIdx.y) * Shape::kRows;
-  const std::size_t col0 = static_cast<std::size_t>(blockIdx.x) * Shape::kCols;
+  const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32, g = lane / 4, c = lane % 4;
+  const std::size_t row0 = static_cast<std::size_t>(blockIdx.y) * kRows;
+  const std::size_t col0 = static_cast<std::size_t>(blockIdx.x) * Shape::kCols + warp * 16 + g;
+  const int groups = static_cast<int>(in_features / kGroup);
 
-  // staging: a thread unpacks eight codes of a line at a time
-  constexpr int kALoads = Shape::kRows * 4 / kEmulationThreads, kBLoads = Shape::kCols * 4 / kEmulationThreads;
-  constexpr int kAShare = kALoads == 0 ? 1 : kALoads;
-  uint2 a_codes[kAShare], b_codes[kBLoads];
-  const bool loads_a = kALoads != 0 || tid < Shape::kRows * 4;
-  const auto fetch = [&](const std::size_t k0) {
+  // rows: a thread unpacks eight codes at a time, piece (row, group, eighth)
+  uint2 x_codes[kShare];
+  const auto fetch_rows = [&](const int group0) {
 #pragma unroll
-    for (int i = 0; i < kAShare; ++i) {
-      const std::size_t row = row0 + (tid + i * kEmulationThreads) / 4;
-      a_codes[i] = loads_a && row < rows
-                       ? __ldg(reinterpret_cast<const uint2 *>(input_codes + row * in_features + k0 + tid % 4 * 8))
-                       : make_uint2(0U, 0U);
-    }
-#pragma unroll
-    for (int i = 0; i < kBLoads; ++i) {
-      const std::size_t col = col0 + (tid + i * kEmulationThreads) / 4;
-      b_codes[i] = col < out_features
-                       ? __ldg(reinterpret_cast<const uint2 *>(weight_codes + col * in_features + k0 + tid % 4 * 8))
-                       : make_uint2(0U, 0U);
+    for (int i = 0; i < kShare; ++i) {
+      const int piece = tid + i * kThreads, group = group0 + piece / 4 % kDepth;
+      const std::size_t row = row0 + piece / (4 * kDepth);
+      x_codes[i] = make_uint2(0U, 0U);
+      if ((kPieces % kThreads == 0 || piece < kPieces) && row < rows && group < groups)
+        x_codes[i] = __ldg(reinterpret_cast<const uint2 *>(input_codes + row * in_features + group * kGroup + piece % 4 * 8));
     }
   };
-  const auto stage_codes = [&](Stage &stage) {
-    if (loads_a) {
+  const auto publish_rows = [&](Stage &stage) {
 #pragma unroll
-      for (int i = 0; i < kAShare; ++i) unpack(stage.a, (tid + i * kEmulationThreads) / 4, tid % 4 * 8, a_codes[i], 0U, 1.0F);
+    for (int i = 0; i < kShare; ++i) {
+      const int piece = tid + i * kThreads;
+      if (kPieces % kThreads != 0 && piece >= kPieces) break;
+      const Operands o = operands_of<false>(x_codes[i]);
+      RowGroup &out = stage[piece / 4 % kDepth][piece / (4 * kDepth)];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        out.copies[j][piece % 4] = make_uint4(o.copies[2 * j], o.copies[2 * j], o.copies[2 * j + 1], o.copies[2 * j + 1]);
+      out.powers[piece % 4] = make_uint4(o.powers[0], o.powers[1], o.powers[2], o.powers[3]);
     }
+  };
+  // weights: a stage's worth of groups in flight
+  uint2 w_codes[kDepth][2];
+  const std::uint8_t *w_rows[2];
 #pragma unroll
-    for (int i = 0; i < kBLoads; ++i)
-      unpack(stage.b, (tid + i * kEmulationThreads) / 4, tid % 4 * 8, b_codes[i], 0x01010101U, 32.0F);
+  for (int h = 0; h < 2; ++h) {
+    const std::size_t column = col0 + 8 * h;
+    w_rows[h] = weight_codes + (column < out_features ? column : out_features - 1) * in_features + 8 * c;
+  }
+  const auto fetch_weights = [&](const int d, const int group) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      w_codes[d][h] = __ldg(reinterpret_cast<const uint2 *>(w_rows[h] + min(group, groups - 1) * kGroup));
   };
 
-  float acc[kM][kN][4];
+  float acc[kN][4] = {};
 #pragma unroll
-  for (int m = 0; m < kM; ++m)
-#pragma unroll
-    for (int n = 0; n < kN; ++n)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[m][n][q] = 0.0F;
-
-  fetch(0);
-  stage_codes(stages[0]);
+  for (int d = 0; d < kDepth; ++d) fetch_weights(d, d);
+  fetch_rows(0);
+  publish_rows(stages[0]);
   __syncthreads();
-  for (std::size_t k0 = 0, at = 0; k0 < in_features; k0 += kGroup, at ^= 1) {
+  int at = 0;
+  for (int group0 = 0; group0 < groups; group0 += kDepth, at ^= 1) {
     const Stage &stage = stages[at];
-    const bool more = k0 + kGroup < in_features;
-    if (more) fetch(k0 + kGroup);
-
-    // E of every output
-    float powers[kM][kN][4];
-    {
-      std::uint32_t b_power[kN][2][2];
+    const bool more = group0 + kDepth < groups;
+    if (more) fetch_rows(group0 + kDepth);
 #pragma unroll
-      for (int n = 0; n < kN; ++n) {
-        std::uint32_t r[4];  // the four 8-wide K blocks of eight columns
-        load_matrices(r, shared_address(&stage.b.power[warp_col + n * 8 + lane % 8][lane / 8 * 8]));
-        b_power[n][0][0] = r[0];
-        b_power[n][0][1] = r[1];
-        b_power[n][1][0] = r[2];
-        b_power[n][1][1] = r[3];
-      }
+    for (int d = 0; d < kDepth; ++d) {  // (a group beyond the last meets rows of zeros and changes nothing)
+      const WeightTile w = weight_tile_of(w_codes[d][0], w_codes[d][1]);
+      fetch_weights(d, group0 + d + kDepth);
 #pragma unroll
-      for (int m = 0; m < kM; ++m) {
-        std::uint32_t a_power[2][4];
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-          load_matrices(a_power[half],
-                        shared_address(&stage.a.power[warp_row + m * 16 + lane % 16][half * 16 + lane / 16 * 8]));
-#pragma unroll
-        for (int n = 0; n < kN; ++n) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) powers[m][n][q] = 0.0F;
-#pragma unroll
-          for (int half = 0; half < 2; ++half)
-            mma_bf16(powers[m][n], a_power[half], b_power[n][half][0], b_power[n][half][1]);
-        }
-      }
+      for (int n = 0; n < kN; ++n) advance(acc[n], w, stage[d][8 * n + g], c);
     }
-    std::uint64_t magic[kM][kN][4];
-    int sum[kM][kN][4];
-#pragma unroll
-    for (int m = 0; m < kM; ++m)
-#pragma unroll
-      for (int n = 0; n < kN; ++n)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float value = __uint_as_float(largest_bits(powers[m][n][q], acc[m][n][q]) + (10U << 23U));
-          magic[m][n][q] = pair_of(value, value);
-          sum[m][n][q] = 0;
-        }
-
-#pragma unroll  // (two steps at a time: 3 % slower, four 16 %; with all of them the packing mixes with the multiply-adds)
-    for (int k = 0; k < kGroup; k += 4) {
-      std::uint64_t a_value[kM][2][2], b_value[kN][2][2];
-      std::uint32_t a_sign[kM][2], b_sign[kN][2];
-#pragma unroll
-      for (int m = 0; m < kM; ++m)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int line = warp_row + m * 16 + h * 8 + lane / 4;
-          const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(&stage.a.magnitude[line][k]);
-          a_value[m][h][0] = v.x;
-          a_value[m][h][1] = v.y;
-          a_sign[m][h] = stage.a.sign[line][k / 4];
-        }
-#pragma unroll
-      for (int n = 0; n < kN; ++n)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int line = warp_col + n * 8 + lane % 4 * 2 + h;
-          const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(&stage.b.magnitude[line][k]);
-          b_value[n][h][0] = v.x;
-          b_value[n][h][1] = v.y;
-          b_sign[n][h] = stage.b.sign[line][k / 4];
-        }
-#pragma unroll
-      for (int m = 0; m < kM; ++m)
-#pragma unroll
-        for (int n = 0; n < kN; ++n)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const std::uint64_t t0 = truncated_products(a_value[m][q / 2][0], b_value[n][q % 2][0], magic[m][n][q]);
-            const std::uint64_t t1 = truncated_products(a_value[m][q / 2][1], b_value[n][q % 2][1], magic[m][n][q]);
-            const int sign = static_cast<int>(a_sign[m][q / 2] ^ b_sign[n][q % 2]);
-            sum[m][n][q] = __dp2a_lo(static_cast<int>(low_halves(t0)), sign, sum[m][n][q]);
-            sum[m][n][q] = __dp2a_hi(static_cast<int>(low_halves(t1)), sign, sum[m][n][q]);
-          }
-    }
-#pragma unroll
-    for (int m = 0; m < kM; ++m)
-#pragma unroll
-      for (int n = 0; n < kN; ++n)
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          acc[m][n][q] = advanced(acc[m][n][q], sum[m][n][q],
-                                  static_cast<std::uint32_t>(magic[m][n][q]) - (10U << 23U));
-    if (more) stage_codes(stages[at ^ 1]);
+    if (more) publish_rows(stages[at ^ 1]);
     __syncthreads();
   }
 #pragma unroll
-  for (int m = 0; m < kM; ++m)
+  for (int n = 0; n < kN; ++n)
 #pragma unroll
-    for (int n = 0; n < kN; ++n)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const std::size_t row = row0 + warp_row + m * 16 + q / 2 * 8 + lane / 4;
-        const std::size_t column = col0 + warp_col + n * 8 + lane % 4 * 2 + q % 2;
-        if (row < rows && column < out_features)
-          output[row * out_features + column] = f2bf(acc[m][n][q] * output_scale);
-      }
+    for (int q = 0; q < 4; ++q) {
+      const std::size_t column = col0 + q / 2 * 8, row = row0 + 8 * n + 2 * c + q % 2;
+      if (row < rows && column < out_features)
+        output[row * out_features + column] = f2bf(acc[n][q] * 0x1p14F * output_scale);
+    }
 }
 
-// One or two rows (cached decode): kLanes neighbouring lanes share one output
+// One row (cached decode): kLanes neighbouring lanes share one output
 // column and split each 32-product group between them (a column's group is one
 // 32-byte sector of codes).  The group maximum and the aligned integer sum are
 // combined across them with shuffles - integer addition is exact, so the
 // result is the one accumulator chain of the tiled kernel above, bit for bit.
-// The rows sit unpacked in shared memory: their magnitudes, signs and, two to a
+// The row sits unpacked in shared memory: its magnitudes, signs and, two to a
 // word, exponent fields; the maximum of a group's exponent sums does not need
 // the accumulator and is taken a group ahead of it.
 constexpr int kRowKernelThreads = 128;
 
-template <int kRows, int kLanes, int kAhead>
+template <int kLanes, int kAhead>
 __global__ void __launch_bounds__(kRowKernelThreads)
-qgmma_emulation_rows_kernel(const std::uint8_t *__restrict__ input_codes,
+qgmma_emulation_row_kernel(const std::uint8_t *__restrict__ input_codes,
                             const std::uint8_t *__restrict__ weight_codes,
                             bf16 *__restrict__ output, const std::size_t in_features,
                             const std::size_t out_features, const float output_scale) {
   // (it releases and never waits, so it has to be launched plainly: a dependent launch that completes says nothing about
   // the kernels further back)
   release_dependents();
-  constexpr int kCodes = kGroup / kLanes, kWords = kCodes / 4;
+  constexpr int kRows = 1, kCodes = kGroup / kLanes, kWords = kCodes / 4;
   extern __shared__ __align__(16) unsigned char shared[];
   float *const x_magnitude = reinterpret_cast<float *>(shared);                                // [kRows][in_features]
   std::uint32_t *const x_field = reinterpret_cast<std::uint32_t *>(x_magnitude + kRows * in_features);  // [..][/ 2]
@@ -476,7 +442,7 @@ int launch_tiled(const void *input_codes, const void *weight_codes, const std::s
   auto *const kernel = qgmma_emulation_kernel<Shape>;
   const int status = allow_shared_memory(kernel, smem);
   if (status != kOk) return status;
-  kernel<<<grid, kEmulationThreads, smem, stream>>>(
+  kernel<<<grid, Shape::kThreads, smem, stream>>>(
       static_cast<const std::uint8_t *>(input_codes), static_cast<const std::uint8_t *>(weight_codes),
       static_cast<bf16 *>(output), rows, in_features, out_features, output_scale);
   return check_launch("software E4M3 QGMMA emulation kernel");
@@ -502,15 +468,14 @@ int e4m3_emulated_gemm(const void *input_codes, const void *weight_codes,
                 "software E4M3 linear code buffers must be 8-byte aligned");
   // per K value of a row: magnitude, half a word of exponent field, a sign byte
   const std::size_t row_bytes = rows * in_features * 7;
-  if (rows <= 2 && row_bytes <= 168 * 1024 &&
+  if (rows == 1 && row_bytes <= 168 * 1024 &&
       (reinterpret_cast<std::uintptr_t>(weight_codes) & 15U) == 0) {
     // Two lanes per column share the fixed work of a group between more products, four keep more warps in flight:
     // one row at N x K = 24576 x 8192 takes 133 us with two and 166 with four, at 12288 x 4096 66 and 59 us, at
     // 5760 x 1920 38 and 33 us.  From two warps per scheduler on (148 x 256 threads) two lanes are enough.
     const bool two_lanes = out_features * 2 >= std::size_t{148} * 256;
     const unsigned int blocks = ceil_div_u(out_features, kRowKernelThreads / (two_lanes ? 2 : 4));
-    auto *const kernel = rows == 1 ? (two_lanes ? qgmma_emulation_rows_kernel<1, 2, 8> : qgmma_emulation_rows_kernel<1, 4, 16>)
-                                   : (two_lanes ? qgmma_emulation_rows_kernel<2, 2, 8> : qgmma_emulation_rows_kernel<2, 4, 16>);
+    auto *const kernel = two_lanes ? qgmma_emulation_row_kernel<2, 8> : qgmma_emulation_row_kernel<4, 16>;
     const int status = allow_shared_memory(kernel, row_bytes);
     if (status != kOk) return status;
     // (not a dependent launch: started beside a projection that still runs, its CTAs crowd on the SMs that are free
@@ -525,14 +490,14 @@ int e4m3_emulated_gemm(const void *input_codes, const void *weight_codes,
     return launch_tiled<decltype(shape)>(input_codes, weight_codes, rows, in_features, out_features, output_scale,
                                          output, stream);
   };
-  // The largest tile amortises the unpacking and the fixed work of a group best (1,024 rows, 12288 x 4096: 6.8 ms
-  // against 7.4 ms with 32 rows), unless it pads more rows or leaves SMs without their two CTAs (61 rows: 0.69
-  // against 0.57 ms; 200 rows: 1.98 against 1.79 ms; 16 rows: 0.39 ms with 32 rows per tile, 0.25 ms with 16).
-  if (rows <= 16) return tiled(EmulationShape<16, 64, 1, 1>{});
-  const std::size_t tiles64 = (rows + 63) / 64, tiles32 = (rows + 31) / 32;
-  if (tiles64 * 64 * 100 <= tiles32 * 32 * 106 && tiles64 * ceil_div_u(out_features, 64) >= std::size_t{2} * 148)
-    return tiled(EmulationShape<64, 64, 2, 2>{});
-  return tiled(EmulationShape<32, 64, 2, 1>{});
+  // A warp unpacks its weights for 8, 16 or 64 rows.  64 rows share the unpacking best (509 rows, 12288 x 4096: 1.08 ms against
+  // 1.27 with 16), unless they pad (200 rows: 0.60 against 0.52 ms) or leave SMs without two CTAs (64 rows at 12288 x 4096: 0.22
+  // against 0.19 ms, at 24576 x 8192, twice the CTAs, 0.61 against 0.69).
+  if (rows <= 8) return tiled(EmulationShape<1, 4, 8, 4>{});
+  const std::size_t tall = (rows + 63) / 64 * 64, flat = (rows + 15) / 16 * 16;
+  if (tall * 100 <= flat * 110 && tall / 64 * ceil_div_u(out_features, 64) >= std::size_t{2} * 148)
+    return tiled(EmulationShape<8, 4, 1, 3>{});
+  return tiled(EmulationShape<2, 4, 4, 4>{});
 }
 
 }  // namespace evob

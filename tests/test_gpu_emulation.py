@@ -44,3 +44,33 @@ def test_emulated_projection_at_kernel_edges(ops, oracle, rows, inner, columns, 
     expected = np.empty((rows, columns), np.uint16)
     oracle.qgmma_codes(ptr(x), ptr(w), rows, inner, columns, 0.0625, ptr(expected))
     assert np.array_equal(host_bits(out), expected)
+
+
+@pytest.mark.parametrize("rows,inner,columns", [(2, 288, 65), (8, 32, 15), (9, 160, 17), (16, 96, 4736), (64, 96, 18944),
+                                               (256, 64, 4737), (449, 32, 2433)])
+def test_emulated_projection_with_every_weight_code(ops, oracle, rows, inner, columns):
+    """Weights of all codes, in tiles of 8, 16 and 64 rows with remainders and groups that do not fill a stage.  The code
+    of a NaN counts as 480 (the oracle has none): it meets one value of 0.5 in its group."""
+    rng = np.random.default_rng(rows + inner + columns)
+    x = _codes(rng, "any", (rows, inner))
+    w = rng.permutation(np.resize(np.arange(256, dtype=np.uint8), columns * inner)).reshape(columns, inner)
+    w[(w & 0x7f) == 0x7f] ^= 1
+    x[rows // 2], x[rows // 2, inner - 7] = 0, 0x30
+    w = np.ascontiguousarray(w)
+    values = torch.from_numpy(x).view(torch.float8_e4m3fn).float().numpy()
+    scratch = torch.empty(x.size, dtype=torch.uint8, device="cuda")
+    expected = np.empty((rows, columns), np.uint16)
+    oracle.qgmma_codes(ptr(x), ptr(w), rows, inner, columns, 0.0625, ptr(expected))
+    for code in (None, 0x7f, 0xff):
+        if code is not None:
+            w[columns - 1, inner - 7] = code
+            expected[rows // 2, columns - 1] = f32_to_bf16(np.float32([15.0 if code == 0x7f else -15.0]))[0]
+        out = empty_bits(rows, columns)
+        ops.call("software_e4m3_h100_linear", p(dev_bits(f32_to_bf16(values))), p(dev(w)), rows, inner, columns, 1.0,
+                 0.0625, p(scratch), p(out), stream())
+        got = host_bits(out)
+        if code is not None:  # (the other rows meet 480 as well)
+            got = got[rows // 2], expected[rows // 2]
+            assert np.array_equal(*got)
+        else:
+            assert np.array_equal(got, expected)
