@@ -60,6 +60,7 @@ struct LinearF32Args {
   const float *row_scale = nullptr, *bias = nullptr;
   const int *row_group = nullptr;
   std::size_t row_fanout = 1;
+  std::size_t groups = 0;  // with tile_group; 0 (unknown) keeps the products on the CUDA cores
   const int *tile_group = nullptr, *tile_count = nullptr;
   std::size_t tile_rows = 128;
   bool dependent_launch = false;  // one row: as LinearArgs::dependent_launch

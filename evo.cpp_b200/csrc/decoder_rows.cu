@@ -5,8 +5,7 @@
 
 #include <type_traits>
 
-#include "decoder_types.cuh"
-#include "gates.cuh"
+#include "linear_f32.cuh"
 #include "ops_internal.hpp"
 
 namespace cg = cooperative_groups;
@@ -346,28 +345,8 @@ gated_activation_kernel(const float *__restrict__ input, T *__restrict__ output,
   }
 }
 
-struct F32Params {
-  const bf16 *weight;
-  float *output;
-  int rows, out_features, in_features, accumulate;
-  float alpha, softcap;
-  const float *row_scale, *bias;
-  const int *row_group;
-  int row_fanout;
-  const int *tile_group, *tile_count;
-  int tile_rows;
-};
-
-__device__ __forceinline__ void store_f32_result(const F32Params &p, const std::size_t row, const int column,
-                                                 const float product) {
-  float *const out = p.output + row * p.out_features + column;
-  float value = product * (p.row_scale != nullptr ? p.alpha * p.row_scale[row] : p.alpha);
-  if (p.accumulate != 0) value += *out;
-  if (p.bias != nullptr) value += p.bias[column];
-  *out = soft_cap(value, p.softcap);
-}
-
-// A cluster of `splits` CTAs owns one tile of 16 kRows rows x 128 columns and divides K between its CTAs; every thread
+// Rows and weights that the tensor cores' kernel does not take (inner sizes that are no multiple of 8 or below 64, operands that
+// are not aligned).  A cluster of `splits` CTAs owns one tile of 16 kRows rows x 128 columns and divides K between its CTAs; every thread
 // keeps kRows x 8 outputs as packed pairs, the sums over even and over odd K (fma.rn.f32x2, operands straight from
 // K-contiguous rows of shared memory).  What bounds it is the F32 pipe; the split gives a few dozen rows (one row tile)
 // enough CTAs, and makes the chains of additions short: K / (2 splits) terms in a pair's half, then a sum over the halves
@@ -512,6 +491,48 @@ linear_f32_rows_kernel(const T *__restrict__ input, const F32Params p) {
   }
   sum = warp_sum(sum);
   if (lane == 0) store_f32_result(p, row, column, sum);
+}
+
+// Two rows: a warp per three outputs of both, so that the weights come from L2 once and the rows from L1 once per three
+// columns.  What bounds it is L1 (2 rows of 2048 x 8448: 8.6 us, 4096 x 11264: 17.8; two columns a warp 10.5 and 24.9, one
+// row and column a warp 16.6 and 36.9).
+constexpr int kPairColumns = 3;
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+linear_f32_two_rows_kernel(const T *__restrict__ input, const F32Params p) {
+  wait_for_producers(input);
+  release_dependents();
+  const int column0 = (blockIdx.x * 8 + threadIdx.x / 32) * kPairColumns, lane = threadIdx.x % 32;
+  if (column0 >= p.out_features) return;
+  const bf16 *w[kPairColumns];  // (columns beyond the last are computed and dropped)
+#pragma unroll
+  for (int c = 0; c < kPairColumns; ++c)
+    w[c] = p.weight + static_cast<std::size_t>(min(column0 + c, p.out_features - 1)) * p.in_features;
+  float sum[2][kPairColumns] = {};
+#pragma unroll 4
+  for (int k = 8 * lane; k < p.in_features; k += 256) {
+    float b[kPairColumns][8];
+#pragma unroll
+    for (int c = 0; c < kPairColumns; ++c) load_floats<8>(w[c] + k, b[c]);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      float a[8];
+      load_floats<8>(input + static_cast<std::size_t>(r) * p.in_features + k, a);
+#pragma unroll
+      for (int c = 0; c < kPairColumns; ++c)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum[r][c] = fmaf(a[i], b[c][i], sum[r][c]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int c = 0; c < kPairColumns; ++c) {
+      const float total = warp_sum(sum[r][c]);
+      if (lane == r * kPairColumns + c && column0 + c < p.out_features)
+        store_f32_result(p, static_cast<std::size_t>(r), column0 + c, total);
+    }
 }
 
 bool row_vector_ok(const std::size_t width, const void *a, const void *b, const void *c) {
@@ -695,9 +716,19 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
   p.tile_count = a.tile_count;
   p.tile_rows = static_cast<int>(a.tile_rows);
   const bool vector = a.in_features % 8 == 0 && aligned16(a.input) && aligned16(a.weight);
-  // Every row of the few-row kernel fetches the weights again, from L2 where they fit.  The tile kernel fetches them once,
-  // for 32 rows or more, and its steps wait for memory: 2 rows of 2048 x 8448 take 18 us against 90, 12 rows 72 against 90,
-  // 16 rows of 8448 x 2048 90 against 136, of 2048 x 8448 92 against 91; but 16 rows of 4096 x 22528 (185 MB) 520 against 397.
+  const bool plain = a.row_group == nullptr && a.tile_group == nullptr;
+  // (2 rows of 2048 x 2048: 7 us with either kernel, of 8448 x 2048 14.6 with a warp per output and 18.6 with one per three,
+  // which leaves the SMs four warps each)
+  const bool two_rows = plain && vector && a.rows == 2 && a.out_features >= 4096;
+  // Every row of the few-row kernel fetches the weights again, from L2 where they fit.  The tensor cores' kernel fetches them
+  // once, but takes 12 us to start and to add its shares up: 4 rows of 2048 x 2048 take 14.3 us against 14.3, 12 of 2048 x 512
+  // 10.2 against 12.3, 3 of 2048 x 6144 22.5 against 22.5; 6 of 2048 x 2048 16.4 against 14.3, 16 of 2048 x 8448 96 against 23.
+  constexpr std::size_t kFewRowProducts = std::size_t{24} << 20;
+  if ((a.tile_group != nullptr || a.rows > 16 || (a.rows > 2 && a.rows * a.in_features * a.out_features > kFewRowProducts)) &&
+      tensorcore_linear_f32_applicable(a))
+    return tensorcore_linear_f32(a, p, stream);
+  // Against the tile kernel on the CUDA cores: 2 rows of 2048 x 8448 take 18 us against 90, 12 rows 72 against 90, 16 rows of
+  // 8448 x 2048 90 against 136, of 2048 x 8448 92 against 91; but 16 rows of 4096 x 22528 (185 MB) 520 against 397.
   constexpr std::size_t kL2Weights = std::size_t{96} << 20;
   const bool few_rows = a.row_group != nullptr ||
                         (a.tile_group == nullptr &&
@@ -705,6 +736,9 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
   const auto launch = [&](auto tag) {
     using T = decltype(tag);
     const T *const input = static_cast<const T *>(a.input);
+    if (two_rows)
+      return launch_dependent("F32 linear kernel (two rows)", linear_f32_two_rows_kernel<T>,
+                              dim3(ceil_div_u(a.out_features, 8 * kPairColumns)), 256, 0, stream, true, 1, input, p);
     if (few_rows) {
       const auto kernel = vector ? linear_f32_rows_kernel<T, true> : linear_f32_rows_kernel<T, false>;
       return launch_dependent("F32 linear kernel (few rows)", kernel,

@@ -768,6 +768,7 @@ int evo_b200_projection(const evo_b200_projection_args *args, void *stream) {
     shared(a);
     a.input_type = activation_of(args->float32 == 1);
     a.bias = static_cast<const float *>(args->bias);
+    a.groups = args->groups;
     a.output = static_cast<float *>(args->output);
     return linear_f32(a, as_stream(stream));
   }

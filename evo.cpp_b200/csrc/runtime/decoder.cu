@@ -480,6 +480,7 @@ int Context::expert_feed_forward(Stage &s, const std::size_t i, const std::size_
   } else {
     LinearF32Args a;
     grouping(a, true);
+    a.groups = b.experts;
     a.input_type = type;
     a.output = static_cast<float *>(s.gate_products);
     EVOB_OP(kCatGemmGrouped, linear_f32(a, stream));
@@ -499,6 +500,7 @@ int Context::expert_feed_forward(Stage &s, const std::size_t i, const std::size_
   } else {
     LinearF32Args a;
     grouping(a, false);
+    a.groups = b.experts;
     a.input_type = type;
     a.output = static_cast<float *>(s.expert_out);
     EVOB_OP(kCatGemmGrouped, linear_f32(a, stream));

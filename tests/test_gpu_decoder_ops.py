@@ -145,6 +145,46 @@ def test_few_f32_rows(ops, rows, inner, outer):
     assert np.all(error <= chain * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(wv).T + np.abs(base)))
 
 
+@pytest.mark.parametrize("rows, inner, outer", [(17, 64, 127), (32, 64, 1), (33, 72, 129), (96, 200, 128), (97, 1080, 260), (128, 2048, 40),
+                                                (129, 136, 1000), (3, 2056, 6150), (16, 4104, 2049), (2, 264, 4096), (2, 2056, 4099)])
+def test_f32_products_on_the_tensor_cores(ops, rows, inner, outer):
+    """Every row tile, K blocks and weight tiles with remainders, one CTA and clusters that divide K, and two rows.  A block
+    of 64 products is cut 12 times at 2^-23 of a sum of at most its magnitudes (the smaller planes' cuts are below that), the
+    blocks' sums are rounded: 16 + ceil(inner / 64) / 8 + 8 units of 2^-24.  Then values that are not finite, and the
+    smallest ones: the same infinities and NaNs as multiply-adds give."""
+    import torch
+
+    rng = np.random.default_rng(rows * 1000 + inner)
+    w, wv = activation(rng.normal(0, 1, (outer, inner)), 0)
+    x, base = (rng.normal(0, 1, shape).astype(np.float32) for shape in ((rows, inner), (rows, outer)))
+    x *= np.exp(rng.normal(0, 2, x.shape)).astype(np.float32)
+    exact, out = cuda(x), cuda(base)
+    ops.call("f32_linear", exact.data_ptr(), w.data_ptr(), rows, inner, outer, 1, out.data_ptr(), stream())
+    error = np.abs(out.double().cpu().numpy() - (x.astype(np.float64) @ wv.T + base))
+    bound = (16 + inner / 64 / 8 + 8) * 2.0 ** -24 if rows > 2 else 16 * (-(-inner // 256) + 4) * 2.0 ** -24
+    assert np.all(error <= bound * (np.abs(x).astype(np.float64) @ np.abs(wv).T + np.abs(base)))
+
+    odd = torch.zeros(rows, inner, device="cuda")
+    odd[0, 1], odd[0, 5] = float("inf"), 2.0
+    odd[1, inner - 1], odd[1, 2] = float("nan"), 1.0
+    if rows > 2:
+        odd[2, 3], odd[2, inner - 2] = float("-inf"), float("inf")
+        odd[rows - 1, 7] = 1.5  # meets the infinite weight with planes that are zero
+    w[:, 1], w[:, 3], w[:, inner - 2] = 1.0, -2.0, -0.5
+    w[outer // 2, 7] = float("inf")
+    out = empty((rows, outer), 1)
+    ops.call("f32_linear", odd.data_ptr(), w.data_ptr(), rows, inner, outer, 0, out.data_ptr(), stream())
+    ops.call("check_async_errors", stream())
+    expected = torch.zeros(rows, outer, dtype=torch.float64, device="cuda")
+    for k in (1, 2, 3, 5, 7, inner - 2, inner - 1):  # (0 times an infinity is a NaN here too)
+        expected += odd[:, k:k + 1].double() * w[:, k].double()
+    assert torch.equal(out.isnan(), expected.isnan())
+    assert torch.equal(out.isinf(), expected.isinf())
+    finite = expected.isfinite()
+    assert torch.equal(out[out.isinf()].sign().double(), expected[out.isinf()].sign())
+    assert torch.allclose(out[finite].double(), expected[finite], rtol=2e-7, atol=0.0)
+
+
 def test_few_f32_rows_cost_less_than_a_tile(ops):
     """Two rows are a stream of the weights; a tile pads them to 32 (18 us against 90 at this size)."""
     import torch
