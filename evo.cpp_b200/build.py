@@ -32,7 +32,7 @@ FLAGS = [
 ]
 
 KERNEL_SOURCES = [
-    "errors.cu", "elementwise.cu", "qgmma_emulation.cu", "gemm_tcgen05.cu", "gemv.cu",
+    "errors.cu", "elementwise.cu", "qgmma_emulation.cu", "qgmma_emulation_tcgen05.cu", "gemm_tcgen05.cu", "gemv.cu",
     "hyena_fir.cu", "hyena_fir_fused.cu", "hyena_fir_tcgen05.cu", "hyena_modal.cu", "hyena_decode.cu", "attention.cu", "attention_flash.cu", "attention_tcgen05.cu", "attention_tcgen05_k64.cu", "attention_decode.cu", "kv_q8.cu", "linear_executor.cu", "fp8_codec.cpp",
     "decoder_rows.cu", "linear_f32_tcgen05.cu", "attention_window.cu", "recurrent_mixers.cu", "recurrent_chunks.cu",
     "latent_attention.cu", "experts.cu",

@@ -8,9 +8,10 @@
 //   acc   = truncate_to_13_fraction_bits(sum u)
 // and finally out = bf16(acc * output_scale).
 //
-// mma.sync with an F32 accumulator C adds its 16 products in one alignment: each product's magnitude is cut at 2^-25 of the
-// largest exponent among C and the products (measured on the B200 for BF16 and F16 operands; every test of this file's
-// results depends on it), and the sum at 2^-23 of its own.  So the emulation's products are tensor-core products:
+// A tensor-core product with an F32 accumulator C adds its 16 products in one alignment: each product's magnitude is cut at
+// 2^-25 of the largest exponent among C and the products, and the sum at 2^-23 of its own (measured on the B200 for BF16 and
+// F16 operands of mma.sync and tcgen05.mma; every test of this file's results depends on it).  So the emulation's products
+// are tensor-core products:
 //   * C = 1.5 2^25 u cuts every product at u, for every output its own u;
 //   * the sum in C keeps multiples of 4 u only, so every K value takes four of the 16 places, and the sum is 4 times the
 //     emulated one and exact;
@@ -18,17 +19,18 @@
 //   * the exponent maximum is a product as well: with 2^(6 e) for every operand, a sum over 32 products lies in
 //     [2^(6 E), 2^(6 E + 5)], so its F32 exponent divided by 6 is E whatever the accumulator rounds away
 //     (e is in [-9, 8], so the exponents stay within F32 and BF16).
-// What bounds it: some 36 ALU instructions, 37 of the FMA pipe (copies of operands among them) and 10 MMAs of 8 cycles per
-// 16 x 8 outputs and group, none of them more than half of the time; with few rows the unpacking of the weights, of which no
-// step is shared.  509 rows at 12288 x 4096: 1.08 ms = 24 T products/s (F32 multiply-adds that truncate, one product in half
-// an instruction and its sign in two more: 3.48 ms), 200 rows 0.52 (1.72), 8 rows 0.053 (0.229).
+// Up to some dozens of rows the products run on mma.sync, here; more rows on tcgen05.mma (qgmma_emulation_tcgen05.cu).
+// What bounds it: the unpacking of the weights, of which no step is shared beyond 16 rows, and the latencies of a group's
+// chain.  16 rows at 12288 x 4096: 78 us, 8 rows 53 (F32 multiply-adds that truncate, one product in half an instruction and
+// its sign in two more: 230).
 #include "common.cuh"
 #include "ops_internal.hpp"
+#include "qgmma_operands.cuh"
 
 namespace evob {
 namespace {
 
-constexpr int kGroup = 32;
+using namespace qgmma;
 
 // An E4M3 magnitude as F32: the code's seven bits are a float's exponent and
 // mantissa up to a factor of 2^120, which also normalises subnormal codes
@@ -91,34 +93,6 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const std::uint32_t (&a)[
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Eight codes of a line as tensor-core operands.  An E4M3 code's bits in the place of an F16 value's are the code's value
-// times 2^-8, subnormals and the code 0x7f (480) included.
-struct Operands {
-  std::uint32_t copies[8];  // the value, in both halves
-  std::uint32_t powers[4];  // BF16 pairs 2^(6 (e + 15) - 127), times 2^85 for weights; 0 for a zero
-};
-template <bool kWeights>
-__device__ __forceinline__ Operands operands_of(const uint2 codes) {
-  Operands r;
-#pragma unroll
-  for (int word = 0; word < 2; ++word) {
-    const std::uint32_t c = word == 0 ? codes.x : codes.y;
-    const std::uint32_t upper = (c & 0x80808080U) | ((c >> 1U) & 0x3f3f3f3fU), lower = (c << 7U) & 0x80808080U;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r.copies[4 * word + i] = __byte_perm(lower, upper, 0x4040U + 0x1111U * i);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const std::uint32_t pair = __byte_perm(lower, upper, 0x5140U + 0x2222U * i);
-      std::uint32_t normal, power;  // (every E4M3 value but 0 is a normal F16 number)
-      asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(normal) : "r"(pair), "r"(0x5c005c00U));  // 2^8
-      power = ((normal >> 3U) & 0x0f800f80U) * 6U;
-      if constexpr (kWeights) asm("mul.rn.bf16x2 %0, %0, %1;" : "+r"(power) : "r"(0x6a006a00U));  // 2^85
-      r.powers[2 * word + i] = power;
-    }
-  }
-  return r;
-}
-
 // 16 weight rows' group as mma.sync's A operands: row g, row g + 8, and for the products the same again.
 struct WeightTile {
   std::uint32_t copies[8][4], powers[2][4];
@@ -142,15 +116,6 @@ __device__ __forceinline__ WeightTile weight_tile_of(const uint2 upper, const ui
   }
   return t;
 }
-// 2^(E - 14) as F32 bits (E counts products; an accumulator's own exponent is in the same place) from the sum of the powers,
-// whose exponent field is 6 (E + 23) + 0 .. 5: floor(field / 6) + 90, the high word of bits * 2^32 / 6.  Without a product E
-// is -23: products' E is at least -18, so an accumulator is a multiple of 2^-31 and loses nothing to a unit of 2^-36.
-__device__ __forceinline__ std::uint32_t sixth_of(const std::uint32_t bits) {
-  std::uint32_t d;
-  asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(bits), "r"(0x2aaaaaabU), "r"(90U << 23U));
-  return d;
-}
-
 // A row's group in shared memory: lane c of a quad reads its eight K values as pairs of copies (two K values per 16-byte
 // word, 64 j + 16 c bytes in) and their powers.  Eight lanes of neighbouring rows meet different banks.
 struct __align__(16) RowGroup {
@@ -490,13 +455,15 @@ int e4m3_emulated_gemm(const void *input_codes, const void *weight_codes,
     return launch_tiled<decltype(shape)>(input_codes, weight_codes, rows, in_features, out_features, output_scale,
                                          output, stream);
   };
-  // A warp unpacks its weights for 8, 16 or 64 rows.  64 rows share the unpacking best (509 rows, 12288 x 4096: 1.08 ms against
-  // 1.27 with 16), unless they pad (200 rows: 0.60 against 0.52 ms) or leave SMs without two CTAs (64 rows at 12288 x 4096: 0.22
-  // against 0.19 ms, at 24576 x 8192, twice the CTAs, 0.61 against 0.69).
   if (rows <= 8) return tiled(EmulationShape<1, 4, 8, 4>{});
-  const std::size_t tall = (rows + 63) / 64 * 64, flat = (rows + 15) / 16 * 16;
-  if (tall * 100 <= flat * 110 && tall / 64 * ceil_div_u(out_features, 64) >= std::size_t{2} * 148)
-    return tiled(EmulationShape<8, 4, 1, 3>{});
+  // A group takes about 0.25 us + 1.65 us per 2^20 outputs here (16 rows per warp); with the rows in tiles of 64 on tcgen05.mma
+  // 1.4 us while every CTA has an SM of its own and 2.15 us per 296 CTAs beyond (12288 x 4096: 33 rows 135 and 164 us, 64 rows
+  // 195 and 164; 5760 x 1920: 128 rows 82 and 90 us, 509 rows 242 and 201).
+  const std::size_t flat = (rows + 15) / 16 * 16;
+  const std::size_t ctas = (rows + 63) / 64 * ((out_features + 127) / 128), pairs = (ctas + 295) / 296;
+  const double here = 0.25 + 1.65e-6 * static_cast<double>(flat) * static_cast<double>(out_features);
+  if ((ctas <= 148 ? 1.4 : 2.15 * static_cast<double>(pairs)) < here)
+    return e4m3_emulated_gemm_tcgen05(input_codes, weight_codes, rows, in_features, out_features, output_scale, output, stream);
   return tiled(EmulationShape<2, 4, 4, 4>{});
 }
 

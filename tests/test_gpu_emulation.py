@@ -49,7 +49,7 @@ def test_emulated_projection_at_kernel_edges(ops, oracle, rows, inner, columns, 
 @pytest.mark.parametrize("rows,inner,columns", [(2, 288, 65), (8, 32, 15), (9, 160, 17), (16, 96, 4736), (64, 96, 18944),
                                                (256, 64, 4737), (449, 32, 2433)])
 def test_emulated_projection_with_every_weight_code(ops, oracle, rows, inner, columns):
-    """Weights of all codes, in tiles of 8, 16 and 64 rows with remainders and groups that do not fill a stage.  The code
+    """Weights of all codes, in tiles of 8, 16 and 64 rows (these on tcgen05) with remainders and groups that do not fill a stage.  The code
     of a NaN counts as 480 (the oracle has none): it meets one value of 0.5 in its group."""
     rng = np.random.default_rng(rows + inner + columns)
     x = _codes(rng, "any", (rows, inner))
