@@ -1,7 +1,7 @@
 // Dense projections y = x . W^T on the 5th-generation tensor cores.
 //
 // Large projections (512 rows and 48 tiles of 256 x 256 or more) run on CTA pairs: gemm_tcgen05_pair_kernel, two
-// CTAs of a cluster on one 256 x 256 tile with tcgen05.mma.cta_group::2 (see there).  Everything else,
+// CTAs of a cluster on one 256 x 256 (or 192) tile with tcgen05.mma.cta_group::2 (see there).  Everything else,
 // and every shape when EVO_B200_GEMM_PAIR=0, runs on gemm_tcgen05_kernel:
 // one persistent CTA per SM walks 128 x BN output tiles.  Warp roles:
 //   warp 0   TMA producer: streams 128B-swizzled K-major tiles of x [M,K] and
@@ -492,18 +492,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
 }
 
 // ------------------------------------------------------- CTA pairs (cta_group::2)
-// The same projection with two CTAs of a cluster on one 256 x 256 output tile.  Each CTA loads its own
-// 128 rows of A and its own 128 of the tile's 256 weight rows (TMA without multicast; the copies report
-// to the leader's mbarrier), the leader issues tcgen05.mma.cta_group::2 (M = 256, N = 256), and each CTA
-// ends up with its 128 rows x 256 columns of the accumulator in its own tensor memory and stores them as
-// the one-CTA kernel does.  Per SM a stage is 32 KiB instead of 48 for the same arithmetic: a third
+// The same projection with two CTAs of a cluster on one output tile of 256 rows x kPairN columns (256, or 192 where that
+// fills the last wave better).  Each CTA loads its own 128 rows of A and its own half of the tile's weight rows (TMA without
+// multicast; the copies report to the leader's mbarrier), the leader issues tcgen05.mma.cta_group::2 (M = 256), and each CTA
+// ends up with its 128 rows of the accumulator in its own tensor memory and stores them as the one-CTA kernel does.  Per SM a stage is 32 KiB instead of 48 for the same arithmetic: a third
 // less traffic from L2, and six stages in flight instead of four.
-constexpr int kPairStages = 6;
-constexpr int kPairN = 256;
-
+template <int kPairN>
 struct PairLayout {
-  static constexpr int kABytes = kBlockM * kBlockKBytes;  // 128 rows of A
-  static constexpr int kBBytes = 128 * kBlockKBytes;       // this CTA's 128 weight rows of the tile
+  static constexpr int kPairStages = kPairN == 256 ? 6 : 7;
+  static constexpr int kABytes = kBlockM * kBlockKBytes;          // 128 rows of A
+  static constexpr int kBBytes = kPairN / 2 * kBlockKBytes;       // this CTA's half of the tile's weight rows
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kBarrierOffset = kPairStages * kStageBytes;
   // full[kPairStages], empty[kPairStages], tmem_full[2], tmem_empty[2]
@@ -566,7 +564,7 @@ __device__ __forceinline__ void tc_commit_pair(const std::uint32_t bar) {
       : "memory");
 }
 
-template <bool kFp8>
+template <bool kFp8, int kPairN>
 __host__ __device__ constexpr std::uint32_t pair_instruction_descriptor() {
   std::uint32_t d = 0;
   d |= 1U << 4U;                          // accumulator F32
@@ -577,12 +575,13 @@ __host__ __device__ constexpr std::uint32_t pair_instruction_descriptor() {
   return d;
 }
 
-template <bool kFp8>
+template <bool kFp8, int kPairN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const EpilogueParams ep, const int M, const int N, const int K_bytes,
                          int *const error_word) {
-  using L = PairLayout;
+  using L = PairLayout<kPairN>;
+  constexpr int kPairStages = L::kPairStages;
   extern __shared__ unsigned char smem_raw[];
   unsigned char *const smem = smem_raw + ((1024U - (smem_u32(smem_raw) & 1023U)) & 1023U);
   const std::uint32_t smem_base = smem_u32(smem);
@@ -595,7 +594,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   volatile int *const abort_flag = reinterpret_cast<volatile int *>(smem + L::kAbortOffset);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const std::uint32_t rank = cluster_rank();  // 0: the leader (issues the MMAs, owns the full barriers)
-  constexpr std::uint32_t kTmemColumns = 2 * kPairN;
+  constexpr std::uint32_t kTmemColumns = 512, kBuffer = 256;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPairStages; ++s) {
@@ -641,7 +640,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         int tile_m, tile_n;
         tile_coordinates(tile % tiles_mn, tiles_m, tiles_n, &tile_m, &tile_n);
         const int m0 = tile_m * 256 + static_cast<int>(rank) * 128;
-        const int n0 = tile_n * kPairN + static_cast<int>(rank) * 128 +
+        const int n0 = tile_n * kPairN + static_cast<int>(rank) * (kPairN / 2) +
                        (ep.tile_group != nullptr ? __ldg(ep.tile_group + tile_m) * N : 0);
         const int kb_begin = (tile / tiles_mn) * k_per_split;
         for (int kb = kb_begin; kb < kb_begin + k_per_split; ++kb) {
@@ -667,7 +666,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
-      constexpr std::uint32_t idesc = pair_instruction_descriptor<kFp8>();
+      constexpr std::uint32_t idesc = pair_instruction_descriptor<kFp8, kPairN>();
       int stage = 0;
       std::uint32_t phase = 0;
       int local = 0;
@@ -677,7 +676,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         const std::uint32_t acc_phase = (local >> 1) & 1U;
         if (!mbar_wait(tmem_empty_bar(acc), acc_phase ^ 1U, abort_flag)) break;
         tc_fence_after();
-        const std::uint32_t tmem_d = tmem_base + acc * kPairN;
+        const std::uint32_t tmem_d = tmem_base + acc * kBuffer;
         for (int kb = 0; kb < k_per_split; ++kb) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
             ok = false;
@@ -712,8 +711,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const std::uint32_t acc_phase = (local >> 1) & 1U;
       if (!mbar_wait(tmem_full_bar(acc), acc_phase, abort_flag)) break;
       tc_fence_after();
-      epilogue_tile<kPairN>(ep, M, N, m0, n0, split, tmem_base + acc * kPairN, quarter, lane,
-                            reinterpret_cast<float *>(smem + PairLayout::kStagingOffset + quarter * kStagingBytes));
+      epilogue_tile<kPairN>(ep, M, N, m0, n0, split, tmem_base + acc * kBuffer, quarter, lane,
+                            reinterpret_cast<float *>(smem + L::kStagingOffset + quarter * kStagingBytes));
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -1136,8 +1135,8 @@ int launch_tc(const void *a, const void *b, const EpilogueParams &ep,
   return check_launch("tcgen05 GEMM kernel");
 }
 
-template <bool kFp8>
-int launch_tc_pair(const void *a, const void *b, const EpilogueParams &ep, const std::size_t M, const std::size_t N,
+template <bool kFp8, int kPairN>
+int launch_tc_pair_as(const void *a, const void *b, const EpilogueParams &ep, const std::size_t M, const std::size_t N,
                    const std::size_t K, cudaStream_t stream, const std::size_t groups = 1) {
   const std::size_t weight_k = ep.weight_wrap_blocks > 0 ? static_cast<std::size_t>(ep.weight_wrap_blocks) * 64 : K;
   int status = kOk;
@@ -1146,24 +1145,43 @@ int launch_tc_pair(const void *a, const void *b, const EpilogueParams &ep, const
   CUtensorMap map_a, map_b;
   status = make_map(&map_a, a, kFp8, M, K, kBlockM);
   if (status != kOk) return status;
-  status = make_map(&map_b, b, kFp8, N * groups, weight_k, 128);  // a CTA loads its 128 of the tile's 256 weight rows
+  status = make_map(&map_b, b, kFp8, N * groups, weight_k, kPairN / 2);  // a CTA loads its half of the tile's weight rows
   if (status != kOk) return status;
   static bool configured[64] = {};
   int device = 0;
   cudaGetDevice(&device);
   if (!configured[device]) {
-    if (cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<kFp8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             PairLayout::kTotal) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<kFp8, kPairN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             PairLayout<kPairN>::kTotal) != cudaSuccess)
       return fail(kCuda, "cannot raise the GEMM shared-memory limit");
     configured[device] = true;
   }
   const std::size_t tiles =
       ((M + 255) / 256) * ((N + kPairN - 1) / kPairN) * static_cast<std::size_t>(ep.split_k > 1 ? ep.split_k : 1);
   const std::size_t pairs = std::min<std::size_t>(tiles, static_cast<std::size_t>(state->sm_count) / 2);
-  gemm_tcgen05_pair_kernel<kFp8><<<static_cast<unsigned int>(2 * pairs), kGemmThreads, PairLayout::kTotal, stream>>>(
+  gemm_tcgen05_pair_kernel<kFp8, kPairN><<<static_cast<unsigned int>(2 * pairs), kGemmThreads, PairLayout<kPairN>::kTotal, stream>>>(
       map_a, map_b, ep, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K * (kFp8 ? 1 : 2)),
       state->error_word);
   return check_launch("tcgen05 GEMM kernel (CTA pairs)");
+}
+
+template <bool kFp8>
+int launch_tc_pair(const void *a, const void *b, const EpilogueParams &ep, const std::size_t M, const std::size_t N,
+                   const std::size_t K, cudaStream_t stream, const std::size_t groups = 1) {
+  // Tiles of 192 columns where they take no more waves of pairs than tiles of 256: 2999 x 2048 outputs are 96 wide tiles or
+  // 132 narrow ones on 74 pairs, two waves either way (K = 512: 33.6 and 27.4 us, 768: 35.4 and 29.4, 2048: 33.6 and 32.8;
+  // 3001 x 1920 at K = 1920 42 and 36, at 5120 71 and 67).  One wave more costs more than the width saves (8192 x 2048, four
+  // and five: K = 2048 64 and 70 us, 8448 224 and 266).  A gate pairs 128-column halves, and groups keep their tiles.
+  if (ep.gate_mode == 0 && ep.tile_group == nullptr) {
+    int status = kOk, sm_count = 0;
+    if (tc::error_word(&status, &sm_count) == nullptr) return status;
+    const auto waves = [&](const std::size_t columns) {
+      const std::size_t pairs = static_cast<std::size_t>(sm_count) / 2;
+      return ((M + 255) / 256 * ((N + columns - 1) / columns) + pairs - 1) / pairs;
+    };
+    if (waves(192) <= waves(256)) return launch_tc_pair_as<kFp8, 192>(a, b, ep, M, N, K, stream, groups);
+  }
+  return launch_tc_pair_as<kFp8, 256>(a, b, ep, M, N, K, stream, groups);
 }
 
 template <bool kFp8, int BT>

@@ -104,6 +104,37 @@ def test_pair_kernel_epilogues_at_ragged_sizes(ops):
     assert bool((error <= 0.03 + 0.02 * reference.abs()).all()), float(error.max())
 
 
+@pytest.mark.parametrize("rows,inner,columns", [(520, 72, 4000), (520, 1920, 4225), (769, 520, 3073), (2999, 264, 2050), (1500, 128, 1920)])
+def test_pair_tiles_of_192_columns(ops, rows, inner, columns):
+    """Sizes whose narrow tiles take no more waves than the wide ones, with remainders in every direction: BF16 results with
+    bias and residual, F32 results stored and added, E4M3 operands.  The products are exact, sums of `inner` of them rounded
+    to F32 (at most inner + 4 times 2^-24 of the magnitudes' sum), and once or twice to BF16 (2^-8 of the result, or of 4)."""
+    torch.manual_seed(rows + inner)
+    x = torch.randn(rows, inner, device="cuda").bfloat16()
+    w = (torch.randn(columns, inner, device="cuda") * 0.05).bfloat16()
+    bias, residual = torch.randn(columns, device="cuda").bfloat16(), torch.randn(rows, columns, device="cuda").bfloat16()
+    exact, spread = x.double() @ w.double().T, (inner + 4) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    out = _linear(ops, x, w, bias, residual, 1, 0).view(torch.bfloat16)
+    first = exact + bias.double()
+    error = (out.double() - (first + residual.double())).abs()
+    assert bool((error <= spread + 2.0 ** -8 * (first.abs() + (first + residual.double()).abs() + 0.01)).all())
+    base = torch.randn(rows, columns, device="cuda")
+    for accumulate in (0, 1):
+        sums = base.clone()
+        ops.call("bf16_linear_f32_result", p(x), p(w), rows, inner, columns, accumulate, None, 0, p(sums), stream())
+        ops.call("check_async_errors", stream())
+        assert bool(((sums.double() - exact - accumulate * base.double()).abs() <= spread + 2.0 ** -23 * (exact.abs() + base.double().abs())).all())
+    if inner % 16 == 0:
+        codes = (torch.randn(columns, inner, device="cuda") * 0.5).to(torch.float8_e4m3fn)
+        scratch, out = torch.empty(rows * inner, dtype=torch.uint8, device="cuda"), empty_bits(rows, columns)
+        ops.call("e4m3_tensorcore_linear", p(x), p(codes), rows, inner, columns, 4.0, 0.25, p(scratch), p(out), stream())
+        ops.call("check_async_errors", stream())
+        rounded = (x.float() * 4.0).clamp(-448, 448).to(torch.float8_e4m3fn).double()
+        exact = rounded @ codes.double().T * 0.25
+        spread = (inner + 4) * 2.0 ** -24 * 0.25 * (rounded.abs() @ codes.double().abs().T)
+        assert bool(((out.view(torch.bfloat16).double() - exact).abs() <= spread + 2.0 ** -8 * exact.abs()).all())
+
+
 def test_gated_up_projection_matches_two_linears_and_gate(ops, oracle):
     rng = np.random.default_rng(11)
     rows, inner, hidden = 150, 256, 384
