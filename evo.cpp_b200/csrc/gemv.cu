@@ -85,16 +85,32 @@ __device__ __forceinline__ bf16 gelu_round_small(const float x) {
   }
 }
 
-// Result `column` of row r (of `out_index` where rows are grouped) from its sum, or from the sums of a gated pair.
+// What a result is added to.  A stream reads it beside x, so that the trip to memory does not follow the sums.
+struct Addends {
+  float first = 0.0F, second = 0.0F;  // F32: the old result and the bias; BF16: the residual and the bias
+};
+__device__ __forceinline__ Addends addends_of(const GemvParams &p, const int r, const std::size_t out_index, const int out_columns,
+                                              const int column) {
+  Addends a;
+  if (p.out_f32 != nullptr) {
+    if (p.accumulate_f32 != 0) a.first = p.out_f32[out_index * out_columns + column];
+    if (p.bias_f32 != nullptr) a.second = p.bias_f32[column];
+  } else if (p.gate_mode == 0) {
+    if (p.residual != nullptr) a.first = bf2f(p.residual[static_cast<std::size_t>(r) * out_columns + column]);
+    if (p.bias_mode != 0) a.second = bf2f(p.bias[column]);
+  }
+  return a;
+}
+
+// Result `column` of row `out_index` from its sum, or from the sums of a gated pair.
 template <class Total>
-__device__ __forceinline__ void finish_column(const GemvParams &p, const int r, const std::size_t out_index,
-                                              const int out_columns, const int column, const float alpha, const int local,
+__device__ __forceinline__ void finish_column(const GemvParams &p, const std::size_t out_index, const int out_columns,
+                                              const int column, const float alpha, const int local, const Addends &addends,
                                               const Total &total) {
   if (p.out_f32 != nullptr) {
-    float *const slot = p.out_f32 + out_index * out_columns + column;
     float value = total(local) * alpha;
-    if (p.bias_f32 != nullptr) value += p.bias_f32[column];
-    *slot = soft_cap(p.accumulate_f32 != 0 ? *slot + value : value, p.softcap);
+    if (p.bias_f32 != nullptr) value += addends.second;
+    p.out_f32[out_index * out_columns + column] = soft_cap(p.accumulate_f32 != 0 ? addends.first + value : value, p.softcap);
     return;
   }
   bf16 *const out_row = p.out + out_index * out_columns;
@@ -112,11 +128,10 @@ __device__ __forceinline__ void finish_column(const GemvParams &p, const int r, 
     out_row[column] = f2bf(activated * second);
   } else {
     float value = total(local) * alpha;
-    if (p.bias_mode == 1) value += bf2f(p.bias[column]);
+    if (p.bias_mode == 1) value += addends.second;
     value = rbf(value);
-    if (p.bias_mode == 2) value = rbf(value + bf2f(p.bias[column]));
-    if (p.residual != nullptr)
-      value = rbf(value + bf2f(p.residual[static_cast<std::size_t>(r) * out_columns + column]));
+    if (p.bias_mode == 2) value = rbf(value + addends.second);
+    if (p.residual != nullptr) value = rbf(value + addends.first);
     out_row[column] = f2bf(value);
   }
 }
@@ -219,7 +234,7 @@ gemv_kernel(const GemvParams p) {
   if (r >= p.rows || column >= out_columns) return;
   const std::size_t out_index = grouped ? blockIdx.y : r;
   const float alpha = grouped && p.row_scale != nullptr ? p.alpha * p.row_scale[out_index] : p.alpha;
-  finish_column(p, r, out_index, out_columns, column, alpha, local, [&](const int c) {
+  finish_column(p, out_index, out_columns, column, alpha, local, addends_of(p, r, out_index, out_columns, column), [&](const int c) {
     float sum = 0.0F;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) sum += partial[w][c][r];
@@ -238,7 +253,8 @@ gemv_kernel(const GemvParams p) {
 // and a stream is as slow as its fullest SM.
 // Grouped rows (blockIdx.y) take their weights' rows the same way, once they know their group.
 // Bound: HBM, and in a step the way from one kernel's end to the next one's first data.  48 decode steps of Gigusun:
-// 12.3 ms, 12.8 with two CTAs of one team each that pack; of Kikepel 11.4 and 11.9.
+// 12.3 ms, 12.8 with two CTAs of one team each that pack; of Kikepel 11.4 and 11.9.  A trip to memory that nothing hides is
+// 0.3 us of a kernel: old results and gains read beside x instead of where they are used take Gigusun's steps to 12.07 ms.
 constexpr int kTeams = 2, kRingBytes = 48 * 1024;
 constexpr int kStreamShared = 116 * 1024;  // more than half of an SM's
 constexpr int kTeamShared = kStreamShared / kTeams;
@@ -337,10 +353,20 @@ gemv_stream_kernel(const GemvParams p) {
     release_dependents();
     wait_for_producers(x);
   }
-  float xv[kChunks][kPer];
+  constexpr bool kEarlyAddends = kChunks * kPer <= 64;
+  Addends early;
+  if (kEarlyAddends && tid < columns) early = addends_of(p, 0, blockIdx.y, out_columns, column0 + tid);
+  // what a front multiplies with is on its way beside x as well, where there are registers for it
+  constexpr bool kEarlyGain = kFront == Front::kRms && kChunks <= 2;
+  float xv[kChunks][kPer], gain[kEarlyGain ? kChunks : 1][8], factors[4];
+  if constexpr (kFront == Front::kPoly) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) factors[i] = p.front[i];
+  }
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     if (piece0 + 32 * c < piece_end) {
+      if constexpr (kEarlyGain) load_floats<8>(p.front + static_cast<std::size_t>(piece0 + 32 * c) * 8, gain[c]);
       const Source *const source = x + static_cast<std::size_t>(piece0 + 32 * c) * kPer;
       if constexpr (std::is_same_v<Source, float>) load_floats<8>(source, xv[c]);
       else unpack16<kFp8>(*reinterpret_cast<const uint4 *>(source), xv[c]);
@@ -387,14 +413,14 @@ gemv_stream_kernel(const GemvParams p) {
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
         if (piece0 + 32 * c < piece_end) {
-          float gain[8];
-          load_floats<8>(p.front + static_cast<std::size_t>(piece0 + 32 * c) * 8, gain);
+          const int at = kEarlyGain ? c : 0;
+          if constexpr (!kEarlyGain) load_floats<8>(p.front + static_cast<std::size_t>(piece0 + 32 * c) * 8, gain[0]);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) xv[c][i] = rounded(xv[c][i] * factor * gain[i]);
+          for (int i = 0; i < 8; ++i) xv[c][i] = rounded(xv[c][i] * factor * gain[at][i]);
         }
     } else {
-      const float a = p.front[0] * rsqrtf(sums[0]), b = p.front[1] * rsqrtf(sums[1]), c3 = p.front[2] * rsqrtf(sums[2]);
-      const float e = p.front[3];
+      const float a = factors[0] * rsqrtf(sums[0]), b = factors[1] * rsqrtf(sums[1]), c3 = factors[2] * rsqrtf(sums[2]);
+      const float e = factors[3];
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
         if (piece0 + 32 * c < piece_end) {
@@ -457,7 +483,8 @@ gemv_stream_kernel(const GemvParams p) {
   team_barrier();
   const float alpha = p.row_scale != nullptr ? p.alpha * p.row_scale[blockIdx.y] : p.alpha;
   for (int local = tid; local < columns; local += kThreads)
-    finish_column(p, 0, blockIdx.y, out_columns, column0 + local, alpha, local,
+    finish_column(p, blockIdx.y, out_columns, column0 + local, alpha, local,
+                  kEarlyAddends && local == tid ? early : addends_of(p, 0, blockIdx.y, out_columns, column0 + local),
                   [&](const int index) {  // (of a gated pair: 2 local, 2 local + 1)
                     const int row = gated ? (index & 1) * columns + index / 2 : index;
                     const float4 a = reinterpret_cast<const float4 *>(partial)[2 * row],
