@@ -817,11 +817,12 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       int stage = 0;
       std::uint32_t phase = 0;
       const auto k_of = [&](const int kb) { return kFp8 ? kb * kBlockKBytes : kb * (kBlockKBytes / 2); };
+      const std::uint64_t once = policy_read_once();  // (the weights; tokens and partial sums are read again)
       // the first weights do not depend on the kernel that writes the tokens
       const int early = k_per_split < L::kStages ? k_per_split : L::kStages;
       for (int s = 0; s < early; ++s) {
         mbar_expect_tx(full_bar(s), L::kStageBytes);
-        tma_load_2d(smem_base + s * L::kStageBytes, &map_w, full_bar(s), k_of(kb_begin + s), n0);
+        tma_load_2d(smem_base + s * L::kStageBytes, &map_w, full_bar(s), k_of(kb_begin + s), n0, once);
       }
       wait_for_producers();
       for (int kb = kb_begin; kb < kb_begin + k_per_split; ++kb) {
@@ -829,7 +830,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         if (kb - kb_begin >= early) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1U, abort_flag)) break;
           mbar_expect_tx(full_bar(stage), L::kStageBytes);
-          tma_load_2d(w_dst, &map_w, full_bar(stage), k_of(kb), n0);
+          tma_load_2d(w_dst, &map_w, full_bar(stage), k_of(kb), n0, once);
         }
         tma_load_2d(w_dst + L::kWBytes, &map_x, full_bar(stage), k_of(kb), 0);
         if (++stage == L::kStages) {

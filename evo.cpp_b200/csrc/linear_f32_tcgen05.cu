@@ -122,11 +122,15 @@ linear_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const T *__
 
   if (warp == kProducerWarp) {
     if (lane == 0) {
+      const std::uint64_t once = policy_read_once();
       for (int block = first; block < last; ++block) {
         const int i = block - first, stage = i % L::kStages;
         if (i >= L::kStages && !mbar_wait(empty(stage), (i / L::kStages - 1) & 1, abort_flag)) break;
         mbar_expect_tx(w_full(stage), L::kWBytes);
-        tma_load_2d(smem_base + stage * L::kStageBytes, &map_w, w_full(stage), block * kBlockK, group * p.out_features + n0);
+        const std::uint32_t w_dst = smem_base + stage * L::kStageBytes;
+        const int weight_row = group * p.out_features + n0;
+        if (gridDim.y == 1) tma_load_2d(w_dst, &map_w, w_full(stage), block * kBlockK, weight_row, once);
+        else tma_load_2d(w_dst, &map_w, w_full(stage), block * kBlockK, weight_row);
       }
     }
   } else if (warp == kMmaWarp) {

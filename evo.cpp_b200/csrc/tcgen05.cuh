@@ -74,6 +74,21 @@ __device__ __forceinline__ void tma_load_2d(const std::uint32_t dst,
       "l"(map), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// The same with an L2 policy.
+__device__ __forceinline__ void tma_load_2d(const std::uint32_t dst, const CUtensorMap *const map, const std::uint32_t bar,
+                                            const int x, const int y, const std::uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%3, %4}], [%2], %5;" ::"r"(dst),
+      "l"(map), "r"(bar), "r"(x), "r"(y), "l"(policy)
+      : "memory");
+}
+// What is read once and the first to leave L2.
+__device__ __forceinline__ std::uint64_t policy_read_once() {
+  std::uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  return policy;
+}
 __device__ __forceinline__ void tma_load_3d(const std::uint32_t dst,
                                             const CUtensorMap *const map,
                                             const std::uint32_t bar,
