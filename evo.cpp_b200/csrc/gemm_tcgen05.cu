@@ -1087,11 +1087,22 @@ DeviceState *device_state(int *status) {
   std::lock_guard<std::mutex> lock(mutex);
   DeviceState &state = states[device];
   if (state.error_word == nullptr) {
-    if (cudaMalloc(&state.error_word, sizeof(int)) != cudaSuccess ||
-        cudaMemset(state.error_word, 0, sizeof(int)) != cudaSuccess) {
+    // (the first call may be one that the caller captures: neither the allocation nor the clearing belongs to the capture)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaStream_t own = nullptr;
+    const bool exchanged = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    int *word = nullptr;
+    const bool ready = cudaMalloc(&word, sizeof(int)) == cudaSuccess &&
+                       cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess &&
+                       cudaMemsetAsync(word, 0, sizeof(int), own) == cudaSuccess && cudaStreamSynchronize(own) == cudaSuccess;
+    if (own != nullptr) cudaStreamDestroy(own);
+    if (exchanged) cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ready) {
+      if (word != nullptr) cudaFree(word);
       *status = fail(kCuda, "cannot allocate the GEMM error word");
       return nullptr;
     }
+    state.error_word = word;
     cudaDeviceGetAttribute(&state.sm_count, cudaDevAttrMultiProcessorCount,
                            device);
     if (state.sm_count <= 0) state.sm_count = kSmCount;

@@ -493,3 +493,30 @@ def test_extreme_gates_stay_finite(pkg, ops):
         out = case.run(40).double().cpu().numpy()
         assert np.isfinite(out).all() and np.isfinite(expected).all()
         assert_near(out, expected, 1, factor=50.0)
+
+
+CAPTURED_FIRST = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import conftest, torch
+ops = conftest.load_package().ops()
+x, w, out = torch.randn(40, 64, device="cuda"), torch.randn(96, 64, device="cuda").bfloat16(), torch.zeros(40, 96, device="cuda")
+torch.cuda.synchronize()
+graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+with torch.cuda.graph(graph, stream=side):
+    ops.call("f32_linear", x.data_ptr(), w.data_ptr(), 40, 64, 96, 0, out.data_ptr(), side.cuda_stream)
+graph.replay()
+torch.cuda.synchronize()
+exact = x.double() @ w.double().T
+assert float((out - exact).abs().max()) <= 32 * 2.0 ** -24 * float((x.double().abs() @ w.double().abs().T).max())
+"""
+
+
+def test_first_product_of_a_process_can_be_captured():
+    """The per-device error word is made by the first kernel that needs it, also while the caller captures that launch."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    run = subprocess.run([sys.executable, "-c", CAPTURED_FIRST, str(Path(__file__).parent)], capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
