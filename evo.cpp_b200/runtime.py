@@ -6,6 +6,7 @@ CPU-baseline legs of the benchmark, upstream's own CPU build of the same ABI
 """
 from __future__ import annotations
 
+import array
 import ctypes
 from pathlib import Path
 
@@ -338,6 +339,17 @@ class Scheduler:
             self.handle = None
 
 
+def token_words(tokens):
+    """Token ids as a ctypes array of 32-bit words.  A list of plain integers in their range goes through array.array, which
+    takes less than half of the time; every other case is left to ctypes, with its conversions and errors."""
+    if type(tokens) is list and set(map(type, tokens)) == {int}:
+        try:
+            return (ctypes.c_uint32 * len(tokens)).from_buffer(array.array("I", tokens))
+        except OverflowError:  # ctypes takes such an id modulo 2^32
+            pass
+    return (ctypes.c_uint32 * len(tokens))(*tokens)
+
+
 class Context:
     def __init__(self, library: EvoLibrary, handle, vocab: int, width: int):
         self.library, self.handle, self.vocab, self.width = library, handle, vocab, width
@@ -394,13 +406,13 @@ class Context:
 
     def prefill_tokens(self, tokens, mode: int = 0) -> np.ndarray:
         """evo_b200_context_prefill_tokens: token ids, one of the PREFILL_* forms; F32 logits [tokens, vocab]."""
-        ids = (ctypes.c_uint32 * len(tokens))(*tokens)
+        ids = token_words(tokens)
         return self._collect(lambda cb: self.library.lib.evo_b200_context_prefill_tokens(
             self.handle, ids, len(tokens), mode, cb, None), self.vocab)
 
     def embed_tokens(self, tokens, layer: int, first_chunk: bool = True) -> np.ndarray:
         """evo_b200_context_embed_tokens: block output of `layer` for one chunk of token ids, F32 [tokens, width]."""
-        ids = (ctypes.c_uint32 * len(tokens))(*tokens)
+        ids = token_words(tokens)
         return self._collect(lambda cb: self.library.lib.evo_b200_context_embed_tokens(
             self.handle, ids, len(tokens), layer, int(first_chunk), cb, None), self.width)
 

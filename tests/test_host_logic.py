@@ -648,3 +648,17 @@ def test_pool_of_pinned_results(tmp_path):
                     str(csrc / "runtime" / "host_pool.cpp"), "-o", str(program)], check=True)
     done = subprocess.run([str(program)], capture_output=True, text=True)
     assert done.returncode == 0 and done.stdout.strip() == "ok", done.stdout + done.stderr
+
+
+def test_token_ids_convert_as_ctypes_converts_them(rt):
+    """Plain lists take another way to the same words; what ctypes refuses stays refused."""
+    for tokens in ([], [0], [5, 4294967295, 17], [-1, 3], [1 << 32, 2], [True, 7], (1, 2, 3), np.array([3, 9], np.int64).tolist(), range(5)):
+        assert list(rt.token_words(tokens)) == list((ctypes.c_uint32 * len(tokens))(*tokens))
+    for tokens in ([1.0], ["7"], [None, 1], [np.int64(3)], [2, np.uint32(3)]):
+        try:
+            expected = list((ctypes.c_uint32 * len(tokens))(*tokens))
+        except Exception as error:  # noqa: BLE001
+            with pytest.raises(type(error)):
+                rt.token_words(tokens)
+        else:
+            assert list(rt.token_words(tokens)) == expected
