@@ -409,13 +409,23 @@ rms_norm_few_rows_kernel(const bf16 *__restrict__ input, const float *__restrict
   }
   __syncthreads();
   const float denominator = partial[0];
+  const auto finish = [&](const auto &quotient) {
 #pragma unroll
-  for (int k = 0; k < kPerThread; ++k) {
-    const std::size_t column = threadIdx.x + k * kThreads;
-    if (!kWhole && column >= static_cast<std::size_t>(width)) break;
-    const bf16 result = f2bf(rbf(__fdiv_rn(bits2f_bf16(raw[k]), denominator)) * rbf(gain[k]));
-    if (output != nullptr) output[row * width + column] = result;
-    if (codes != nullptr) codes[row * width + column] = e4m3_code(bf2f(result) * quant_scale);
+    for (int k = 0; k < kPerThread; ++k) {
+      const std::size_t column = threadIdx.x + k * kThreads;
+      if (!kWhole && column >= static_cast<std::size_t>(width)) break;
+      const bf16 result = f2bf(rbf(quotient(bits2f_bf16(raw[k]))) * rbf(gain[k]));
+      if (output != nullptr) output[row * width + column] = result;
+      if (codes != nullptr) codes[row * width + column] = e4m3_code(bf2f(result) * quant_scale);
+    }
+  };
+  // As in store_normalized_row: the same quotient after its rounding.  Bound by latencies, of which a division is one per column:
+  // 16 tokens through a 4096-wide model 0.550 -> 0.546 ms, three steps of a 1920-wide one 1.352 -> 1.333 with the prompt.
+  if (denominator >= 1e-30F && denominator <= 1e30F) {
+    const float reciprocal = __frcp_rn(denominator);
+    finish([&](const float value) { return value * reciprocal; });
+  } else {
+    finish([&](const float value) { return __fdiv_rn(value, denominator); });
   }
 }
 

@@ -131,6 +131,22 @@ def test_rms_norm_and_fused_codes(ops, oracle):
         assert np.array_equal(codes.cpu().numpy(), expected_codes)
 
 
+@pytest.mark.parametrize("epsilon, scale", [(1e-32, 1e-25), (1e31, 1.0), (3e-30, 1e-26), (0.5e30, 4.0)])
+@pytest.mark.parametrize("rows, width", [(2, 512), (3, 300)])
+def test_few_normalised_rows_with_denominators_at_the_ends(ops, rows, width, epsilon, scale):
+    """Denominators on either side of the range in which a row is multiplied by a reciprocal.  Squares that vanish or are nothing
+    beside epsilon leave BF16(epsilon) as the denominator: every bit is known."""
+    rng = np.random.default_rng(width)
+    x_bits = rand_bf16(rng, rows, width, scale=scale)
+    gain = (1 + 0.1 * rng.standard_normal(width)).astype(np.float32)
+    out = empty_bits(rows, width)
+    ops.call("bf16_rms_norm", p(dev_bits(x_bits)), p(dev(gain)), rows, width, epsilon, p(out), None, 1.0, stream())
+    denominator = bf16_to_f32(f32_to_bf16(np.float32([epsilon])))[0]
+    quotient = bf16_to_f32(f32_to_bf16(bf16_to_f32(x_bits) / denominator))
+    expected = f32_to_bf16(quotient * bf16_to_f32(f32_to_bf16(gain)))
+    assert np.array_equal(host_bits(out).reshape(rows, width), expected.reshape(rows, width))
+
+
 def test_pointwise_bit_exact(ops, oracle):
     rng = np.random.default_rng(5)
     n = 8 * 1000 + 5
