@@ -495,6 +495,18 @@ def test_extreme_gates_stay_finite(pkg, ops):
         assert_near(out, expected, 1, factor=50.0)
 
 
+@TYPES
+def test_steps_with_keys_and_queries_of_infinite_length(pkg, ops, float32):
+    """Squares that overflow give zero vectors: nothing is read from the state or written to it, and nothing is NaN.  A product
+    of the vectors that is summed before they are scaled is infinite here."""
+    case = Recurrence(pkg, ops, delta=True, rows=3, heads=4, kv_heads=2, dim=40, vdim=24, float32=float32, seed=11)
+    case.conv[:] = np.abs(case.conv) + 0.1
+    case.device[0].copy_(cuda(case.conv))
+    case.projection[:, :case.value_column] = case.projection[:, :case.value_column].abs() * 1e20 + 1e20
+    for _ in range(3):
+        assert bool((case.run(1) == 0).all()) and bool((case.state == 0).all())
+
+
 CAPTURED_FIRST = """
 import sys
 sys.path.insert(0, sys.argv[1])
