@@ -125,12 +125,12 @@ qgmma_emulation_tcgen05_kernel(const std::uint8_t *__restrict__ input_codes, con
   const int groups = static_cast<int>(in_features / kGroup);
 
   // codes of a group: half of the thread's weight row, and eight codes of a row (row tid / 4, codes 8 (tid % 4) ..)
-  const bool has_row = tid < kRows * 4;
+  static_assert(kEmulationThreads == kRows * 4, "a thread per eight codes of the rows' group");
   const int x_row = tid / 4, x_part = tid % 4;
   uint2 w_codes[2], x_codes;
   const std::uint8_t *const w_at = weight_codes + (column < out_features ? column : out_features - 1) * in_features + 16 * half;
   const std::uint8_t *const x_at = input_codes + (row0 + x_row) * in_features + 8 * x_part;
-  const bool x_live = has_row && row0 + x_row < rows;
+  const bool x_live = row0 + x_row < rows;
   const auto fetch = [&](const int group) {
     const std::size_t k = static_cast<std::size_t>(min(group, groups - 1)) * kGroup;
 #pragma unroll
@@ -150,17 +150,15 @@ qgmma_emulation_tcgen05_kernel(const std::uint8_t *__restrict__ input_codes, con
       for (int j = 0; j < 4; ++j) w_powers[4 * i + j] = o.powers[j];
     }
     tmem_store_8(lane_base + L::kWeightPowers + group % 2 * 16 + half * 8, w_powers);
-    if (has_row) {
-      const Operands o = operands_of<false>(x_codes);
-      *reinterpret_cast<uint4 *>(smem + L::kPowerOffset + group % 2 * L::kAtomBytes + x_row * 128 + ((x_part ^ (x_row & 7)) << 4)) =
-          make_uint4(o.powers[0], o.powers[1], o.powers[2], o.powers[3]);
-      unsigned char *const at = smem + (group % 3 * 2 + x_part / 2) * L::kAtomBytes + x_row * 128;
+    const Operands o = operands_of<false>(x_codes);
+    *reinterpret_cast<uint4 *>(smem + L::kPowerOffset + group % 2 * L::kAtomBytes + x_row * 128 + ((x_part ^ (x_row & 7)) << 4)) =
+        make_uint4(o.powers[0], o.powers[1], o.powers[2], o.powers[3]);
+    unsigned char *const at = smem + (group % 3 * 2 + x_part / 2) * L::kAtomBytes + x_row * 128;
 #pragma unroll
-      for (int chunk = 0; chunk < 4; ++chunk) {
-        const int c = chunk / 2 * 4;
-        *reinterpret_cast<uint4 *>(at + (((x_part % 2 * 4 + chunk) ^ (x_row & 7)) << 4)) =
-            make_uint4(o.copies[c], o.copies[c + 1], o.copies[c + 2], o.copies[c + 3]);
-      }
+    for (int chunk = 0; chunk < 4; ++chunk) {
+      const int c = chunk / 2 * 4;
+      *reinterpret_cast<uint4 *>(at + (((x_part % 2 * 4 + chunk) ^ (x_row & 7)) << 4)) =
+          make_uint4(o.copies[c], o.copies[c + 1], o.copies[c + 2], o.copies[c + 3]);
     }
   };
   // 16 places of a product: four K values' copies (two in a word), then the same again
@@ -219,8 +217,10 @@ qgmma_emulation_tcgen05_kernel(const std::uint8_t *__restrict__ input_codes, con
       if (group + 1 < groups) issue_powers(group + 1);
       commit_from_warp(bar);
     }
-    unpack(group + 2, values);  // (behind the last groups: unused)
-    fetch(group + 3);
+    if (group + 2 < groups) {
+      unpack(group + 2, values);
+      fetch(group + 3);
+    }
     return true;
   };
 
@@ -262,6 +262,8 @@ qgmma_emulation_tcgen05_kernel(const std::uint8_t *__restrict__ input_codes, con
       }
     }
   }
+  // no store to TMEM is on its way when its columns change hands (a turn that gave up leaves some behind)
+  tmem_store_wait();
   tc_fence_before();
   __syncthreads();
   if (!ok) {  // products may still be on their way

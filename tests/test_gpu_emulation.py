@@ -49,8 +49,8 @@ def test_emulated_projection_at_kernel_edges(ops, oracle, rows, inner, columns, 
 @pytest.mark.parametrize("rows,inner,columns", [(2, 288, 65), (8, 32, 15), (9, 160, 17), (16, 96, 4736), (64, 96, 18944),
                                                (256, 64, 4737), (449, 32, 2433)])
 def test_emulated_projection_with_every_weight_code(ops, oracle, rows, inner, columns):
-    """Weights of all codes, in tiles of 8, 16 and 64 rows (these on tcgen05) with remainders and groups that do not fill a stage.  The code
-    of a NaN counts as 480 (the oracle has none): it meets one value of 0.5 in its group."""
+    """Weights of all codes, in tiles of 8, 16 and 64 rows (the last on tcgen05: 64 x 18944 and 256 x 4737) with remainders and groups
+    that do not fill a stage.  The code of a NaN counts as 480 (the oracle has none): it meets one value of 0.5 in its group."""
     rng = np.random.default_rng(rows + inner + columns)
     x = _codes(rng, "any", (rows, inner))
     w = rng.permutation(np.resize(np.arange(256, dtype=np.uint8), columns * inner)).reshape(columns, inner)
@@ -74,6 +74,29 @@ def test_emulated_projection_with_every_weight_code(ops, oracle, rows, inner, co
             assert np.array_equal(*got)
         else:
             assert np.array_equal(got, expected)
+
+
+@pytest.mark.parametrize("kind", ["any", "sparse", "subnormal", "extreme", "cancel", "gaps"])
+@pytest.mark.parametrize("inner", [32, 64, 128, 160, 288, 1056])
+@pytest.mark.parametrize("rows,columns", [(129, 6001), (321, 7701)])
+def test_emulated_products_in_tensor_memory(ops, oracle, rows, columns, inner, kind):
+    """Tiles of 64 rows x 128 columns with remainders, on an SM each and in more than one wave of two an SM, so that tensor memory
+    changes hands while others compute; group counts that fill the rings of unpacked groups several times over, odd ones and one
+    and two.  The rows and the weights repeat every 43 and every 203, which no tile does."""
+    rng = np.random.default_rng(rows + inner)
+    x, w = (_codes(rng, "any" if kind == "gaps" else kind, (lines, inner)) for lines in (43, 203))
+    if kind == "gaps":  # groups without a product between large and small ones
+        scale = rng.integers(0, 3, (1, inner // 32)).repeat(32, 1)
+        x = np.ascontiguousarray(np.where(scale == 0, 0, np.where(scale == 1, x & 0x87, x)).astype(np.uint8))
+    expected = np.empty((43, 203), np.uint16)
+    oracle.qgmma_codes(ptr(x), ptr(w), 43, inner, 203, 0.0625, ptr(expected))
+    x, w = x[np.arange(rows) % 43], w[np.arange(columns) % 203]
+    values = torch.from_numpy(x).view(torch.float8_e4m3fn).float().numpy()
+    scratch, out = torch.empty(x.size, dtype=torch.uint8, device="cuda"), empty_bits(rows, columns)
+    ops.call("software_e4m3_h100_linear", p(dev_bits(f32_to_bf16(values))), p(dev(w)), rows, inner, columns, 1.0, 0.0625, p(scratch),
+             p(out), stream())
+    ops.call("check_async_errors", stream())
+    assert np.array_equal(host_bits(out), expected[np.arange(rows) % 43][:, np.arange(columns) % 203])
 
 
 @pytest.mark.parametrize("kind", ["any", "sparse", "subnormal", "extreme", "cancel"])
