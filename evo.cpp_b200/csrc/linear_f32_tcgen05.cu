@@ -28,7 +28,7 @@ namespace {
 
 using namespace tc;
 
-constexpr int kWeightRows = 128, kBlockK = 64;
+constexpr int kWeightRows = 128, kBlockK = 64, kMostSplits = 8;
 constexpr int kProducerWarp = 0, kMmaWarp = 1, kSplitWarp = 10, kWorkers = 256, kF32Threads = 64 + 2 * kWorkers;
 
 template <int BT, int kPlanes>
@@ -40,7 +40,8 @@ struct F32Layout {
   static constexpr int kBarrierCount = 3 * kStages + 4;  // weights full[], rows full[], empty[], sums full[2], sums empty[2]
   static constexpr int kTmemPtrOffset = kBarrierOffset + kBarrierCount * 8;
   static constexpr int kAbortOffset = kTmemPtrOffset + 8;
-  static constexpr int kTotal = kAbortOffset + 8 + 1024;  // + alignment slack
+  static constexpr int kColumnOffset = kAbortOffset + 8;  // a byte per weight row of the tile: some weight is infinite
+  static constexpr int kTotal = kColumnOffset + kWeightRows + 1024;  // + alignment slack
   static constexpr int kBufferColumns = BT <= 32 ? 32 : BT <= 64 ? 64 : 128;
   static constexpr int kSumStride = kWeightRows + 4;
   static_assert(kStages >= 3 && BT * kSumStride * 4 <= kBarrierOffset, "the sums take the ring's place");
@@ -55,8 +56,33 @@ __device__ __forceinline__ void tmem_load_16(const std::uint32_t taddr, std::uin
       : "memory");
 }
 
-// A result that is not finite is made again in plain multiply-adds, by a warp: planes of an infinite value, or planes that
-// meet an infinite weight, would turn an infinity into a NaN.
+// Values that are not finite lie in the largest plane alone, so that their products and sums are those of multiply-adds.  An
+// infinite weight is left: planes that are zero meet it and give a NaN where the value gives an infinity.  A column that has
+// such a weight makes its results that are not finite again in plain multiply-adds, a warp each; a CTA with any result that is
+// not finite looks for these columns once, whatever its rows hold.  (1,024 rows of 2048 x 2816 that fill up eight experts' tiles: 70 us
+// where they are finite, 152 where they are NaNs or infinities; 80 and 2700 with every such result made again.)
+__device__ __noinline__ bool any_infinite(const bf16 *const w, const int K) {
+  std::uint32_t infinite = 0;
+#pragma unroll 4
+  for (int k = 8 * (threadIdx.x % 32); k < K; k += 256) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(w + k);
+    const std::uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      infinite |= (words[i] & 0x7fffU) == 0x7f80U || (words[i] & 0x7fff0000U) == 0x7f800000U ? 1U : 0U;
+  }
+  return __any_sync(0xffffffffU, infinite != 0) != 0;
+}
+__device__ __forceinline__ std::uint64_t pair_of(const float lo, const float hi) {
+  std::uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ std::uint64_t fma_pair(const std::uint64_t a, const std::uint64_t b, const std::uint64_t c) {
+  std::uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
 template <typename T>
 __device__ __noinline__ float plain_product(const T *const x, const bf16 *const w, const int K) {
   float sum = 0.0F;
@@ -209,24 +235,62 @@ linear_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const T *__
         }
       }
     };
+    const auto store_plane = [&](const float (&from)[8], const int stage, const int row, const int plane) {
+      std::uint32_t words[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        words[e] = __byte_perm(__float_as_uint(from[2 * e]), __float_as_uint(from[2 * e + 1]), 0x7632);
+      *reinterpret_cast<uint4 *>(smem + stage * L::kStageBytes + L::kWBytes + plane * L::kPlaneBytes + row * 128 + ((chunk ^ (row & 7)) << 4)) =
+          make_uint4(words[0], words[1], words[2], words[3]);
+    };
+    // what a plane leaves
+    const auto take_rest = [](float (&from)[8]) {
+      const std::uint64_t minus = pair_of(-1.0F, -1.0F);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        const std::uint64_t top = pair_of(__uint_as_float(__float_as_uint(from[e]) & 0xffff0000U),
+                                          __uint_as_float(__float_as_uint(from[e + 1]) & 0xffff0000U));
+        const std::uint64_t rest = fma_pair(top, minus, pair_of(from[e], from[e + 1]));
+        from[e] = __uint_as_float(static_cast<std::uint32_t>(rest));
+        from[e + 1] = __uint_as_float(static_cast<std::uint32_t>(rest >> 32U));
+      }
+    };
     const auto split = [&](float (&from)[kPieces][8], const int block) {
       const int i = block - first, stage = i % L::kStages;
       if (i >= L::kStages && !mbar_wait(empty(stage), (i / L::kStages - 1) & 1, abort_flag)) return false;
-      unsigned char *const planes = smem + stage * L::kStageBytes + L::kWBytes;
+      std::uint64_t probe[kPieces];
 #pragma unroll
       for (int j = 0; j < kPieces; ++j) {
         const int row = tid / 8 + 32 * j;
-        unsigned char *const at = planes + row * 128 + ((chunk ^ (row & 7)) << 4);
 #pragma unroll
         for (int plane = 0; plane < kPlanes; ++plane) {
-          std::uint32_t words[4];
+          store_plane(from[j], stage, row, plane);
+          if (plane + 1 < kPlanes) take_rest(from[j]);
+        }
+        // the last rest of a value that is not finite is a NaN
+        probe[j] = 0;
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            words[e] = __byte_perm(__float_as_uint(from[j][2 * e]), __float_as_uint(from[j][2 * e + 1]), 0x7632);
-          *reinterpret_cast<uint4 *>(at + plane * L::kPlaneBytes) = make_uint4(words[0], words[1], words[2], words[3]);
-          if (plane + 1 < kPlanes) {
+        for (int e = 0; e < 8; e += 2) probe[j] = fma_pair(pair_of(from[j][e], from[j][e + 1]), 0ULL, probe[j]);
+      }
+      if constexpr (kPlanes > 1) {
+        std::uint64_t any = probe[0];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) from[j][e] -= __uint_as_float(__float_as_uint(from[j][e]) & 0xffff0000U);
+        for (int j = 1; j < kPieces; ++j) any |= probe[j];
+        if ((any & 0x7fffffff7fffffffULL) != 0) {
+          fetch(from, block);
+#pragma unroll
+          for (int j = 0; j < kPieces; ++j) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (isnan(from[j][e])) from[j][e] = __uint_as_float(0x7fff0000U);  // one without its lower half, too
+#pragma unroll
+            for (int plane = 0; plane < kPlanes; ++plane) {
+              store_plane(from[j], stage, tid / 8 + 32 * j, plane);
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (!isfinite(from[j][e])) from[j][e] = 0.0F;
+              if (plane + 1 < kPlanes) take_rest(from[j]);
+            }
           }
         }
       }
@@ -256,21 +320,66 @@ linear_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const T *__
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2U * L::kBufferColumns)
                  : "memory");
   }
-  // a share of the tile per CTA, neighbouring threads on neighbouring columns
-  const int live = min(BT, p.rows - m0) * kWeightRows;
+  // a share of the tile's rows per CTA, a warp per row
   float *const sums = reinterpret_cast<float *>(smem);
-  for (int item = rank * kF32Threads + threadIdx.x; item < live; item += splits * kF32Threads) {
-    const int r = item / kWeightRows, c = item % kWeightRows;  // (a warp's columns are of one row)
-    float total = 0.0F;
-    for (int other = 0; other < splits; ++other) total += cluster.map_shared_rank(sums, other)[r * L::kSumStride + c];
-    const bool inside = n0 + c < p.out_features;
-    for (std::uint32_t odd = __ballot_sync(0xffffffffU, inside && !isfinite(total)); odd != 0; odd &= odd - 1) {
-      const int column = n0 + c - lane + __ffs(static_cast<int>(odd)) - 1;
-      const float plain = plain_product(input + static_cast<std::size_t>(m0 + r) * K,
-                                        p.weight + (static_cast<std::size_t>(group) * p.out_features + column) * K, K);
-      if (n0 + c == column) total = plain;
+  constexpr int kWarps = kF32Threads / 32, kColumns = kWeightRows / 32;
+  const int rows_end = min(BT, p.rows - m0), first_row = rank * kWarps + warp, row_step = splits * kWarps;
+  const auto totals = [&](const int r, float (&total)[kColumns]) {
+#pragma unroll
+    for (int i = 0; i < kColumns; ++i) total[i] = 0.0F;
+#pragma unroll
+    for (int other0 = 0; other0 < kMostSplits; other0 += 4) {  // (in order, four CTAs' parts on their way)
+      if (other0 >= splits) break;
+      float part[4][kColumns] = {};
+#pragma unroll
+      for (int o = 0; o < 4; ++o)
+        if (other0 + o < splits) {
+          const float *const from = cluster.map_shared_rank(sums, other0 + o) + r * L::kSumStride + lane;
+#pragma unroll
+          for (int i = 0; i < kColumns; ++i) part[o][i] = from[32 * i];
+        }
+#pragma unroll
+      for (int o = 0; o < 4; ++o)
+#pragma unroll
+        for (int i = 0; i < kColumns; ++i) total[i] += part[o][i];
     }
-    if (inside) store_f32_result(p, static_cast<std::size_t>(m0 + r), n0 + c, total);
+  };
+  bool odd = false;  // some result has to be looked at again
+  for (int r = first_row; r < rows_end; r += row_step) {
+    float total[kColumns];
+    totals(r, total);
+#pragma unroll
+    for (int i = 0; i < kColumns; ++i) {
+      const int column = n0 + 32 * i + lane;
+      if (column >= p.out_features) continue;
+      if (kPlanes == 1 || isfinite(total[i])) store_f32_result(p, static_cast<std::size_t>(m0 + r), column, total[i]);
+      else odd = true;
+    }
+  }
+  if (kPlanes > 1 && __syncthreads_or(odd) != 0) {
+    unsigned char *const infinite = smem + L::kColumnOffset;
+    const bf16 *const weights = p.weight + (static_cast<std::size_t>(group) * p.out_features + n0) * K;
+    for (int c = warp; c < min(kWeightRows, p.out_features - n0); c += kWarps) {
+      const bool found = any_infinite(weights + static_cast<std::size_t>(c) * K, K);
+      if (lane == 0) infinite[c] = found ? 1 : 0;
+    }
+    __syncthreads();
+    for (int r = first_row; r < rows_end; r += row_step) {
+      float total[kColumns];
+      totals(r, total);
+#pragma unroll
+      for (int i = 0; i < kColumns; ++i) {
+        const int column = n0 + 32 * i + lane;
+        const bool left = column < p.out_features && !isfinite(total[i]);
+        for (std::uint32_t again = __ballot_sync(0xffffffffU, left && infinite[32 * i + lane] != 0); again != 0; again &= again - 1) {
+          const int place = __ffs(static_cast<int>(again)) - 1;
+          const float plain = plain_product(input + static_cast<std::size_t>(m0 + r) * K,
+                                            weights + static_cast<std::size_t>(32 * i + place) * K, K);
+          if (lane == place) total[i] = plain;
+        }
+        if (left) store_f32_result(p, static_cast<std::size_t>(m0 + r), column, total[i]);
+      }
+    }
   }
   cluster.sync();  // remote shared memory stays alive until every CTA has read it
 }
@@ -293,10 +402,10 @@ int launch(const LinearF32Args &a, const F32Params &p, cudaStream_t stream) {
   // The GPCs' 148 SMs take so many clusters of 1 to 8 of these CTAs at once (cudaOccupancyMaxActiveClusters).  A CTA's K blocks
   // take about as long as its start and end from four blocks on, so the split with the fewest blocks in all waves is best (4096 x
   // 11264, 90 rows: 94 us undivided in one wave, 98 in halves and 74 in thirds in two, 77 in quarters in three).
-  constexpr unsigned int kResident[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+  constexpr unsigned int kResident[kMostSplits + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
   unsigned int splits = 1;
   std::size_t best = ~std::size_t{0};
-  for (unsigned int s = 1; s <= 8 && s <= blocks; ++s) {
+  for (unsigned int s = 1; s <= kMostSplits && s <= blocks; ++s) {
     const std::size_t waves = (static_cast<std::size_t>(tiles) * row_tiles + kResident[s] - 1) / kResident[s];
     const std::size_t cost = waves * ((blocks + s - 1) / s + 4);
     if (cost < best) best = cost, splits = s;

@@ -185,6 +185,83 @@ def test_f32_products_on_the_tensor_cores(ops, rows, inner, outer):
     assert torch.allclose(out[finite].double(), expected[finite], rtol=2e-7, atol=0.0)
 
 
+def projected(pkg, ops, x, w, float32, **more):
+    """x . W^T through the kernels of the F32 profile (1: F32 rows, 2: BF16 rows)."""
+    import ctypes
+
+    out = empty((x.shape[0], w.shape[-2]), 1)
+    args = pkg.Projection(input=x.data_ptr(), weight=w.data_ptr(), output=out.data_ptr(), rows=x.shape[0], in_features=w.shape[-1],
+                          out_features=w.shape[-2], alpha=1.0, float32=float32, f32_result=1, row_fanout=1, **more)
+    ops.call("projection", ctypes.addressof(args), stream())
+    return out
+
+
+@pytest.mark.parametrize("float32", [1, 2], ids=["f32", "bf16"])
+@pytest.mark.parametrize("rows, inner, outer", [(17, 64, 127), (96, 200, 129), (97, 1080, 260), (128, 2048, 40), (40, 4104, 2049)])
+def test_products_of_rows_and_weights_that_are_not_finite(pkg, ops, float32, rows, inner, outer):
+    """Infinities and NaNs come out as multiply-adds give them, whole rows of them, NaNs whose payload lies in their lower half,
+    columns with infinite weights (some meet infinite values) and with a NaN; everything else is as if they were not there."""
+    import torch
+
+    rng = np.random.default_rng(rows + inner)
+    x, w = cuda(rng.normal(0, 1, (rows, inner)).astype(np.float32)), cuda(rng.normal(0, 1, (outer, inner)).astype(np.float32)).bfloat16()
+    inf, nan = float("inf"), float("nan")
+    x[0], x[1, inner // 2], x[2, 5], x[3, inner - 1] = nan, nan, inf, -inf
+    x[4, 9], x[4, inner - 4] = inf, -inf
+    x[5], x[6, ::2], x[7, 8] = inf, -inf, 3e38
+    w[1, 5], w[outer // 2, 8], w[outer - 1, inner - 1], w[3, 6], w[7, 5] = inf, inf, -inf, nan, 0.0
+    x[8, 6], x[8, 8] = 0.0, 1.5
+    w[4] = 2.0 ** -20 * w[4]
+    w[4, 5:9] = 2.0 ** -100
+    if float32 == 1:
+        x.view(torch.int32)[9, 3], x.view(torch.int32)[10, inner - 2] = 0x7f800001, -0x007ffffe   # NaNs with one bit below
+    else:
+        x = x.bfloat16()
+    out = projected(pkg, ops, x, w, float32)
+    ops.call("check_async_errors", stream())
+    expected = torch.zeros(rows, outer, dtype=torch.float64, device="cuda")
+    for begin in range(0, inner, 64):  # (products before sums: infinities that meet zeros)
+        expected += (x[:, None, begin:begin + 64].double() * w[None, :, begin:begin + 64].double()).sum(2)
+    assert torch.equal(out.isnan(), expected.isnan())
+    bound = expected.abs() > 3e38  # (finite in 64 bits, not in 32)
+    assert torch.equal(out.isinf() | bound, expected.isinf() | bound)
+    assert torch.equal(out[expected.isinf()].sign().double(), expected[expected.isinf()].sign())
+    finite = expected.isfinite() & ~bound
+    magnitudes = torch.nan_to_num(x.double().abs(), 0.0, 0.0) @ torch.nan_to_num(w.double().abs(), 0.0, 0.0).T
+    assert bool(((out.double() - expected).abs() <= (24 + inner / 512) * 2.0 ** -24 * magnitudes)[finite].all())
+
+
+def test_rows_that_fill_up_a_tile_cost_no_more_than_rows(pkg, ops):
+    """An expert's tile holds a live row and what lay in the workspace: its values change nothing, and NaNs and infinities no
+    more than the time of another pass over the weights and a slower unpacking (every result made again: 34 times as long)."""
+    import torch
+
+    experts, inner, outer = 8, 2048, 2816
+    w = torch.randn(experts, outer, inner, device="cuda").bfloat16()
+    group, count = torch.arange(experts, device="cuda", dtype=torch.int32), torch.tensor([experts], device="cuda", dtype=torch.int32)
+    live = torch.randn(experts, inner, device="cuda")
+    seen = []
+    for fill in (0.5, float("nan"), float("inf")):
+        x = torch.full((experts, 128, inner), fill, device="cuda")
+        x[:, 0] = live
+        call = lambda: projected(pkg, ops, x.view(-1, inner), w, 1, groups=experts, tile_group=group.data_ptr(),
+                                 tile_count=count.data_ptr(), tile_rows=128)
+        out = call().view(experts, 128, outer)[:, 0].clone()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call()
+        times = []
+        for _ in range(8):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            begin.record()
+            graph.replay()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end))
+        seen.append((out, min(times)))
+    assert all(torch.equal(out, seen[0][0]) and time < 6 * seen[0][1] for out, time in seen), [time for _, time in seen]
+
+
 def test_few_f32_rows_cost_less_than_a_tile(ops):
     """Two rows are a stream of the weights; a tile pads them to 32 (18 us against 90 at this size)."""
     import torch
