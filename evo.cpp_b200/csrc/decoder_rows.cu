@@ -716,7 +716,8 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
   p.tile_count = a.tile_count;
   p.tile_rows = static_cast<int>(a.tile_rows);
   const bool vector = a.in_features % 8 == 0 && aligned16(a.input) && aligned16(a.weight);
-  const bool plain = a.row_group == nullptr && a.tile_group == nullptr;
+  // (up to 16 rows that share inputs without a group take a warp per output, the kernel that looks at row_fanout)
+  const bool plain = a.row_group == nullptr && a.tile_group == nullptr && a.row_fanout == 1;
   // (2 rows of 2048 x 2048: 7 us with either kernel, of 8448 x 2048 14.6 with a warp per output and 18.6 with one per three,
   // which leaves the SMs four warps each)
   const bool two_rows = plain && vector && a.rows == 2 && a.out_features >= 4096;
@@ -724,7 +725,7 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
   // once, but takes 12 us to start and to add its shares up: 4 rows of 2048 x 2048 take 14.3 us against 14.3, 12 of 2048 x 512
   // 10.2 against 12.3, 3 of 2048 x 6144 22.5 against 22.5; 6 of 2048 x 2048 16.4 against 14.3, 16 of 2048 x 8448 96 against 23.
   constexpr std::size_t kFewRowProducts = std::size_t{24} << 20;
-  if ((a.tile_group != nullptr || a.rows > 16 || (a.rows > 2 && a.rows * a.in_features * a.out_features > kFewRowProducts)) &&
+  if ((a.tile_group != nullptr || a.rows > 16 || (a.rows > 2 && plain && a.rows * a.in_features * a.out_features > kFewRowProducts)) &&
       tensorcore_linear_f32_applicable(a))
     return tensorcore_linear_f32(a, p, stream);
   // Against the tile kernel on the CUDA cores: 2 rows of 2048 x 8448 take 18 us against 90, 12 rows 72 against 90, 16 rows of

@@ -262,6 +262,22 @@ def test_rows_that_fill_up_a_tile_cost_no_more_than_rows(pkg, ops):
     assert all(torch.equal(out, seen[0][0]) and time < 6 * seen[0][1] for out, time in seen), [time for _, time in seen]
 
 
+@pytest.mark.parametrize("rows, fanout, inner, outer", [(2, 2, 264, 4099), (4, 2, 72, 6146), (8, 4, 2048, 2056), (12, 3, 1024, 4096)])
+def test_a_few_rows_that_share_inputs(pkg, ops, rows, fanout, inner, outer):
+    """row_fanout without groups, at sizes at which other rows go to other kernels: row r is input row r / row_fanout, of which there
+    are no more than that.  Chains of inner / 32 products, a sum over 32 lanes."""
+    import ctypes
+
+    rng = np.random.default_rng(rows + inner)
+    (x, xv), (w, wv) = activation(rng.normal(0, 1, (rows // fanout, inner)), 1), activation(rng.normal(0, 1, (outer, inner)), 0)
+    out = empty((rows, outer), 1)
+    args = pkg.Projection(input=x.data_ptr(), weight=w.data_ptr(), output=out.data_ptr(), rows=rows, in_features=inner,
+                          out_features=outer, alpha=1.0, float32=1, f32_result=1, row_fanout=fanout)
+    ops.call("projection", ctypes.addressof(args), stream())
+    bound = (inner / 32 + 8) * 2.0 ** -24 * (np.abs(xv) @ np.abs(wv).T)
+    assert np.all(np.abs(out.double().cpu().numpy() - (xv @ wv.T).repeat(fanout, 0).reshape(rows, outer)) <= bound.repeat(fanout, 0))
+
+
 def test_few_f32_rows_cost_less_than_a_tile(ops):
     """Two rows are a stream of the weights; a tile pads them to 32 (18 us against 90 at this size)."""
     import torch
