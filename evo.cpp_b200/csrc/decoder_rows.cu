@@ -493,44 +493,45 @@ linear_f32_rows_kernel(const T *__restrict__ input, const F32Params p) {
   if (lane == 0) store_f32_result(p, row, column, sum);
 }
 
-// Two rows: a warp per three outputs of both, so that the weights come from L2 once and the rows from L1 once per three
-// columns.  What bounds it is L1 (2 rows of 2048 x 8448: 8.6 us, 4096 x 11264: 17.8; two columns a warp 10.5 and 24.9, one
-// row and column a warp 16.6 and 36.9).
-constexpr int kPairColumns = 3;
+// Two to four rows of many columns: a warp per three columns of all rows, so that the weights come from L2 (or memory) once
+// and the rows from L1 once per three columns; a result's sums have the order of the kernel above.  What bounds it is L1 where
+// the weights are in L2 (2, 3 and 4 rows of 2048 x 8448: 7.3, 9.4 and 11.4 us; with two columns a warp 8.0, 10.4 and 12.9, with a
+// row and a column a warp 14.8, 19.5 and 24.8), and memory where they are not (9.4, 10.8 and 12.7 us, 3.7 to 2.7 TB/s).
+constexpr int kFewRowColumns = 3;
 
-template <typename T>
+template <typename T, int kRows>
 __global__ void __launch_bounds__(256)
-linear_f32_two_rows_kernel(const T *__restrict__ input, const F32Params p) {
+linear_f32_few_rows_kernel(const T *__restrict__ input, const F32Params p) {
   wait_for_producers(input);
   release_dependents();
-  const int column0 = (blockIdx.x * 8 + threadIdx.x / 32) * kPairColumns, lane = threadIdx.x % 32;
+  const int column0 = (blockIdx.x * 8 + threadIdx.x / 32) * kFewRowColumns, lane = threadIdx.x % 32;
   if (column0 >= p.out_features) return;
-  const bf16 *w[kPairColumns];  // (columns beyond the last are computed and dropped)
+  const bf16 *w[kFewRowColumns];  // (columns beyond the last are computed and dropped)
 #pragma unroll
-  for (int c = 0; c < kPairColumns; ++c)
+  for (int c = 0; c < kFewRowColumns; ++c)
     w[c] = p.weight + static_cast<std::size_t>(min(column0 + c, p.out_features - 1)) * p.in_features;
-  float sum[2][kPairColumns] = {};
+  float sum[kRows][kFewRowColumns] = {};
 #pragma unroll 4
   for (int k = 8 * lane; k < p.in_features; k += 256) {
-    float b[kPairColumns][8];
+    float b[kFewRowColumns][8];
 #pragma unroll
-    for (int c = 0; c < kPairColumns; ++c) load_floats<8>(w[c] + k, b[c]);
+    for (int c = 0; c < kFewRowColumns; ++c) load_floats<8>(w[c] + k, b[c]);
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < kRows; ++r) {
       float a[8];
       load_floats<8>(input + static_cast<std::size_t>(r) * p.in_features + k, a);
 #pragma unroll
-      for (int c = 0; c < kPairColumns; ++c)
+      for (int c = 0; c < kFewRowColumns; ++c)
 #pragma unroll
         for (int i = 0; i < 8; ++i) sum[r][c] = fmaf(a[i], b[c][i], sum[r][c]);
     }
   }
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
+  for (int r = 0; r < kRows; ++r)
 #pragma unroll
-    for (int c = 0; c < kPairColumns; ++c) {
+    for (int c = 0; c < kFewRowColumns; ++c) {
       const float total = warp_sum(sum[r][c]);
-      if (lane == r * kPairColumns + c && column0 + c < p.out_features)
+      if (lane == r * kFewRowColumns + c && column0 + c < p.out_features)
         store_f32_result(p, static_cast<std::size_t>(r), column0 + c, total);
     }
 }
@@ -718,14 +719,16 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
   const bool vector = a.in_features % 8 == 0 && aligned16(a.input) && aligned16(a.weight);
   // (up to 16 rows that share inputs without a group take a warp per output, the kernel that looks at row_fanout)
   const bool plain = a.row_group == nullptr && a.tile_group == nullptr && a.row_fanout == 1;
-  // (2 rows of 2048 x 2048: 7 us with either kernel, of 8448 x 2048 14.6 with a warp per output and 18.6 with one per three,
-  // which leaves the SMs four warps each)
-  const bool two_rows = plain && vector && a.rows == 2 && a.out_features >= 4096;
-  // Every row of the few-row kernel fetches the weights again, from L2 where they fit.  The tensor cores' kernel fetches them
-  // once, but takes 12 us to start and to add its shares up: 4 rows of 2048 x 2048 take 14.3 us against 14.3, 12 of 2048 x 512
-  // 10.2 against 12.3, 3 of 2048 x 6144 22.5 against 22.5; 6 of 2048 x 2048 16.4 against 14.3, 16 of 2048 x 8448 96 against 23.
+  // Three columns a warp need columns for every SM, and more of them the more rows the tensor cores' kernel would take along (weights
+  // from memory: 2 rows of 2048 x 2048 7.4 us against 6.8 with a warp per output, of 2048 x 4096 7.9 against 10.6; 3 rows 8.9 against
+  // 10.5 on the tensor cores; 4 rows of 2048 x 4096 11.3 against 10.5, of 2048 x 6144 12.3 against 15.8, of 4096 x 11264 37.9 against 39.0).
+  const bool few_wide_rows = plain && vector && a.rows >= 2 && a.rows <= 4 && a.out_features >= (a.rows < 4 ? 4096U : 6144U);
+  // Every row of a warp per output fetches the weights again, from L2 where they fit.  The tensor cores' kernel fetches them
+  // once, but takes 12 us alone to start and to add its shares up: 4 rows of 2048 x 2048 take 14.3 us against 14.3, 12 of 2048 x 512
+  // 10.2 against 12.3; 6 of 2048 x 2048 16.4 against 14.3, 16 of 2048 x 8448 96 against 23.
   constexpr std::size_t kFewRowProducts = std::size_t{24} << 20;
-  if ((a.tile_group != nullptr || a.rows > 16 || (a.rows > 2 && plain && a.rows * a.in_features * a.out_features > kFewRowProducts)) &&
+  if (!few_wide_rows &&
+      (a.tile_group != nullptr || a.rows > 16 || (a.rows > 2 && plain && a.rows * a.in_features * a.out_features > kFewRowProducts)) &&
       tensorcore_linear_f32_applicable(a))
     return tensorcore_linear_f32(a, p, stream);
   // Against the tile kernel on the CUDA cores: 2 rows of 2048 x 8448 take 18 us against 90, 12 rows 72 against 90, 16 rows of
@@ -737,9 +740,13 @@ int linear_f32(const LinearF32Args &a, cudaStream_t stream) {
   const auto launch = [&](auto tag) {
     using T = decltype(tag);
     const T *const input = static_cast<const T *>(a.input);
-    if (two_rows)
-      return launch_dependent("F32 linear kernel (two rows)", linear_f32_two_rows_kernel<T>,
-                              dim3(ceil_div_u(a.out_features, 8 * kPairColumns)), 256, 0, stream, true, 1, input, p);
+    if (few_wide_rows) {
+      const auto kernel = a.rows == 2   ? linear_f32_few_rows_kernel<T, 2>
+                          : a.rows == 3 ? linear_f32_few_rows_kernel<T, 3>
+                                        : linear_f32_few_rows_kernel<T, 4>;
+      return launch_dependent("F32 linear kernel (a few wide rows)", kernel, dim3(ceil_div_u(a.out_features, 8 * kFewRowColumns)),
+                              256, 0, stream, true, 1, input, p);
+    }
     if (few_rows) {
       const auto kernel = vector ? linear_f32_rows_kernel<T, true> : linear_f32_rows_kernel<T, false>;
       return launch_dependent("F32 linear kernel (few rows)", kernel,

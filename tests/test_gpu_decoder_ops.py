@@ -278,6 +278,31 @@ def test_a_few_rows_that_share_inputs(pkg, ops, rows, fanout, inner, outer):
     assert np.all(np.abs(out.double().cpu().numpy() - (xv @ wv.T).repeat(fanout, 0).reshape(rows, outer)) <= bound.repeat(fanout, 0))
 
 
+@pytest.mark.parametrize("float32", [1, 2], ids=["f32", "bf16"])
+@pytest.mark.parametrize("rows, inner, outer", [(2, 8, 4096), (2, 264, 4099), (3, 2056, 4096), (3, 256, 4097), (4, 520, 6144), (4, 72, 6146)])
+def test_a_few_wide_rows(pkg, ops, float32, rows, inner, outer):
+    """Three columns a warp, with remainders of columns and of the inner size, bias, alpha and soft cap.  A chain of products has
+    ceil(inner / 256) * 8 terms, the lanes' sum five and the epilogue three: so many units of 2^-24 of the magnitudes, and the
+    soft cap's own 4 of its bound."""
+    import ctypes
+    import torch
+
+    rng = np.random.default_rng(rows + inner + outer)
+    (x, xv), (w, wv) = activation(rng.normal(0, 1, (rows, inner)), float32 == 1), activation(rng.normal(0, 1, (outer, inner)), 0)
+    bias = rng.normal(0, 1, outer).astype(np.float32)
+    db, out = cuda(bias), empty((rows, outer), 1)
+    for softcap in (0.0, 50.0):
+        args = pkg.Projection(input=x.data_ptr(), weight=w.data_ptr(), output=out.data_ptr(), bias=db.data_ptr(), rows=rows,
+                              in_features=inner, out_features=outer, alpha=0.5, softcap=softcap, float32=float32, f32_result=1,
+                              row_fanout=1)
+        ops.call("projection", ctypes.addressof(args), stream())
+        expected = 0.5 * (xv @ wv.T) + bias
+        bound = (8 * -(-inner // 256) + 8) * 2.0 ** -24 * (0.5 * (np.abs(xv) @ np.abs(wv).T) + np.abs(bias))
+        if softcap:
+            expected, bound = softcap * np.tanh(expected / softcap), bound + 4 * 2.0 ** -23 * softcap
+        assert np.all(np.abs(out.double().cpu().numpy() - expected) <= bound)
+
+
 def test_few_f32_rows_cost_less_than_a_tile(ops):
     """Two rows are a stream of the weights, 32 a tile (7.4 us against 15.7 at this size, on the GPU alone: a call through ctypes
     can take as long as the two rows)."""
