@@ -46,9 +46,9 @@ struct RowFront {
 // gemv.cu: whether one row of these sizes and buffers takes it.
 bool row_front_applicable(const RowFront &front, const void *input, const void *weight, std::size_t in_features,
                           std::size_t out_features);
-// [rows, in] (F32 or BF16) x BF16 [out, in]^T in F32 fused multiply-adds.  output = [output +] alpha *
-// row_scale[r] * product + bias, then softcap tanh(output / softcap) where softcap > 0.  Grouped weights
-// [groups, out, in]: see LinearArgs (row_group / row_fanout, or tile_group / tile_count / tile_rows).
+// [rows, in] (F32 or BF16) x BF16 [out, in]^T in F32: fused multiply-adds, and for more rows the exact products of a row's three
+// BF16 parts on the tensor cores (linear_f32_tcgen05.cu, errors there).  output = [output +] alpha * row_scale[r] * product +
+// bias, then softcap tanh(output / softcap) where softcap > 0.  Grouped weights [groups, out, in]: see LinearArgs (row_group / row_fanout, or tile_group / tile_count / tile_rows).
 struct LinearF32Args {
   const void *input = nullptr;
   Activation input_type = Activation::kF32;

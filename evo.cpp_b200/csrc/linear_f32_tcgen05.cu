@@ -1,6 +1,7 @@
-// F32 projections of a few rows or more on the tensor cores, without losing precision: an F32 value is the exact sum of
-// three BF16 values (its significand's 24 bits in eights, cut toward zero), a BF16 weight is one, and so a product is the
-// sum of three exact BF16 products.
+// F32 projections of a few rows or more on the tensor cores, with all bits of the operands: an F32 value of at least 2^-110 is
+// the exact sum of three BF16 values (its significand's 24 bits in eights, cut toward zero), a BF16 weight is one, and so a
+// product is the sum of three exact BF16 products.  Below 2^-110 the bits of a value below 2^-133 are lost, at most 2^-133 |w| of
+// a product; multiply-adds keep them.
 //
 // The weights are the M = 128 operand and stream through shared memory once (TMA, 64 K values a block); the rows are the
 // narrow one, split into their planes by eight warps that read them as F32 from L2.  A K block's 192 products per output
@@ -10,8 +11,11 @@
 //
 // What bounds it: the weight stream (two bytes a weight) and, from 64 rows on, the splitting of the rows and the reading of
 // the block sums beside 12 MMAs per block.  90 rows of a 2048-wide model with 8448 inner columns: 25 products in 0.55 ms, 3.18
-// as multiply-adds on the CUDA cores; 90 rows of 2048 x 8448 31 us against 154, 1,000 rows 215 against 1294.  Errors against
-// float64 (2-norm) are smaller than the multiply-adds': 1.2e-7 against 2.1e-7 at K = 2048, 1.4e-7 against 4.2e-7 at 8448.
+// as multiply-adds on the CUDA cores; 90 rows of 2048 x 8448 20 us behind one another, 1,000 rows 149.
+// Errors against float64 (2-norm over normal operands, against multiply-adds in the CUDA cores' tiles): smaller where products
+// have both signs, 0.9e-7 against 1.1e-7 at K = 256, 1.05e-7 against 2.1e-7 at 2048, 1.2e-7 against 4.2e-7 at 8448.  Where all
+// have one sign the cuts add up: results are 0.85e-7 of themselves too small on average (1.4e-7 where a few values carry a
+// sum; multiply-adds below 1e-9), and errors 0.96e-7 against 0.52e-7, 0.99e-7 against 0.67e-7 and 1.00e-7 against 1.02e-7.
 #include <cooperative_groups.h>
 
 #include <algorithm>

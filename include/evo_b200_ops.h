@@ -383,7 +383,11 @@ EVO_B200_API int evo_b200_poly_norm(const void *input, const void *coefficients,
 /* table[h, d] = r1[h] ln(1 + r2[h] d). */
 EVO_B200_API int evo_b200_distance_bias_table(const void *r1, const void *r2, size_t heads, size_t distances,
                                               void *table, void *stream);
-/* F32 [rows, in] x BF16 [out, in]^T with F32 multiply-adds; output (+)= product. */
+/* F32 [rows, in] x BF16 [out, in]^T in F32; output (+)= product.  Up to 16 rows (fewer where rows x in x out is large) and inner
+ * sizes below 64 or no multiple of 8: F32 multiply-adds.  Otherwise every row is three BF16 parts, exactly, whose exact products
+ * tensor cores add in F32, cut toward zero over at most 64 values of `in` and rounded between them: errors are those of
+ * multiply-adds or smaller for sums of both signs, and up to 1.5e-7 of a sum whose terms all have one sign (towards zero; up to 0.6e-7
+ * to 1.0e-7 by multiply-adds, either way).  What a row's values hold below 2^-133 is lost. */
 EVO_B200_API int evo_b200_f32_linear(const void *input, const void *weight, size_t rows, size_t in_features,
                                      size_t out_features, int accumulate, void *output, void *stream);
 /* BF16 [rows, in] x BF16 [out, in]^T, the F32 accumulator stored (or added) without rounding; the split
@@ -471,8 +475,8 @@ EVO_B200_API int evo_b200_layer_norm(const evo_b200_layer_norm_args *args, void 
  * u = clamp(b, +-limit), over weight rows in alternating blocks of 128 gate and 128 up rows; output [rows,
  * out_features / 2].  bias F32 in the weight's row order.  Grouped weights [groups, out, in]: row_group [rows] with
  * row_fanout output rows per input row, or tiles of tile_rows (128, 256) rows with tile_group and tile_count (all
- * int32 on the device).  float32: F32 operands and results in F32 multiply-adds (gate: 0 only); 2: BF16 operands in
- * the same kernels. */
+ * int32 on the device).  float32: F32 operands and results in F32 (gate: 0 only; the products as evo_b200_f32_linear's, and with tiles
+ * and `groups` given on the tensor cores); 2: BF16 operands in the same kernels. */
 typedef struct evo_b200_projection_args {
   size_t struct_size;
   const void *input, *weight, *bias, *row_scale;

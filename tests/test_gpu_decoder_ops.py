@@ -149,9 +149,11 @@ def test_few_f32_rows(ops, rows, inner, outer):
                                                 (129, 136, 1000), (3, 2056, 6150), (16, 4104, 2049), (2, 264, 4096), (2, 2056, 4099)])
 def test_f32_products_on_the_tensor_cores(ops, rows, inner, outer):
     """Every row tile, K blocks and weight tiles with remainders, one CTA and clusters that divide K, and two rows.  A block
-    of 64 products is cut 12 times at 2^-23 of a sum of at most its magnitudes (the smaller planes' cuts are below that), the
-    blocks' sums are rounded: 16 + ceil(inner / 64) / 8 + 8 units of 2^-24.  Then values that are not finite, and the
-    smallest ones: the same infinities and NaNs as multiply-adds give."""
+    of 64 products is cut at 2^-23 of a sum of at most its magnitudes four times with the largest plane (8 units of 2^-24; the smaller
+    planes' eight cuts are 2^-8 of these), the blocks' and the CTAs' sums are rounded: 16 + inner / 512 + 8 units allow for that
+    with clusters of eight, and for 8 units beyond.  (A product more than 2^-11 below the largest is cut as well, at 2^-25 of
+    it: 32 units if all but one were, a tenth of a unit here.)  Then values that are not finite: the same infinities and NaNs as
+    multiply-adds give."""
     import torch
 
     rng = np.random.default_rng(rows * 1000 + inner)
@@ -183,6 +185,38 @@ def test_f32_products_on_the_tensor_cores(ops, rows, inner, outer):
     finite = expected.isfinite()
     assert torch.equal(out[out.isinf()].sign().double(), expected[out.isinf()].sign())
     assert torch.allclose(out[finite].double(), expected[finite], rtol=2e-7, atol=0.0)
+
+
+@pytest.mark.parametrize("spread", [0.0, 2.0])
+@pytest.mark.parametrize("rows, inner", [(128, 256), (90, 2056), (40, 8448)])
+def test_f32_products_of_one_sign(ops, rows, inner, spread):
+    """The tensor cores' cuts do not cancel here: a block's four cuts with the largest plane take up to 2^-23 of its sum each, half
+    of that on average, so results are too small by at most 4 units of 2^-24 on average, and too large by no more than the
+    roundings' own mean (a tenth of a unit)."""
+    rng = np.random.default_rng(inner + int(spread))
+    w, wv = activation(np.abs(rng.normal(0, 1, (384, inner))), 0)
+    x = np.abs(rng.normal(0, 1, (rows, inner)) * np.exp(rng.normal(0, 1, (rows, inner)) * spread)).astype(np.float32)
+    exact, out = cuda(x), empty((rows, 384), 1)
+    ops.call("f32_linear", exact.data_ptr(), w.data_ptr(), rows, inner, 384, 0, out.data_ptr(), stream())
+    expected = x.astype(np.float64) @ wv.T
+    mean = np.mean((out.double().cpu().numpy() - expected) / expected)
+    assert -4 * 2.0 ** -24 <= mean <= 0.1 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("exponent", [-100, -110, -118, -126, -132, -140, -149])
+def test_f32_products_of_the_smallest_values(ops, exponent):
+    """What lies below 2^-133 of a value is lost, and nothing else: 2^-133 of a weight beside the bound of other values and half
+    of the smallest F32 number per addition."""
+    rng = np.random.default_rng(-exponent)
+    rows, inner, outer = 40, 264, 130
+    w, wv = activation(rng.normal(0, 1, (outer, inner)) * np.exp2(rng.integers(0, 30, (outer, 1))), 0)
+    x = (rng.normal(0, 1, (rows, inner)) * 2.0 ** exponent).astype(np.float32)
+    exact, out = cuda(x), empty((rows, outer), 1)
+    ops.call("f32_linear", exact.data_ptr(), w.data_ptr(), rows, inner, outer, 0, out.data_ptr(), stream())
+    xv = x.astype(np.float64)
+    error = np.abs(out.double().cpu().numpy() - xv @ wv.T)
+    bound = (24 + inner / 512) * 2.0 ** -24 * (np.abs(xv) @ np.abs(wv).T) + 2.0 ** -133 * np.abs(wv).sum(1) + inner * 2.0 ** -150
+    assert np.all(error <= bound)
 
 
 def projected(pkg, ops, x, w, float32, **more):
