@@ -51,15 +51,6 @@ struct F32Layout {
   static_assert(kStages >= 3 && BT * kSumStride * 4 <= kBarrierOffset, "the sums take the ring's place");
 };
 
-__device__ __forceinline__ void tmem_load_16(const std::uint32_t taddr, std::uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-}
-
 // Values that are not finite lie in the largest plane alone, so that their products and sums are those of multiply-adds.  An
 // infinite weight is left: planes that are zero meet it and give a NaN where the value gives an infinity.  A column that has
 // such a weight makes its results that are not finite again in plain multiply-adds, a warp each; a CTA with any result that is
@@ -391,8 +382,8 @@ linear_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const T *__
 template <typename T, int BT>
 int launch(const LinearF32Args &a, const F32Params &p, cudaStream_t stream) {
   using L = F32Layout<BT, std::is_same_v<T, float> ? 3 : 1>;
-  int status = kOk, sm_count = 0;
-  int *const error = error_word(&status, &sm_count);
+  int status = kOk;
+  int *const error = error_word(&status, nullptr);
   if (error == nullptr) return status;
   CUtensorMap map;
   // (a tile beyond the last group's rows reads zeros, beyond another's rows of the next group: neither is stored)
@@ -403,7 +394,8 @@ int launch(const LinearF32Args &a, const F32Params &p, cudaStream_t stream) {
     return fail(kCuda, "cannot raise the shared-memory limit of the F32 linear kernel");
   const unsigned int tiles = ceil_div_u(a.out_features, kWeightRows), row_tiles = ceil_div_u(a.rows, BT);
   const std::size_t blocks = (a.in_features + kBlockK - 1) / kBlockK;
-  // The GPCs' 148 SMs take so many clusters of 1 to 8 of these CTAs at once (cudaOccupancyMaxActiveClusters).  A CTA's K blocks
+  // The GPCs of a B200 (148 SMs) take so many clusters of 1 to 8 of these CTAs at once (cudaOccupancyMaxActiveClusters; another part
+  // would get the same results in other times).  A CTA's K blocks
   // take about as long as its start and end from four blocks on, so the split with the fewest blocks in all waves is best (4096 x
   // 11264, 90 rows: 94 us undivided in one wave, 98 in halves and 74 in thirds in two, 77 in quarters in three).
   constexpr unsigned int kResident[kMostSplits + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
