@@ -495,8 +495,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
 // The same projection with two CTAs of a cluster on one output tile of 256 rows x kPairN columns (256, or 192 where that
 // fills the last wave better).  Each CTA loads its own 128 rows of A and its own half of the tile's weight rows (TMA without
 // multicast; the copies report to the leader's mbarrier), the leader issues tcgen05.mma.cta_group::2 (M = 256), and each CTA
-// ends up with its 128 rows of the accumulator in its own tensor memory and stores them as the one-CTA kernel does.  Per SM a stage is 32 KiB instead of 48 for the same arithmetic: a third
-// less traffic from L2, and six stages in flight instead of four.
+// ends up with its 128 rows of the accumulator in its own tensor memory and stores them as the one-CTA kernel does.  Per SM a
+// stage is 32 KiB instead of 48 for the same arithmetic, a third less traffic from L2, and six stages are in flight instead of
+// four (192 columns: 28 KiB, seven stages).
 template <int kPairN>
 struct PairLayout {
   static constexpr int kPairStages = kPairN == 256 ? 6 : 7;

@@ -9,8 +9,9 @@
 // core cuts its sums toward zero, and 64 terms of the largest plane are as far as that may go.  A cluster divides K and
 // adds its CTAs' sums in order.
 //
-// What bounds it: the weight stream (two bytes a weight) and, from 64 rows on, the splitting of the rows and the reading of
-// the block sums beside 12 MMAs per block.  90 rows of a 2048-wide model with 8448 inner columns: 25 products in 0.55 ms, 3.18
+// What bounds it: up to some dozens of rows the weight stream (32 rows of 4096 x 4096: 17 us, 2 TB/s) and the start and end of a
+// CTA; at 90 rows the latencies of a block's steps (tensor pipe 33 %, issue slots 37 %, no unit above 45 %); at 1,000 rows L1, which
+// takes the rows in as F32 and the planes (71 %), with the tensor pipe at 43 % and issue slots at 51 %.  90 rows of a 2048-wide model with 8448 inner columns: 25 products in 0.48 ms, 3.18
 // as multiply-adds on the CUDA cores; 90 rows of 2048 x 8448 20 us behind one another, 1,000 rows 149.
 // Errors against float64 (2-norm over normal operands, against multiply-adds in the CUDA cores' tiles): smaller where products
 // have both signs, 0.9e-7 against 1.1e-7 at K = 256, 1.05e-7 against 2.1e-7 at 2048, 1.2e-7 against 4.2e-7 at 8448.  Where all
