@@ -608,11 +608,12 @@ norm_gate_quads_kernel(const float *__restrict__ input, const float *__restrict_
 // its part of the state in registers between the read-out and the update (a warp per set of channels, a lane
 // per column), and the output norm's sums meet in distributed shared memory, where every CTA stores its parts in all others:
 // one cluster barrier.
-// What bounds it is trips to memory and the first execution of its code: all reads are issued before any is used, the taps'
-// products come without a loop.  The key and the query are scaled before their product is summed (a sum of unscaled values
+// What bounds it is trips to memory and the first execution of its code: the delta rule's reads are issued before any is used, the
+// taps' products come without a loop.  The key and the query are scaled before their product is summed (a sum of unscaled values
 // can be infinite where both factors are zero), and every sum keeps the order of the block's warps.  In a step of Gigusun (dim 128)
-// it ends 8.8 us behind the projection in front of it for the delta rule (10.4 with reads where they are used), 7.0 for linear
-// attention; 48 steps 12.07 -> 11.84 ms.
+// it ends 8.8 us behind the projection in front of it for the delta rule (10.4 with reads where they are used).  Steps behind one another
+// (16 heads, 8 keys, 128 x 128, states in L2): 6.7 us for the delta rule, 9.2 with reads where they are used; linear attention 5.1, 5.9
+// with its decays' ranks read in turn and 6.3 with its columns read in front of the decays.
 constexpr int kDecodeRanks = 8, kDecodeThreads = 256, kDecodeWarps = kDecodeThreads / 32;
 constexpr int kDecodeMaxGroup = 64;  // heads per key head
 
@@ -629,7 +630,11 @@ struct ConvInput {
   float x[kHeldTaps], weight[kHeldTaps];
 };
 
-template <bool kDelta, typename T>
+// kOneBlock: no CTA has more than 32 columns, one turn of the loop over them.  The two forms differ in what they ask for behind the first
+// turn, and with it in registers: the first has 128 and stands beside the CTAs of the kernels around it (a step of Gigusun 0.7 %
+// faster than with the other, which takes 255); the other is the faster one where the loop turns (16 heads of 64 x 256 on two keys, eight turns:
+// 19.6 us, 26.1 with the first).
+template <bool kDelta, bool kOneBlock, typename T>
 __global__ void __launch_bounds__(kDecodeThreads)
 decode_kernel(const T *__restrict__ projection, T *const history, const float *__restrict__ conv,
               const float *__restrict__ decay_rate, const float *__restrict__ decay_shift,
@@ -668,7 +673,7 @@ decode_kernel(const T *__restrict__ projection, T *const history, const float *_
     for (int j = 0; j < kHeldTaps; ++j) sum = fmaf(in.weight[j], in.x[j], sum);
     return silu_f32(sum);
   };
-  // everything that the step reads is asked for before any of it is used: a trip to memory is 0.4 us
+  // what the step reads is asked for before any of it is used, but for the linear form's columns: a trip to memory is 0.4 us
   const int d = threadIdx.x;  // kDecodeThreads == kDecoderMaxHeadDim: a thread per key channel
   const bool has_channel = d < p.dim;
   ConvInput k_in{}, q_in{};
@@ -711,7 +716,7 @@ decode_kernel(const T *__restrict__ projection, T *const history, const float *_
       v_raw = to_float(projection[p.value_column + head * p.value_dim + column]);
     }
   };
-  read_columns(0);
+  if constexpr (kDelta) read_columns(0);
   float gate = 0.0F, own_gain = 0.0F;  // of this thread's first column
   if (threadIdx.x < count) {
     gate = to_float(projection[p.gate_column + g * columns + begin + threadIdx.x]);
@@ -723,9 +728,22 @@ decode_kernel(const T *__restrict__ projection, T *const history, const float *_
       q = convolved(q_in, g * p.dim + d);
     } else {
       const int channel = g * p.dim + d;
-#pragma unroll 16
-      for (int r = 0; r < p.rank; ++r)
-        z = fmaf(decay_weight[static_cast<std::size_t>(r) * p.heads * p.dim + channel], to_float(projection[p.beta_column + r]), z);
+      const auto add_ranks = [&](const int r0, auto size, const bool whole) {  // (a batch's reads are on their way together)
+        constexpr int kSize = decltype(size)::value;
+        float w[kSize], x[kSize];
+#pragma unroll
+        for (int i = 0; i < kSize; ++i) {
+          const bool inside = whole || r0 + i < p.rank;
+          w[i] = inside ? decay_weight[static_cast<std::size_t>(r0 + i) * p.heads * p.dim + channel] : 0.0F;
+          x[i] = inside ? to_float(projection[p.beta_column + r0 + i]) : 0.0F;
+        }
+#pragma unroll
+        for (int i = 0; i < kSize; ++i)
+          if (whole || r0 + i < p.rank) z = fmaf(w[i], x[i], z);
+      };
+      int r = 0;
+      for (; r + 16 <= p.rank; r += 16) add_ranks(r, std::integral_constant<int, 16>{}, true);
+      for (; r < p.rank; r += 8) add_ranks(r, std::integral_constant<int, 8>{}, false);
       alpha[d] = expf(-softplus_f32(-z) * p.inverse_tau);
     }
   }
@@ -755,12 +773,37 @@ decode_kernel(const T *__restrict__ projection, T *const history, const float *_
   __syncthreads();
   const float key_query = kDelta ? shared_sum(2) : 0.0F;
   for (int c0 = 0; c0 < count; c0 += 32) {
-    if (c0 != 0) read_columns(c0);
+    if constexpr (!kDelta) {
+      read_columns(c0);  // (in front of the decays their registers cost more than the trip: 6.3 us instead of 5.1)
+    } else if (c0 != 0) {
+      if constexpr (kOneBlock) {
+        read_columns(c0);
+      } else {
+        const int c = begin + c0 + lane;
+        live = c0 + lane < count;
+        head = g * group + (live ? c / p.value_dim : 0);
+        column = live ? c % p.value_dim : 0;
+      }
+    }
     float *const cells = state + static_cast<std::size_t>(head) * p.dim * p.value_dim + column;
+    if (!kOneBlock && kDelta && c0 != 0) {
+#pragma unroll
+      for (int i = 0; i < kHeld; ++i) {
+        const int row = warp + kDecodeWarps * i;
+        held[i] = live && row < p.dim && p.fresh == 0 ? cells[static_cast<std::size_t>(row) * p.value_dim] : 0.0F;
+      }
+    }
     float v = v_raw, beta = 0.0F, decay = 1.0F;
     if (live) {
       if constexpr (kDelta) {
-        v = convolved(v_in, p.value_column + head * p.value_dim + column);
+        const int channel = p.value_column + head * p.value_dim + column;
+        if (!kOneBlock && c0 != 0) {
+          v = conv_silu(projection, 0, history, p.channels, conv, p.taps, p.fresh != 0, 0, channel);
+          beta_raw = to_float(projection[p.beta_column + head]), decay_raw = to_float(projection[p.decay_column + head]);
+          rate = decay_rate[head], shift = decay_shift[head];
+        } else {
+          v = convolved(v_in, channel);
+        }
         v = to_float(from_float<T>(v));  // the prompt's kernels keep convolved values in the activation type
         beta = sigmoid_f32(beta_raw);
         decay = expf(rate * softplus_f32(decay_raw + shift));
@@ -800,14 +843,30 @@ decode_kernel(const T *__restrict__ projection, T *const history, const float *_
         cells[static_cast<std::size_t>(row) * p.value_dim] = kDelta ? fmaf(key[row], u, held[i]) : held[i];
     }
   }
+  // The squares of this CTA's part of every head, in the order of a block's sum: a chain per thread, warps, their sums in order.
+  // One block of columns is one warp's sum, which needs no exchange.
+  float *const parts = &partial[0][0][0];
+  static_assert(kDecodeMaxGroup * kDecodeWarps <= 2 * kDecodeWarps * 32, "a sum per head and warp");
+  const auto head_begin = [&](const int local) { return max(local * p.value_dim, begin) - begin; };
+  const auto head_end = [&](const int local) { return min((local + 1) * p.value_dim, begin + count) - begin; };
+  if constexpr (!kOneBlock) {
+    for (int local = begin / p.value_dim; local < group && local * p.value_dim < begin + count; ++local) {
+      float square = 0.0F;
+      for (int c = head_begin(local) + threadIdx.x; c < head_end(local); c += kDecodeThreads) square = fmaf(outputs[c], outputs[c], square);
+      square = warp_sum(square);
+      if (lane == 0) parts[local * kDecodeWarps + warp] = square;
+    }
+    __syncthreads();
+  }
   cluster.barrier_wait();  // every CTA of the cluster runs
   for (int local = warp; local < group; local += kDecodeWarps) {
-    const int from = max(local * p.value_dim, begin) - begin, to = min((local + 1) * p.value_dim, begin + count) - begin;
     float square = 0.0F;
-    for (int c0 = from; c0 < to && c0 < from + kDecodeThreads; c0 += 32) {  // (chains and sums as a block's threads and warps form them)
-      float chain = 0.0F;
-      for (int c = c0 + lane; c < to; c += kDecodeThreads) chain = fmaf(outputs[c], outputs[c], chain);
-      square += warp_sum(chain);
+    if constexpr (!kOneBlock) {
+      if (head_begin(local) < head_end(local))
+        for (int w = 0; w < kDecodeWarps; ++w) square += parts[local * kDecodeWarps + w];
+    } else {
+      const int c = head_begin(local) + lane;
+      square = warp_sum(c < head_end(local) ? outputs[c] * outputs[c] : 0.0F);
     }
     if (lane < kDecodeRanks) cluster.map_shared_rank(&squares[0][0], lane)[rank * kDecodeMaxGroup + local] = square;
   }
@@ -837,8 +896,8 @@ decode_kernel(const T *__restrict__ projection, T *const history, const float *_
             i + 2 < p.taps ? (p.fresh == 0 ? history[static_cast<std::size_t>(i + 1) * p.channels + column] : from_float<T>(0.0F))
                            : projection[column];
     };
-    const bool one_read = count <= 32;  // every warp still holds its lane's value channel
-    for (int c = threadIdx.x; c < count; c += kDecodeThreads) advance(p.value_column + g * columns + begin + c, one_read ? &v_in : nullptr);
+    // (of one block of columns every warp still holds its lane's value channel)
+    for (int c = threadIdx.x; c < count; c += kDecodeThreads) advance(p.value_column + g * columns + begin + c, kOneBlock ? &v_in : nullptr);
     if (rank == 0 && has_channel) {
       advance(g * p.dim + d, &q_in);
       advance(p.key_column + g * p.dim + d, &k_in);
@@ -865,9 +924,10 @@ int launch_decode(const RecurrentArgs &a, cudaStream_t stream) {
   p.epsilon = a.epsilon;
   p.fresh = a.fresh ? 1 : 0;
   const std::size_t columns = (kDelta ? a.heads / a.kv_heads : 1) * a.value_dim;
-  return launch_dependent("recurrent decode kernel", decode_kernel<kDelta, T>,
+  const std::size_t share = (columns + kDecodeRanks - 1) / kDecodeRanks;
+  return launch_dependent("recurrent decode kernel", share <= 32 ? decode_kernel<kDelta, true, T> : decode_kernel<kDelta, false, T>,
                           dim3(kDecodeRanks, static_cast<unsigned int>(kDelta ? a.kv_heads : a.heads)), kDecodeThreads,
-                          (columns + kDecodeRanks - 1) / kDecodeRanks * sizeof(float), stream, true, kDecodeRanks,
+                          share * sizeof(float), stream, true, kDecodeRanks,
                           static_cast<const T *>(a.projection), static_cast<T *>(a.conv_history), a.conv, a.decay_rate,
                           a.decay_shift, a.decay_weight, a.decay_bias, a.output_norm, a.state, static_cast<T *>(a.output), p);
 }

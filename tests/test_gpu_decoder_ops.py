@@ -651,6 +651,22 @@ def test_extreme_gates_stay_finite(pkg, ops):
 
 
 @TYPES
+@pytest.mark.parametrize("delta, heads, kv_heads, dim, vdim, taps, rank", [
+    (True, 4, 1, 40, 64, 4, 5), (True, 4, 1, 40, 66, 1, 5), (True, 4, 1, 40, 66, 6, 5), (True, 16, 2, 64, 256, 2, 5),
+    (True, 5, 1, 24, 512, 4, 5), (True, 3, 1, 256, 100, 6, 5), (False, 2, 2, 40, 256, 4, 3), (False, 2, 2, 40, 257, 4, 16),
+    (False, 3, 3, 128, 512, 4, 17), (False, 4, 4, 256, 8, 4, 24), (False, 2, 2, 20, 264, 4, 9)])
+def test_single_steps_of_wide_groups(pkg, ops, float32, delta, heads, kv_heads, dim, vdim, taps, rank):
+    """32 and 33 columns a CTA and many blocks of them, taps that are held and that are not, decays of whole and partial batches
+    of ranks: six tokens, one after another, carry the state and the history.  (BF16 rounds the six tokens' values, each by 2^-9 of
+    itself; with terms that cancel a cell of the state can be half as large as they are: 2 6 2^-9.)"""
+    case = Recurrence(pkg, ops, delta=delta, rows=6, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, float32=float32, taps=taps,
+                      rank=rank, seed=dim + vdim + taps)
+    expected, state = case.expected(6)
+    assert_near(np.concatenate([case.run(1).float().cpu().numpy() for _ in range(6)]).astype(np.float64), expected, float32, factor=4.0)
+    assert_near(case.state, state, float32 or not delta, factor=2.0)
+
+
+@TYPES
 def test_steps_with_keys_and_queries_of_infinite_length(pkg, ops, float32):
     """Squares that overflow give zero vectors: nothing is read from the state or written to it, and nothing is NaN.  A product
     of the vectors that is summed before they are scaled is infinite here."""
