@@ -1182,10 +1182,13 @@ template <bool kFp8>
 int launch_tc_pair(const void *a, const void *b, const EpilogueParams &ep, const std::size_t M, const std::size_t N,
                    const std::size_t K, cudaStream_t stream, const std::size_t groups = 1) {
   // Tiles of 192 columns where they take no more waves of pairs than tiles of 256: 2999 x 2048 outputs are 96 wide tiles or
-  // 132 narrow ones on 74 pairs, two waves either way (K = 512: 33.6 and 27.4 us, 768: 35.4 and 29.4, 2048: 33.6 and 32.8;
-  // 3001 x 1920 at K = 1920 42 and 36, at 5120 71 and 67).  One wave more costs more than the width saves (8192 x 2048, four
+  // 132 narrow ones on 74 pairs, two waves either way.  What they save is the end of a tile, and a share of its products; what they cost is
+  // more traffic per product, so results of 4 bytes gain at every K (3001 x 1920: K = 512 20.8 -> 17.9 us, 2048 32.3 -> 31.4, 8448 95.1 ->
+  // 94.1; from 14 % faster to 1.5 % slower over 100 sizes) and BF16 results at short ones (15.0 -> 13.9, 28.5 -> 28.9, 88.9 -> 90.4; 512 x
+  // 6144 at K = 2048 19.4 -> 18.0; up to 5 % slower from K = 4096 on).  One wave more costs more than the width saves (8192 x 2048, four
   // and five: K = 2048 64 and 70 us, 8448 224 and 266).  A gate pairs 128-column halves, and groups keep their tiles.
-  if (ep.gate_mode == 0 && ep.tile_group == nullptr) {
+  const bool narrow_pays = ep.out_f32 != nullptr || K * (kFp8 ? 1 : 2) <= 4096;
+  if (narrow_pays && ep.gate_mode == 0 && ep.tile_group == nullptr) {
     int status = kOk, sm_count = 0;
     if (tc::error_word(&status, &sm_count) == nullptr) return status;
     const auto waves = [&](const std::size_t columns) {
