@@ -88,6 +88,21 @@ __device__ __forceinline__ bf16 gelu_round_small(const float x) {
 // What a result is added to.  A stream reads it beside x, so that the trip to memory does not follow the sums.
 struct Addends {
   float first = 0.0F, second = 0.0F;  // F32: the old result and the bias; BF16: the residual and the bias
+  __device__ __forceinline__ float old_result() const { return first; }
+  __device__ __forceinline__ float bias_f32() const { return second; }
+  __device__ __forceinline__ float residual() const { return first; }
+  __device__ __forceinline__ float bias() const { return second; }
+};
+// The same, read where it is used: the kernel of a few rows has no registers to hold it (8 E4M3 rows of 5120 x 1920 18.6 us, 20.5
+// with the word that was spilled for it).
+struct LateAddends {
+  const GemvParams &p;
+  std::size_t old_index, residual_index;
+  int column;
+  __device__ __forceinline__ float old_result() const { return p.out_f32[old_index]; }
+  __device__ __forceinline__ float bias_f32() const { return p.bias_f32[column]; }
+  __device__ __forceinline__ float residual() const { return bf2f(p.residual[residual_index]); }
+  __device__ __forceinline__ float bias() const { return bf2f(p.bias[column]); }
 };
 __device__ __forceinline__ Addends addends_of(const GemvParams &p, const int r, const std::size_t out_index, const int out_columns,
                                               const int column) {
@@ -103,14 +118,15 @@ __device__ __forceinline__ Addends addends_of(const GemvParams &p, const int r, 
 }
 
 // Result `column` of row `out_index` from its sum, or from the sums of a gated pair.
-template <class Total>
+template <class Added, class Total>
 __device__ __forceinline__ void finish_column(const GemvParams &p, const std::size_t out_index, const int out_columns,
-                                              const int column, const float alpha, const int local, const Addends &addends,
+                                              const int column, const float alpha, const int local, const Added &addends,
                                               const Total &total) {
   if (p.out_f32 != nullptr) {
     float value = total(local) * alpha;
-    if (p.bias_f32 != nullptr) value += addends.second;
-    p.out_f32[out_index * out_columns + column] = soft_cap(p.accumulate_f32 != 0 ? addends.first + value : value, p.softcap);
+    if (p.bias_f32 != nullptr) value += addends.bias_f32();
+    p.out_f32[out_index * out_columns + column] =
+        soft_cap(p.accumulate_f32 != 0 ? addends.old_result() + value : value, p.softcap);
     return;
   }
   bf16 *const out_row = p.out + out_index * out_columns;
@@ -128,10 +144,10 @@ __device__ __forceinline__ void finish_column(const GemvParams &p, const std::si
     out_row[column] = f2bf(activated * second);
   } else {
     float value = total(local) * alpha;
-    if (p.bias_mode == 1) value += addends.second;
+    if (p.bias_mode == 1) value += addends.bias();
     value = rbf(value);
-    if (p.bias_mode == 2) value = rbf(value + addends.second);
-    if (p.residual != nullptr) value = rbf(value + addends.first);
+    if (p.bias_mode == 2) value = rbf(value + addends.bias());
+    if (p.residual != nullptr) value = rbf(value + addends.residual());
     out_row[column] = f2bf(value);
   }
 }
@@ -234,7 +250,8 @@ gemv_kernel(const GemvParams p) {
   if (r >= p.rows || column >= out_columns) return;
   const std::size_t out_index = grouped ? blockIdx.y : r;
   const float alpha = grouped && p.row_scale != nullptr ? p.alpha * p.row_scale[out_index] : p.alpha;
-  finish_column(p, out_index, out_columns, column, alpha, local, addends_of(p, r, out_index, out_columns, column), [&](const int c) {
+  const LateAddends addends{p, out_index * out_columns + column, static_cast<std::size_t>(r) * out_columns + column, column};
+  finish_column(p, out_index, out_columns, column, alpha, local, addends, [&](const int c) {
     float sum = 0.0F;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) sum += partial[w][c][r];
