@@ -1184,18 +1184,20 @@ int launch_tc_pair(const void *a, const void *b, const EpilogueParams &ep, const
   // Tiles of 192 columns where they take no more waves of pairs than tiles of 256: 2999 x 2048 outputs are 96 wide tiles or
   // 132 narrow ones on 74 pairs, two waves either way.  What they save is the end of a tile, and a share of its products; what they cost is
   // more traffic per product, so results of 4 bytes gain at every K (3001 x 1920: K = 512 20.8 -> 17.9 us, 2048 32.3 -> 31.4, 8448 95.1 ->
-  // 94.1; from 14 % faster to 1.5 % slower over 100 sizes) and BF16 results at short ones (15.0 -> 13.9, 28.5 -> 28.9, 88.9 -> 90.4; 512 x
-  // 6144 at K = 2048 19.4 -> 18.0; up to 5 % slower from K = 4096 on).  One wave more costs more than the width saves (8192 x 2048, four
-  // and five: K = 2048 64 and 70 us, 8448 224 and 266).  A gate pairs 128-column halves, and groups keep their tiles.
-  const bool narrow_pays = ep.out_f32 != nullptr || K * (kFp8 ? 1 : 2) <= 4096;
-  if (narrow_pays && ep.gate_mode == 0 && ep.tile_group == nullptr) {
+  // 94.1; from 14 % faster to 1.5 % slower over 100 sizes) and BF16 results at short ones (K = 512 15.0 -> 13.9, 1920 26.6 -> 26.3; 512 x
+  // 6144 at K = 2048 19.3 -> 18.9).  Beyond that BF16 results lose 2 to 5 % in one wave (1500 x 1920, K = 8448: 46.5 -> 48.1) and break even in
+  // more where the narrow tiles are the fewer columns (2999 x 1920, K = 5120: 56.5 and 56.6 with the rows in L2, 70.2 -> 69.1 in a model).
+  // One wave more costs more than the width saves (8192 x 2048, four and five: K = 2048 64 and 70 us, 8448 224 and 266).  A gate
+  // pairs 128-column halves, and groups keep their tiles.
+  if (ep.gate_mode == 0 && ep.tile_group == nullptr) {
     int status = kOk, sm_count = 0;
     if (tc::error_word(&status, &sm_count) == nullptr) return status;
-    const auto waves = [&](const std::size_t columns) {
-      const std::size_t pairs = static_cast<std::size_t>(sm_count) / 2;
-      return ((M + 255) / 256 * ((N + columns - 1) / columns) + pairs - 1) / pairs;
-    };
-    if (waves(192) <= waves(256)) return launch_tc_pair_as<kFp8, 192>(a, b, ep, M, N, K, stream, groups);
+    const auto tiles = [&](const std::size_t columns) { return (M + 255) / 256 * ((N + columns - 1) / columns); };
+    const std::size_t pairs = static_cast<std::size_t>(sm_count) / 2;
+    const bool more_waves = (tiles(192) + pairs - 1) / pairs > (tiles(256) + pairs - 1) / pairs;
+    const bool narrow_pays = ep.out_f32 != nullptr || K * (kFp8 ? 1 : 2) <= 4096 ||
+                             (tiles(256) > pairs && tiles(192) * 192 < tiles(256) * 256);
+    if (!more_waves && narrow_pays) return launch_tc_pair_as<kFp8, 192>(a, b, ep, M, N, K, stream, groups);
   }
   return launch_tc_pair_as<kFp8, 256>(a, b, ep, M, N, K, stream, groups);
 }

@@ -105,7 +105,7 @@ def test_pair_kernel_epilogues_at_ragged_sizes(ops):
 
 
 @pytest.mark.parametrize("rows,inner,columns", [(520, 72, 4000), (520, 1920, 4225), (769, 520, 3073), (2999, 264, 2050), (1500, 128, 1920),
-                                               (600, 2080, 4096)])
+                                               (600, 2080, 4096), (2999, 2080, 1920)])
 def test_pair_tiles_of_192_columns(ops, rows, inner, columns):
     """Sizes whose narrow tiles take no more waves than the wide ones, with remainders in every direction: BF16 results with
     bias and residual, F32 results stored and added, E4M3 operands.  The products are exact, sums of `inner` of them rounded
