@@ -263,6 +263,13 @@ def test_products_of_rows_and_weights_that_are_not_finite(pkg, ops, float32, row
     finite = expected.isfinite() & ~bound
     magnitudes = torch.nan_to_num(x.double().abs(), 0.0, 0.0) @ torch.nan_to_num(w.double().abs(), 0.0, 0.0).T
     assert bool(((out.double() - expected).abs() <= (24 + inner / 512) * 2.0 ** -24 * magnitudes)[finite].all())
+    if float32 == 1:  # added to an old result: once, whichever way a result took
+        old = torch.randn(rows, outer, device="cuda")
+        added = old.clone()
+        ops.call("f32_linear", x.data_ptr(), w.data_ptr(), rows, inner, outer, 1, added.data_ptr(), stream())
+        assert torch.equal(added.isnan(), out.isnan()) and torch.equal(added.isinf(), out.isinf())
+        sums = old + out
+        assert torch.equal(added[sums.isfinite()], sums[sums.isfinite()])
 
 
 def test_rows_that_fill_up_a_tile_cost_no_more_than_rows(pkg, ops):
